@@ -68,6 +68,49 @@ __device__ __noinline__ float fmtPq255(float v, float kWhite) {
     return __fmul_rn(fmtExp2(__fmul_rn(78.84375f, fmtLog2(r))), 255.0f);
 }
 
+// Linear RgbaF16's mismatch needs only the integer part of the largest channel difference of two fmtPq255 levels, so the
+// synthesis reads the levels off a piecewise linear table and evaluates fmtPq255 itself only where the table cannot
+// tell that integer. Segment i covers the floats y = clamp(v kWhite, 0, 1) whose bits >> kPqShift are kPqBase + i (64
+// segments per octave, 2^-40 .. 1; all smaller y share segment 0), as (slope, intercept): level ~= y slope + intercept,
+// the chord moved half its sag up. Over every float y in [0, 1] the table is within 0.00383 of fmtPq255 (enumerated;
+// fmtPq255's own rounding noise is 0.0035 of that), so a difference of two levels is within kPqTol of the exact one.
+// The series costs ~140 instructions a level, six levels a pixel; a segment ~8. A 3840x2160 pair at t = 1/3, 2/3: 1175
+// us with the series for every pixel, 863 us so (1.6 % of the pixels undecided). 32 segments per octave would leave 2 %.
+constexpr int kPqShift = 17, kPqOctaves = 40, kPqSegs = (kPqOctaves << (23 - kPqShift)) + 1;
+constexpr uint32_t kPqBase = (uint32_t)(127 - kPqOctaves) << (23 - kPqShift);
+constexpr float kPqTol = 0.008f;
+constexpr size_t kPqSegBytes = (size_t)kPqSegs * 8;
+static_assert(kPqSegs <= fgk::kPqSegMax, "the host allocates kPqSegMax segments");
+
+__device__ double pqLevel(double y) {   // ST 2084 x 255
+    const double t = pow(y, 0.1593017578125);
+    return 255.0 * pow((0.8359375 + 18.8515625 * t) / (1.0 + 18.6875 * t), 78.84375);
+}
+__global__ void __launch_bounds__(256) k_pq_seg(float2* seg) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= kPqSegs) return;
+    const double y0 = (double)__uint_as_float((kPqBase + (uint32_t)i) << kPqShift);
+    const double y1 = (double)__uint_as_float((kPqBase + (uint32_t)i + 1u) << kPqShift);
+    double s = 0.0, c;
+    if (i == 0) {
+        c = 0.5 * (pqLevel(0.0) + pqLevel(y1));
+    } else if (i == kPqSegs - 1) {
+        c = pqLevel(1.0);
+    } else {
+        const double l0 = pqLevel(y0), l1 = pqLevel(y1), ym = sqrt(y0 * y1);
+        s = (l1 - l0) / (y1 - y0);
+        c = l0 - s * y0 + 0.5 * (pqLevel(ym) - (l0 + s * (ym - y0)));
+    }
+    seg[i] = make_float2((float)s, (float)c);
+}
+
+__device__ __forceinline__ float pqApprox(const float2* seg, float v, float kWhite) {
+    const float y = __saturatef(__fmul_rn(v, kWhite));   // NaN -> 0, the level fmtPq255 gives it
+    const int i = max((int)__float_as_uint(y), (int)(kPqBase << kPqShift)) - (int)(kPqBase << kPqShift);
+    const float2 t = seg[i >> kPqShift];
+    return __fmaf_rn(y, t.x, t.y);
+}
+
 __device__ __forceinline__ float h2f(uint32_t h16) { return __half2float(__ushort_as_half((unsigned short)h16)); }
 
 // ============================================================================================== pixel access
@@ -403,6 +446,17 @@ __device__ __forceinline__ int mismatch(const FmtConst& f, const float wa[3], co
     return (int)fminf(m, 255.0f);
 }
 
+// linear RgbaF16: the same from the segment table; false where the table leaves two integers possible
+__device__ __forceinline__ bool mismatchPq(const FmtConst& f, const float2* seg, const float wa[3], const float wc[3], int& e) {
+    float m = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        m = fmaxf(m, fabsf(__fsub_rn(pqApprox(seg, wa[k], f.kWhite), pqApprox(seg, wc[k], f.kWhite))));
+    const int lo = floorPos(fmaxf(__fsub_rn(m, kPqTol), 0.0f)), hi = floorPos(__fadd_rn(m, kPqTol));
+    e = min(lo, 255);
+    return lo == hi;
+}
+
 // resolve.comp: m = 0.5 (a + c) at t = 0.5, else (1 - t) a + t c; out = m (1 - u) + n u
 __device__ __forceinline__ float mixF(float a, float c, const SynthParams& p) {
     return p.mid ? __fmul_rn(0.5f, __fadd_rn(a, c)) : __fadd_rn(__fmul_rn(p.wA, a), __fmul_rn(p.wC, c));
@@ -452,7 +506,7 @@ template <int F, bool kCut, bool kUi = false, class Sink>
 __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int by, Sink& sink) {
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ SyCoef rowc[kSyEH];
-    __shared__ unsigned int cnt;
+    __shared__ unsigned int cnt, nSlow;
     __shared__ int gReg[4];
     const int X0 = bx * kSyT, Y0 = by * kSyTH;
     const int tid = threadIdx.x, ex = tid & (kSyE - 1), ey0 = tid / kSyE;
@@ -463,7 +517,7 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
         }
         return;
     }
-    if (tid == 0) cnt = 0;
+    if (tid == 0) cnt = nSlow = 0;
     float2* hrow;
     uint8_t* e;
     unsigned short* hsum;
@@ -475,15 +529,20 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
     // pixels, (kSyTH / 2) x (kSyE / 2))
     float* mix = reinterpret_cast<float*>(hsum + kSyEH * kSyHS);
     float2* mixc = reinterpret_cast<float2*>(mix + kSyTH * kSyE);
+    // linear RgbaF16: the PQ segment table, and the region pixels it cannot decide (a queue over hsum, written later)
+    const bool pq = F == kFmtF16 && p.f.linear;
+    float2* seg = reinterpret_cast<float2*>(mix + 3 * kSyTH * kSyE);
+    unsigned short* slow = hsum;
+    static_assert(kSyE * kSyEH <= kSyEH * kSyHS && kSyE * kSyEH <= 65536, "every region pixel fits the queue");
+    if (pq) {
+        for (int i = tid; i < kPqSegs; i += kSyThreads) seg[i] = __ldg(p.pqSeg + i);
+        __syncthreads();
+    }
     const int lx = ex - kSyAp, x = X0 + lx;
-    // 2. the mismatch over the region, and the blend inputs of the output pixels
-    for (int k = 0; k < kSyK; k++) {
-        const int ey = ey0 + (kSyThreads / kSyE) * k;
-        const SyCoef cy = rowc[ey];
-        const float2 h = syHalfVec(cy, hrow, ex);
-        float wa[3], wc[3];
-        const float pax = __fsub_rn(cx.pos, __fmul_rn(kA, h.x)), pay = __fsub_rn(cy.pos, __fmul_rn(kA, h.y));
-        const float pcx = __fadd_rn(cx.pos, __fmul_rn(kC, h.x)), pcy = __fadd_rn(cy.pos, __fmul_rn(kC, h.y));
+    // both warps of a region pixel (at pos, with half-vector h), the tap rejection applied
+    auto warps = [&](float posx, float posy, float2 h, float wa[3], float wc[3]) {
+        const float pax = __fsub_rn(posx, __fmul_rn(kA, h.x)), pay = __fsub_rn(posy, __fmul_rn(kA, h.y));
+        const float pcx = __fadd_rn(posx, __fmul_rn(kC, h.x)), pcy = __fadd_rn(posy, __fmul_rn(kC, h.y));
         warp<F>(p, p.a, p.ac, pax, pay, wa);
         warp<F>(p, p.c, p.cc, pcx, pcy, wc);
         if (kUi) {
@@ -497,7 +556,21 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
                 }
             }
         }
-        e[ey * kSyES + ex] = (uint8_t)mismatch<F>(p.f, wa, wc);
+    };
+    // 2. the mismatch over the region, and the blend inputs of the output pixels
+    for (int k = 0; k < kSyK; k++) {
+        const int ey = ey0 + (kSyThreads / kSyE) * k;
+        const SyCoef cy = rowc[ey];
+        const float2 h = syHalfVec(cy, hrow, ex);
+        float wa[3], wc[3];
+        warps(cx.pos, cy.pos, h, wa, wc);
+        if (pq) {
+            int m;
+            if (!mismatchPq(p.f, seg, wa, wc, m)) slow[atomicAdd(&nSlow, 1u)] = (unsigned short)(ey * kSyE + ex);
+            e[ey * kSyES + ex] = (uint8_t)m;
+        } else {
+            e[ey * kSyES + ex] = (uint8_t)mismatch<F>(p.f, wa, wc);
+        }
         const int ly = ey - kSyAp;
         if ((unsigned)ly < (unsigned)kSyTH) {   // warp-uniform
             if (kYuv) {
@@ -526,6 +599,17 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
         }
     }
     __syncthreads();
+    if (pq) {   // the undecided pixels (about 1.6 % on natural content), dealt out over all threads: warped again, exact
+        const int n = (int)nSlow;
+        for (int i = tid; i < n; i += kSyThreads) {
+            const int sx = slow[i] & (kSyE - 1), sy = slow[i] / kSyE;
+            const SyCoef cy = rowc[sy];
+            float wa[3], wc[3];
+            warps((float)clampi(X0 - kSyAp + sx, 0, p.W - 1), cy.pos, syHalfVec(cy, hrow, sx), wa, wc);
+            e[sy * kSyES + sx] = (uint8_t)mismatch<F>(p.f, wa, wc);
+        }
+        __syncthreads();
+    }
     // 3. horizontal 7-sums (as k_synth)
     syRowSums(e, hsum, tid);
     __syncthreads();
@@ -859,11 +943,11 @@ static size_t fmtSynthSmem(int format, int fs) {
     const size_t mix = format == kFmtNv12 || format == kFmtP010
                            ? (size_t)kSyTH * kSyE * 4 + (size_t)((kSyTH + 1) / 2) * (kSyE / 2) * 8
                            : (size_t)3 * kSyTH * kSyE * 4;
-    return synthSmemBytes(fs) + mix;
+    return synthSmemBytes(fs) + mix + (format == kFmtF16 ? kPqSegBytes : 0);   // linear RgbaF16: the PQ segments
 }
 
 cudaError_t prepareFormatKernels() {
-    const int smem = (int)fmtSynthSmem(kFmtRgb10, 1);   // the largest
+    const int smem = (int)fmtSynthSmem(kFmtF16, 1);   // the largest
     cudaError_t e = cudaFuncSetAttribute(k_synth_fmt<kFmtRgb10>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt<kFmtF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt<kFmtNv12>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -972,6 +1056,11 @@ __global__ void __launch_bounds__(256) k_pq_table(float* tab, float kWhite) {
 }
 cudaError_t launchPqTable(float* tab, float kWhite, cudaStream_t s) {
     k_pq_table<<<65536 / 256, 256, 0, s>>>(tab, kWhite);
+    return cudaGetLastError();
+}
+
+cudaError_t launchPqSegments(float2* seg, cudaStream_t s) {
+    k_pq_seg<<<divUp(kPqSegs, 256), 256, 0, s>>>(seg);
     return cudaGetLastError();
 }
 

@@ -143,6 +143,7 @@ struct SynthParams {
     FmtConst f;
     const uint8_t* ac; const uint8_t* cc; size_t cpitch;
     uint8_t* outc; size_t outCPitch;
+    const float2* pqSeg;           // linear RgbaF16: the PQ segment table (launchPqSegments)
     // CrosshairV2's warp-tap rejection (8-bit RGBA): the UI masks of prev and curr (header + bytes, see UiV2Params);
     // both null = off
     const uint32_t* uiA; const uint32_t* uiC;
@@ -240,6 +241,9 @@ cudaError_t prepareFormatKernels();
 cudaError_t launchLumaFmt(const LumaPyrParams& p, cudaStream_t s);
 // the PQ level of every half value (65536 floats) for a linear RgbaF16 luma at this white level
 cudaError_t launchPqTable(float* tab, float kWhite, cudaStream_t s);
+// linear RgbaF16's synthesis: the PQ levels as a piecewise linear table (at most kPqSegMax segments, any white level)
+constexpr int kPqSegMax = 2562;
+cudaError_t launchPqSegments(float2* seg, cudaStream_t s);
 cudaError_t launchSynthFmt(const SynthParams& p, cudaStream_t s);
 // many syntheses of one of the other formats in one persistent launch (as launchSynthBatch), and their fallbacks
 cudaError_t launchSynthFmtBatch(const SynthBatchArgs& b, int format, int grid, size_t smem, cudaStream_t s);

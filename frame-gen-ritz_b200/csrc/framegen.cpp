@@ -223,6 +223,7 @@ struct Interpolator::Impl {
     char* arena = nullptr;
     size_t arenaBytes = 0;
     float* luma = nullptr;
+    float2* pqSeg = nullptr;  // linear RgbaF16: the PQ segment table of the synthesis
     float* pqTab = nullptr;   // linear RgbaF16: the PQ level of every half value (the luma pass looks them up)
     float2* field = nullptr;
     float* sads = nullptr;
@@ -474,6 +475,7 @@ struct Interpolator::Impl {
         if (arena) cudaFree(arena);
         arena = nullptr;
         pqTab = nullptr;
+        pqSeg = nullptr;
         arenaBytes = 0;
         for (cudaEvent_t e : events) cudaEventDestroy(e);
         events.clear();
@@ -512,6 +514,7 @@ struct Interpolator::Impl {
         const size_t oLeafOf = take((size_t)nb0 * 4), oLeafCnt = take(P.leaves.size() * 4), oLeafS = take(P.leaves.size() * 4);
         const bool pqLuma = fmt == Format::RgbaF16 && fc.linear;
         const size_t oPq = take(pqLuma ? (size_t)65536 * 4 : 0);
+        const size_t oPqSeg = take(pqLuma ? (size_t)fgk::kPqSegMax * 8 : 0);
         if (cudaMalloc(&arena, off) != cudaSuccess) { arena = nullptr; cudaGetLastError(); return kErrAlloc; }
         arenaBytes = off;
         cudaMemset(arena, 0, off);
@@ -524,7 +527,9 @@ struct Interpolator::Impl {
         blurCnt = (unsigned int*)(arena + oBlur);
         emap = (uint8_t*)(arena + oEmap);
         pqTab = pqLuma ? (float*)(arena + oPq) : nullptr;
+        pqSeg = pqLuma ? (float2*)(arena + oPqSeg) : nullptr;
         if (pqTab) fgk::launchPqTable(pqTab, fc.kWhite, 0);
+        if (pqSeg) fgk::launchPqSegments(pqSeg, 0);
         cudaMemcpy(arena + oLeaves, P.leaves.data(), P.leaves.size() * 8, cudaMemcpyHostToDevice);
         if (!P.inner.empty()) cudaMemcpy(arena + oInner, P.inner.data(), P.inner.size() * 8, cudaMemcpyHostToDevice);
         cudaMemcpy(arena + oDepth, P.depthStart.data(), P.depthStart.size() * 4, cudaMemcpyHostToDevice);
@@ -746,6 +751,7 @@ struct Interpolator::Impl {
         sp.untrusted = untrusted;
         sp.emap = capture ? emap : nullptr;
         sp.f = fc;
+        sp.pqSeg = pqSeg;
         sp.ac = (const uint8_t*)prev.chroma; sp.cc = (const uint8_t*)curr.chroma; sp.cpitch = prev.chromaPitch;
         sp.outc = (uint8_t*)out.chroma; sp.outCPitch = out.chromaPitch;
         return sp;

@@ -152,48 +152,111 @@ __device__ __forceinline__ float warpSum(float v) {
 }
 
 // ============================================================================================== luma tower
-constexpr int kTowerFloats = 1024 + 256 + 64 + 16 + 4 + 1;   // a 32x32 level-0 tile and its 16x16 .. 1x1 levels above
+constexpr int kTowerFloats = 1024 + 256 + 64 + 16 + 4 + 2;   // a 32x32 level-0 tile and its 16x16 .. 1x1 levels above
 
 // round half-even to a multiple of 2^-10 (the grid of the other formats' coarse pyramid levels)
 __device__ __forceinline__ float round10(float v) { return __fmul_rn(rintf(__fmul_rn(v, 1024.0f)), 1.0f / 1024.0f); }
 
+// one pixel (lx, ly) of level L of a tile's tower: the mean of the valid 2x2 pixels below it (sum * 1/4 when full,
+// sum / count at the odd edges), stored and kept in sl. ROUND: rounded to 2^-10.
+template <bool ROUND, int L>
+__device__ __forceinline__ void towerPx(const LumaPyrParams& p, float (*sl)[kTowerFloats], int tx0, int ty0, int lx, int ly) {
+    constexpr int side = 32 >> (L - 1), ns = side / 2;
+    constexpr int off = L == 1 ? 0 : L == 2 ? 1024 : L == 3 ? 1280 : L == 4 ? 1344 : 1360, noff = off + side * side;
+    const int X = (tx0 >> L) + lx, Y = (ty0 >> L) + ly;
+    float va = 0.0f, vc = 0.0f;
+    if (X < p.lw[L] && Y < p.lh[L]) {
+        const float* a = sl[0] + off + 2 * ly * side + 2 * lx;
+        const float* c = sl[1] + off + 2 * ly * side + 2 * lx;
+        const bool fx = 2 * X + 1 < p.lw[L - 1], fy = 2 * Y + 1 < p.lh[L - 1];
+        float sa = a[0], sc = c[0];
+        if (fx && fy) {
+            va = __fmul_rn(__fadd_rn(__fadd_rn(__fadd_rn(sa, a[1]), a[side]), a[side + 1]), 0.25f);
+            vc = __fmul_rn(__fadd_rn(__fadd_rn(__fadd_rn(sc, c[1]), c[side]), c[side + 1]), 0.25f);
+        } else if (fx || fy) {
+            const int o = fx ? 1 : side;
+            va = __fmul_rn(__fadd_rn(sa, a[o]), 0.5f);
+            vc = __fmul_rn(__fadd_rn(sc, c[o]), 0.5f);
+        } else {
+            va = sa;
+            vc = sc;
+        }
+        if (ROUND) { va = round10(va); vc = round10(vc); }
+        p.la[L][(size_t)Y * p.lw[L] + X] = va;
+        p.lc[L][(size_t)Y * p.lw[L] + X] = vc;
+    }
+    sl[0][noff + ly * ns + lx] = va;
+    sl[1][noff + ly * ns + lx] = vc;
+}
+
 // interp.pyramid :73-77 above one 32x32 level-0 tile held in sl[.][0..1023] (tx0, ty0: the tile's origin): levels
-// 1 .. p.nlev-1 of the tile's tower, each pixel the mean of the valid 2x2 pixels below it (sum * 1/4 when full,
-// sum / count at the odd edges), written to p.la / p.lc and kept in sl for the next level. ROUND: rounded to 2^-10.
+// 1 .. p.nlev-1 of the tile's tower, written to p.la / p.lc: level 1 by the whole CTA (a pixel per thread), the rest by
+// the first warp alone (no CTA barrier).
 template <bool ROUND>
 __device__ __forceinline__ void lumaTower(const LumaPyrParams& p, float (*sl)[kTowerFloats], int tx0, int ty0) {
-    int off = 0, side = 32;
-    for (int l = 1; l < p.nlev; l++) {
-        const int noff = off + side * side, ns = side >> 1;
-        const int X0 = tx0 >> l, Y0 = ty0 >> l;
-        const int pw = p.lw[l - 1], ph = p.lh[l - 1];
-        for (int i = threadIdx.x; i < ns * ns; i += 256) {
-            const int lx = i % ns, ly = i / ns, X = X0 + lx, Y = Y0 + ly;
-            float va = 0.0f, vc = 0.0f;
-            if (X < p.lw[l] && Y < p.lh[l]) {
-                float sa = 0.0f, sc = 0.0f;
-                int n = 0;
-                for (int j = 0; j < 2; j++)
-                    for (int k = 0; k < 2; k++)
-                        if (2 * X + k < pw && 2 * Y + j < ph) {
-                            const int ci = off + (2 * ly + j) * side + 2 * lx + k;
-                            sa = __fadd_rn(sa, sl[0][ci]);
-                            sc = __fadd_rn(sc, sl[1][ci]);
-                            n++;
-                        }
-                va = n == 4 ? __fmul_rn(sa, 0.25f) : __fdiv_rn(sa, (float)n);
-                vc = n == 4 ? __fmul_rn(sc, 0.25f) : __fdiv_rn(sc, (float)n);
-                if (ROUND) { va = round10(va); vc = round10(vc); }
-                p.la[l][(size_t)Y * p.lw[l] + X] = va;
-                p.lc[l][(size_t)Y * p.lw[l] + X] = vc;
-            }
-            sl[0][noff + i] = va;
-            sl[1][noff + i] = vc;
+    const int t = threadIdx.x;
+    if (p.nlev < 2) return;
+    towerPx<ROUND, 1>(p, sl, tx0, ty0, t & 15, t >> 4);
+    if (p.nlev < 3) return;
+    __syncthreads();
+    if (t >= 32) return;
+    towerPx<ROUND, 2>(p, sl, tx0, ty0, t & 7, t >> 3);
+    towerPx<ROUND, 2>(p, sl, tx0, ty0, t & 7, (t >> 3) + 4);
+    __syncwarp();
+    if (p.nlev < 4 || t >= 16) return;
+    towerPx<ROUND, 3>(p, sl, tx0, ty0, t & 3, t >> 2);
+    __syncwarp(0xffffu);
+    if (p.nlev < 5 || t >= 4) return;
+    towerPx<ROUND, 4>(p, sl, tx0, ty0, t & 1, t >> 1);
+    __syncwarp(0xfu);
+    if (p.nlev < 6 || t) return;
+    towerPx<ROUND, 5>(p, sl, tx0, ty0, 0, 0);
+}
+
+// q = 16 x a level-0 luma value (a multiple of 1/16, at most 255) in the low 16 bits, as the float's bits
+__device__ __forceinline__ uint32_t q16(float v) { return (uint32_t)__float_as_int(__fmaf_rn(v, 16.0f, 8388608.0f)); }
+
+// the pair-plane words (LumaPyrParams::pa / pc) of a 32x32 level-0 tile held in sl[.][0..1023]: pixel x's word is the
+// tile's own but for its column 31, whose high half belongs to the next tile's column 0 (each tile writes that half of
+// the word to its left)
+__device__ __forceinline__ void storePairs(const LumaPyrParams& p, const float (*sl)[kTowerFloats], int tx0, int ty0) {
+    const int fw = p.lw[0], fh = p.lh[0];
+    const int lx = threadIdx.x & 31, x = tx0 + lx;
+    if (x >= fw) return;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        uint32_t* plane = k ? p.pc : p.pa;
+        for (int ly = threadIdx.x >> 5; ly < 32 && ty0 + ly < fh; ly += 8) {
+            uint32_t* o = plane + (size_t)(ty0 + ly) * fw + x;
+            const uint32_t q = q16(sl[k][ly * 32 + lx]);
+            if (x == fw - 1) *o = __byte_perm(q, q, 0x5410);
+            else if (lx < 31) *o = __byte_perm(q, q16(sl[k][ly * 32 + lx + 1]), 0x5410);
+            else *reinterpret_cast<unsigned short*>(o) = (unsigned short)q;
+            if (lx == 0 && x > 0) reinterpret_cast<unsigned short*>(o)[-1] = (unsigned short)q;
         }
-        __syncthreads();
-        off = noff;
-        side = ns;
     }
+}
+
+// the pair words of two neighbouring pixels of a row (q0, q1; next: the pixel to their right) at the 8-byte aligned o;
+// edge: the second word's high half is the next tile's; left: this tile writes the high half of the word to its left
+__device__ __forceinline__ void storePairs2(uint32_t* o, uint32_t q0, uint32_t q1, uint32_t next, bool edge, bool left) {
+    const uint32_t w0 = q0 | (q1 << 16);
+    if (edge) {
+        o[0] = w0;
+        *reinterpret_cast<unsigned short*>(o + 1) = (unsigned short)q1;
+    } else {
+        *reinterpret_cast<uint2*>(o) = make_uint2(w0, q1 | (next << 16));
+    }
+    if (left) reinterpret_cast<unsigned short*>(o)[-1] = (unsigned short)q0;
+}
+
+// a level-0 value rewritten after the luma pass (CrosshairV2's estimate fill): its two halves in the pair plane
+__device__ __forceinline__ void storePairPx(uint32_t* plane, int fw, int x, int y, float v) {
+    unsigned short* o = reinterpret_cast<unsigned short*>(plane + (size_t)y * fw + x);
+    const unsigned short q = (unsigned short)q16(v);
+    o[0] = q;
+    if (x > 0) o[-1] = q;
+    if (x == fw - 1) o[1] = q;
 }
 
 // ============================================================================================== synthesis tile
@@ -328,7 +391,110 @@ __device__ __forceinline__ float2 syHalfVec(const SyCoef& cy, const float2* hrow
                        __fadd_rn(__fmul_rn(h0.y, cy.a0), __fmul_rn(h1.y, cy.a1)));
 }
 
+// ============================================================================================== scene-cut mean, spread
+// One leaf of the pairwise tree by one warp, in numpy's order: lanes 0..7 are its 8 accumulators (independent loads),
+// combined as ((r0 + r1) + (r2 + r3)) + ((r4 + r5) + (r6 + r7)), then the tail; leaves under 8 elements by lane 0
+// alone. Also returns (in every lane) the leaf's sum of roundEven(sad * 256), the debug counter's share.
+__device__ __forceinline__ float warpLeafSum(const float* a, int n, int lane, unsigned int& s256) {
+    unsigned int s = 0;
+    for (int i = lane; i < n; i += 32) s += (unsigned int)__float2int_rn(__fmul_rn(__ldcg(a + i), 256.0f));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    s256 = s;
+    float res = 0.0f;
+    if (n < 8) {
+        if (lane == 0)
+            for (int i = 0; i < n; i++) res = __fadd_rn(res, __ldcg(a + i));
+        return __shfl_sync(0xffffffffu, res, 0);
+    }
+    const int body = n - (n % 8);
+    float r = 0.0f;
+    if (lane < 8) {
+        r = __ldcg(a + lane);
+        for (int i = 8 + lane; i < body; i += 8) r = __fadd_rn(r, __ldcg(a + i));
+    }
+    const float r1 = __shfl_down_sync(0xffffffffu, r, 1);   // lane 2k: r[2k] + r[2k+1]
+    const float p2 = __fadd_rn(r, r1);
+    const float p2b = __shfl_down_sync(0xffffffffu, p2, 2);  // lane 4k: (r0 + r1) + (r2 + r3)
+    const float p4 = __fadd_rn(p2, p2b);
+    const float p4b = __shfl_down_sync(0xffffffffu, p4, 4);
+    if (lane == 0) {
+        res = __fadd_rn(p4, p4b);
+        for (int i = body; i < n; i++) res = __fadd_rn(res, __ldcg(a + i));
+    }
+    return __shfl_sync(0xffffffffu, res, 0);
+}
+
+// leaf `leaf` of the scene-cut mean (its SADs complete and visible), by one warp; the warp that completes the last leaf
+// adds the inner nodes, one height per step, and writes the mean, the cut decision and the debug counter
+__device__ __forceinline__ void cutMeanLeaf(const CutPlan& pl, const float* sads, int nb, float cutSad, DevState* st, int leaf,
+                                            int lane) {
+    const int2 lf = pl.leaves[leaf];
+    unsigned int s256;
+    const float v = warpLeafSum(sads + lf.x, lf.y, lane, s256);
+    unsigned int done = 0;
+    if (lane == 0) {
+        pl.gvals[leaf] = v;
+        pl.leafS256[leaf] = s256;
+        __threadfence();
+        done = atomicAdd(&st->subDone, 1u);
+    }
+    done = __shfl_sync(0xffffffffu, done, 0);
+    if (done != (unsigned int)pl.nLeaves - 1u) return;
+    __threadfence();
+    for (int d = 0; d < pl.nSteps; d++) {
+        for (int j = pl.depthStart[d] + lane; j < pl.depthStart[d + 1]; j += 32) {
+            const int2 c = pl.inner[j];
+            pl.gvals[pl.nLeaves + j] = __fadd_rn(__ldcg(pl.gvals + c.x), __ldcg(pl.gvals + c.y));
+        }
+        __threadfence_block();
+        __syncwarp();
+    }
+    unsigned int tot = 0;
+    for (int i = lane; i < pl.nLeaves; i += 32) tot += __ldcg(pl.leafS256 + i);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    if (lane == 0) {
+        const float mean = __fdiv_rn(__ldcg(pl.gvals + pl.root), (float)nb);
+        st->sadMean = mean;
+        st->cut = mean > cutSad ? 1u : 0u;
+        st->sadSum256 = tot;
+        st->subDone = 0;
+    }
+}
+
+// the scene-cut mean's share of the warp that wrote the SAD of block b (warp-uniform call)
+__device__ __forceinline__ void cutMeanShare(const SubpixParams& p, int b, int nb, int lane) {
+    const CutPlan& pl = p.plan;
+    const int leaf = pl.leafOf[b];
+    unsigned int old = 0;
+    if (lane == 0) {
+        __threadfence();   // this warp's SAD before its arrival
+        old = atomicAdd(pl.leafCnt + leaf, 1u);
+    }
+    old = __shfl_sync(0xffffffffu, old, 0);
+    if (old != (unsigned int)pl.leaves[leaf].y - 1u) return;
+    __threadfence();
+    if (lane == 0) pl.leafCnt[leaf] = 0;
+    cutMeanLeaf(pl, p.sads, nb, p.cutSad, p.st, leaf, lane);
+}
+
 inline unsigned int divUp(int a, int b) { return (unsigned int)((a + b - 1) / b); }
+
+// the CTA ranges of a merged launch's items
+template <class P, class F>
+static int layoutMerged(Merged<P>& m, F ctasOf) {   // ctasOf(item, gx&) -> the item's CTA count
+    int total = 0;
+    for (int i = 0; i < m.n; i++) {
+        int gx = 1;
+        const int c = ctasOf(m.item[i], gx);
+        m.first[i] = total;
+        m.gx[i] = gx;
+        total += c;
+    }
+    m.first[m.n] = total;
+    return total;
+}
 
 template <typename... KArgs, typename... Args>
 cudaError_t launchPdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {

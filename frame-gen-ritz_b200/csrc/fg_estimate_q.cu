@@ -1,0 +1,594 @@
+// The estimate's passes on integer luma: level 0 as pair planes (LumaPyrParams::pa / pc), a word holding a pixel and its
+// right neighbour as 16-bit multiples of 1/16 level. Bilinear taps are two-way dot products (dp2a) of a word with byte
+// weights, absolute differences one instruction (sad), all sums exact in 32 bits: the same values as the float kernels
+// of fg_kernels.cu, which run where level 0 is not a multiple of 1/16 (flowScale 4 with 3-pixel cells).
+//
+// All three passes are bound by instruction issue (66-77 % issue, ALU and FMA-heavy pipes 40-60 %). Measured (ncu,
+// 3840x2160 at flowScale 2, float kernel -> this one; warp instructions): level-0 search 41.4 -> 28.6 us (30.1 -> 20.1
+// M), sub-pixel 65.9 -> 24 us (38.6 -> 17 M, the scene-cut sum moved to the pixel-field launch), pixel field 80.4 ->
+// 43 us (52.8 -> 26.2 M). The pair planes cost the luma pass nothing: float level 0 is written only where a pass reads it.
+#include "fg_device.h"
+
+namespace fgk {
+
+// ============================================================================================== seed + search
+// interp.seed_from :131-144 and interp.search :116-124, as k_search_r (fg_kernels.cu), one warp per 8x8 block, for
+// radii 1 and 2. Lane = (column x, rows 2 g and 2 g + 1) of the block: a candidate's score is two absolute differences
+// per lane and one warp reduction. The window's rows stay in registers for all dy of one dx.
+//
+// kPair: level 0's pair planes (the pixel in a word's low half); else a float level whose values times qscale are
+// integers below 2^23: the float 2^23 + v qscale holds them in its low bits, and the exponent cancels in differences.
+template <bool kPair>
+struct QSrc {
+    const void* a;
+    const void* c;
+    float scale;
+    __device__ __forceinline__ uint32_t ld(const void* plane, int i) const {
+        if (kPair) return __ldg(reinterpret_cast<const uint32_t*>(plane) + i) & 0xFFFFu;
+        return __float_as_uint(__fmaf_rn(__ldg(reinterpret_cast<const float*>(plane) + i), scale, 8388608.0f));
+    }
+};
+
+// a warp reduction's result k to lane k
+__device__ __forceinline__ void keepLane(uint32_t& mine, uint32_t r, int lane, int k) { mine = lane == k ? r : mine; }
+
+template <int R, bool kPair>
+__device__ __forceinline__ void searchQCta(const SearchParams& p, int ctaX, int by) {
+    constexpr int T = 8 + 2 * R, TS = 12, D = 2 * R + 1;   // TS: two rows = 24 words, so the 4 row pairs hit all banks
+    static_assert(T <= TS && D * D <= 32, "radius 1 or 2");
+    __shared__ uint32_t win[4][2][T * TS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int bx = ctaX * 4 + warp;
+    if (bx >= p.bw) return;
+    const QSrc<kPair> src = kPair ? QSrc<kPair>{p.pa, p.pc, 0.0f} : QSrc<kPair>{p.la, p.lc, p.qscale};
+    const float unit = kPair ? 1.0f / 1024.0f : 1.0f / (64.0f * p.qscale);   // a block sum -> its mean in levels (exact)
+    const int b = by * p.bw + bx, b0x = bx * kBlock, b0y = by * kBlock;
+    const int lx = lane & 7, ly = (lane >> 3) * 2;
+    // the seed: own parent, the 3 nearest other parents, zero, the global median (2x the parent level's vectors); the
+    // first minimum. A candidate equal to an earlier one could never be picked.
+    int sx = 0, sy = 0;
+    if (!p.top) {
+        int cxs[6], cys[6];
+        bool pen0 = false;   // the first candidate pays lambda too
+        if (p.cnn) {   // the seed net's two candidates, then zero (slots 3..5 repeat it)
+            const float* o = p.cnn + (size_t)b * kSeedNetOut;
+#pragma unroll
+            for (int k = 0; k < 6; k++) {
+                cxs[k] = k < 2 ? __float2int_rn(fminf(fmaxf(o[2 * k], -256.0f), 256.0f)) : 0;
+                cys[k] = k < 2 ? __float2int_rn(fminf(fmaxf(o[2 * k + 1], -256.0f), 256.0f)) : 0;
+            }
+            pen0 = !(o[4] >= 0.0f);
+        } else {
+            const int px = min(bx >> 1, p.pw - 1), py = min(by >> 1, p.ph - 1);
+            const int px1 = clampi(px + ((bx & 1) ? 1 : -1), 0, p.pw - 1), py1 = clampi(py + ((by & 1) ? 1 : -1), 0, p.ph - 1);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {   // own, vertical, horizontal, diagonal neighbour
+                const float2 v = __ldg(p.parent + ((k & 1) ? py1 : py) * p.pw + ((k & 2) ? px1 : px));
+                cxs[k] = 2 * __float2int_rn(v.x);
+                cys[k] = 2 * __float2int_rn(v.y);
+            }
+            cxs[4] = cys[4] = 0;
+            cxs[5] = __float2int_rn(p.med[0]);
+            cys[5] = __float2int_rn(p.med[1]);
+        }
+        const int qx = b0x + lx, qy = b0y + ly;
+        float best = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            bool dup = false;
+#pragma unroll
+            for (int j = 0; j < k; j++) dup |= cxs[j] == cxs[k] && cys[j] == cys[k];
+            if (dup) continue;   // warp-uniform
+            const int cx = cxs[k], cy = cys[k];
+            uint32_t s;
+            if (b0x - abs(cx) >= 0 && b0x + 7 + abs(cx) < p.w && b0y - abs(cy) >= 0 && b0y + 7 + abs(cy) < p.h) {
+                const int ia = (qy - cy) * p.w + (qx - cx), ic = (qy + cy) * p.w + (qx + cx);
+                s = __usad(src.ld(src.a, ia + p.w), src.ld(src.c, ic + p.w), __usad(src.ld(src.a, ia), src.ld(src.c, ic), 0u));
+            } else {
+                const int xa = clampi(qx - cx, 0, p.w - 1), xc = clampi(qx + cx, 0, p.w - 1);
+                s = 0;
+#pragma unroll
+                for (int r = 0; r < 2; r++)
+                    s = __usad(src.ld(src.a, clampi(qy + r - cy, 0, p.h - 1) * p.w + xa),
+                               src.ld(src.c, clampi(qy + r + cy, 0, p.h - 1) * p.w + xc), s);
+            }
+            float cost = __fmul_rn((float)__reduce_add_sync(0xffffffffu, s), unit);
+            if (k > 0 || pen0) cost = __fadd_rn(cost, p.lambda);
+            if (k == 0 || cost < best) { best = cost; sx = cx; sy = cy; }
+        }
+    }
+    // the T x T windows of a at q - s and c at q + s
+    uint32_t* wa = win[warp][0];
+    uint32_t* wc = win[warp][1];
+    const int ax0 = b0x - sx - R, ay0 = b0y - sy - R, cx0 = b0x + sx - R, cy0 = b0y + sy - R;
+    constexpr int LR = 32 / T;   // window rows staged per step
+    const int tr = lane / T, tc = lane % T;
+    if (tr < LR) {
+        const bool in = ax0 >= 0 && ay0 >= 0 && ax0 + T <= p.w && ay0 + T <= p.h && cx0 >= 0 && cy0 >= 0 && cx0 + T <= p.w && cy0 + T <= p.h;
+        if (in) {
+            const int ia = (ay0 + tr) * p.w + ax0 + tc, ic = (cy0 + tr) * p.w + cx0 + tc;
+#pragma unroll
+            for (int r = 0; r < T; r += LR)
+                if (T % LR == 0 || r + tr < T) {
+                    wa[(r + tr) * TS + tc] = src.ld(src.a, ia + r * p.w);
+                    wc[(r + tr) * TS + tc] = src.ld(src.c, ic + r * p.w);
+                }
+        } else {
+            const int xa = clampi(ax0 + tc, 0, p.w - 1), xc = clampi(cx0 + tc, 0, p.w - 1);
+            for (int r = tr; r < T; r += LR) {
+                wa[r * TS + tc] = src.ld(src.a, clampi(ay0 + r, 0, p.h - 1) * p.w + xa);
+                wc[r * TS + tc] = src.ld(src.c, clampi(cy0 + r, 0, p.h - 1) * p.w + xc);
+            }
+        }
+    }
+    __syncwarp();
+    uint32_t mine = 0;   // lane i: the sum of candidate i = (dy + R) D + dx + R
+    const uint32_t* pa = wa + ly * TS + lx;
+    const uint32_t* pc = wc + ly * TS + lx;
+#pragma unroll
+    for (int dxi = 0; dxi < D; dxi++) {
+        uint32_t a[D + 1], c[D + 1];   // rows ly - R .. ly + 1 + R of column lx -+ dx
+#pragma unroll
+        for (int i = 0; i <= D; i++) {
+            a[i] = pa[i * TS + 2 * R - dxi];
+            c[i] = pc[i * TS + dxi];
+        }
+#pragma unroll
+        for (int dyi = 0; dyi < D; dyi++)
+            keepLane(mine, __reduce_add_sync(0xffffffffu, __usad(a[2 * R - dyi + 1], c[dyi + 1], __usad(a[2 * R - dyi], c[dyi], 0u))),
+                     lane, dyi * D + dxi);
+    }
+    const int dy = lane / D - R, dx = lane % D - R;
+    const float sad = __fmul_rn((float)mine, unit);
+    const float cost = __fadd_rn(sad, __fmul_rn(p.lambda, (float)(abs(dx) + abs(dy))));   // = fl32(lambda n) (interp.py:121)
+    // the first minimum: costs are not negative, so their bits order as they do
+    const uint32_t bits = lane < D * D ? __float_as_uint(cost) : 0xffffffffu;
+    const int ci = __ffs(__ballot_sync(0xffffffffu, bits == __reduce_min_sync(0xffffffffu, bits))) - 1;
+    if (lane == ci) {
+        p.out[b] = make_float2((float)(sx + dx), (float)(sy + dy));
+        if (p.sadOut) p.sadOut[b] = sad;
+    }
+}
+template <int R, bool kPair>
+__global__ void __launch_bounds__(128) k_search_q(const SearchParams p) {
+    pdlEnter();
+    searchQCta<R, kPair>(p, blockIdx.x, blockIdx.y);
+}
+template <int R, bool kPair>
+__global__ void __launch_bounds__(128) k_search_q_m(const __grid_constant__ Merged<SearchParams> m) {
+    pdlEnter();
+    int bx, by;
+    const int i = mergedItem(m, bx, by);
+    searchQCta<R, kPair>(m.item[i], bx, by);
+}
+
+// ============================================================================================== sub-pixel refinement
+// interp.flow :162-163: search(., 1, 0.5) then search(., 1, 0.25) around the median-filtered integer vector s, as
+// k_subpix (fg_kernels.cu), one warp per finest-level block. Lane = (column x, rows 2 g and 2 g + 1). Both frames' pair
+// words of rows and columns -1 .. 8 around the block (9 words a row) wait in shared memory; a pass takes, per column
+// offset and frame, 4 rows of horizontal taps (one load and one dp2a each) and forms its 3 row offsets' vertical taps
+// from them: offsets are compile-time per pass and chosen half-pixel row, so a vertical tap is at most one multiply-add.
+constexpr int kQsS = 12, kQsRows = 10, kQsCols = 9;   // row stride (two rows = 24 words: conflict-free), rows, words a row
+
+// 9 candidates (dx, dy) = quarter offsets (b4x + S4 {-1, 0, 1}, BY + S4 {-1, 0, 1}); returns in lane i = (dy + 1) 3 +
+// dx + 1 its sum of absolute differences in units of 1/256 level
+template <int S4, int BY>
+__device__ __forceinline__ uint32_t subPass(const uint32_t* ta, const uint32_t* tc, int b4x, int lane) {
+    uint32_t mine = 0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const int o = b4x + S4 * (d - 1);   // a at x - o / 4, c at x + o / 4
+        const uint32_t wa = ((uint32_t)(-o) & 3u) * 255u + 4u, wc = ((uint32_t)o & 3u) * 255u + 4u;   // (4 - f) | f << 8
+        const uint32_t* qa = ta + ((-o) >> 2);
+        const uint32_t* qc = tc + (o >> 2);
+        uint32_t ha[4], hc[4];   // rows y - 1 .. y + 2
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            ha[i] = __dp2a_lo(qa[i * kQsS], wa, 0u);
+            hc[i] = __dp2a_lo(qc[i * kQsS], wc, 0u);
+        }
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+            constexpr int base[3] = {BY - S4, BY, BY + S4};
+            const int oa = -base[e], oc = base[e];
+            const int ra = 1 + (oa >> 2), rc = 1 + (oc >> 2), fa = oa & 3, fc = oc & 3;
+            uint32_t s = 0;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                uint32_t va, vc;   // x 1 (f = 0), x 2 (f = 2) or x 4
+                if (fa == 0) {
+                    va = ha[i + ra];
+                    vc = hc[i + rc];
+                } else if (fa == 2) {
+                    va = ha[i + ra] + ha[i + ra + 1];
+                    vc = hc[i + rc] + hc[i + rc + 1];
+                } else {
+                    va = ha[i + ra] * (uint32_t)(4 - fa) + ha[i + ra + 1] * (uint32_t)fa;
+                    vc = hc[i + rc] * (uint32_t)(4 - fc) + hc[i + rc + 1] * (uint32_t)fc;
+                }
+                s = __usad(va, vc, s);
+            }
+            keepLane(mine, __reduce_add_sync(0xffffffffu, s) << (fa == 0 ? 2 : (fa == 2 ? 1 : 0)), lane, e * 3 + d);
+        }
+    }
+    return mine;
+}
+
+__device__ __forceinline__ void subpixQCta(const SubpixParams& p, int ctaX, int by) {
+    __shared__ uint32_t tile[4][2][kQsRows * kQsS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int bx = ctaX * 4 + warp;
+    if (bx >= p.bw) return;
+    const int b = by * p.bw + bx, b0x = bx * kBlock, b0y = by * kBlock;
+    const float2 v0 = __ldg(p.in + b);
+    const int sx = __float2int_rn(v0.x), sy = __float2int_rn(v0.y);
+    uint32_t* wa = tile[warp][0];
+    uint32_t* wc = tile[warp][1];
+    const int ax0 = b0x - sx - 1, ay0 = b0y - sy - 1, cx0 = b0x + sx - 1, cy0 = b0y + sy - 1;
+    const int tr = lane / kQsCols, tc = lane % kQsCols;   // 3 rows per step
+    if (tr < 3) {
+        const bool in = ax0 >= 0 && ay0 >= 0 && ax0 + kQsCols < p.w && ay0 + kQsRows <= p.h && cx0 >= 0 && cy0 >= 0 &&
+                        cx0 + kQsCols < p.w && cy0 + kQsRows <= p.h;
+        if (in) {
+            const uint32_t* qa = p.pa + (ay0 + tr) * p.w + ax0 + tc;
+            const uint32_t* qc = p.pc + (cy0 + tr) * p.w + cx0 + tc;
+#pragma unroll
+            for (int r = 0; r < kQsRows; r += 3)
+                if (r + 3 <= kQsRows || r + tr < kQsRows) {
+                    wa[(r + tr) * kQsS + tc] = __ldg(qa + r * p.w);
+                    wc[(r + tr) * kQsS + tc] = __ldg(qc + r * p.w);
+                }
+        } else {   // clamped: left of the frame both halves are pixel 0 (the last column's word repeats its pixel)
+            const int xa = clampi(ax0 + tc, 0, p.w - 1), xc = clampi(cx0 + tc, 0, p.w - 1);
+            for (int r = tr; r < kQsRows; r += 3) {
+                const uint32_t a = __ldg(p.pa + clampi(ay0 + r, 0, p.h - 1) * p.w + xa), c = __ldg(p.pc + clampi(cy0 + r, 0, p.h - 1) * p.w + xc);
+                wa[r * kQsS + tc] = ax0 + tc < 0 ? __byte_perm(a, a, 0x1010) : a;
+                wc[r * kQsS + tc] = cx0 + tc < 0 ? __byte_perm(c, c, 0x1010) : c;
+            }
+        }
+    }
+    __syncwarp();
+    // this lane's column and first row in the tiles: pixel (x, y) is word (x + 1, y + 1); rows from y - 1
+    const uint32_t* ta = wa + (lane >> 3) * 2 * kQsS + (lane & 7) + 1;
+    const uint32_t* tcq = wc + (lane >> 3) * 2 * kQsS + (lane & 7) + 1;
+    const int n = lane < 9 ? abs(lane % 3 - 1) + abs(lane / 3 - 1) : 0;
+    int b4x = 0, b4y = 0;   // the offset chosen so far, quarter pixels
+    float sadBest = 0.0f;
+#pragma unroll
+    for (int pass = 0; pass < 2; pass++) {
+        uint32_t sum;
+        if (pass == 0) sum = subPass<2, 0>(ta, tcq, 0, lane);
+        else if (b4y == 0) sum = subPass<1, 0>(ta, tcq, b4x, lane);
+        else if (b4y < 0) sum = subPass<1, -2>(ta, tcq, b4x, lane);
+        else sum = subPass<1, 2>(ta, tcq, b4x, lane);
+        const float sad = __fmul_rn((float)sum, 1.0f / 16384.0f);
+        const float cost = __fadd_rn(sad, n == 0 ? p.pen[pass][0] : (n == 1 ? p.pen[pass][1] : p.pen[pass][2]));
+        const uint32_t bits = lane < 9 ? __float_as_uint(cost) : 0xffffffffu;   // costs are not negative
+        const int ci = __ffs(__ballot_sync(0xffffffffu, bits == __reduce_min_sync(0xffffffffu, bits))) - 1;
+        const int step = pass ? 1 : 2;
+        b4x += step * (ci % 3 - 1);
+        b4y += step * (ci / 3 - 1);
+        if (pass) sadBest = __shfl_sync(0xffffffffu, sad, ci);
+        else if (p.out0 && lane == 0)
+            p.out0[b] = make_float2(__fadd_rn((float)sx, (float)b4x * 0.25f), __fadd_rn((float)sy, (float)b4y * 0.25f));
+    }
+    if (lane == 0) {
+        p.out[b] = make_float2(__fadd_rn((float)sx, (float)b4x * 0.25f), __fadd_rn((float)sy, (float)b4y * 0.25f));
+        p.sads[b] = sadBest;   // summed for the scene cut by the pixel-field launch
+    }
+}
+__global__ void __launch_bounds__(128) k_subpix_q(const SubpixParams p) {
+    pdlEnter();
+    subpixQCta(p, blockIdx.x, blockIdx.y);
+}
+__global__ void __launch_bounds__(128) k_subpix_q_m(const __grid_constant__ Merged<SubpixParams> m) {
+    pdlEnter();
+    int bx, by;
+    const int i = mergedItem(m, bx, by);
+    subpixQCta(m.item[i], bx, by);
+}
+
+// ============================================================================================== per-pixel field
+// interp.pixel_field :167-183 at flow resolution, as k_pixfield (fg_kernels.cu): per pixel the candidate vectors
+// bilinear block field, own block, block above / below / left / right, zero; each scored by the 5x5 replicate-border
+// box of |a(q - h) - c(q + h)| where every window pixel uses its own candidate; the first minimum wins.
+//
+// One CTA = 60 x 32 outputs (4 block rows) with a 2 px apron, one candidate at a time. A thread owns a region column
+// and the 8 rows of one block row, so a block candidate has one vector, one set of weights and two row pointers per
+// run: per row and frame one load and one dp2a, the lower tap row reused as the next row's upper one. The 2 + 2 apron rows take one more pixel per thread. Errors
+// stay in registers: the vertical 5-sums run down the thread's rows (2 rows above and below from the neighbours through
+// shared memory), the horizontal 5-sums and the choice along rows, 8 pixels per thread. Tiles whose vectors take no tap
+// outside the frame run without any clamp (kIn).
+constexpr int kQfE = 64, kQfAp = 2, kQfTW = kQfE - 2 * kQfAp, kQfTH = 32, kQfNC = 7;
+constexpr int kQfG = kQfTH / 8;                             // block rows (thread rows) of a tile
+constexpr int kQfBX = kQfE / 8 + 4, kQfBY = kQfG + 4;       // block-field region: the tile's, the apron's, +-1 around
+constexpr int kQfVS = kQfE + 4;   // row stride of the vertical sums: 16-byte loads down 8 rows hit all banks once
+
+// the horizontal stage of a bilinear tap at 1/32 position 32 q + X: column and byte weights (left, right). kIn: the tap
+// is known to lie inside the frame; else clamped
+struct QCol {
+    int x;
+    uint32_t w;
+};
+template <bool kIn>
+__device__ __forceinline__ QCol qCol(int q, int X, int w) {
+    const int i = q + (X >> 5);
+    const uint32_t wt = ((uint32_t)X & 31u) * 255u + 32u;   // (32 - f) | f << 8
+    QCol c;
+    c.x = kIn ? i : clampi(i, 0, w - 1);      // the last column's word repeats its pixel
+    c.w = kIn || i >= 0 ? wt : 32u;           // left of the frame: pixel 0 alone
+    return c;
+}
+// a pair-plane word at a byte offset (planes are below 4 GiB)
+__device__ __forceinline__ uint32_t ldPair(const uint32_t* plane, uint32_t off) {
+    return __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(plane) + off));
+}
+// |a(q - h) - c(q + h)| in units of 2^-14 at pixel (qx, qy) for R = rne(32 h)
+template <bool kIn>
+__device__ __forceinline__ uint32_t qErr(const PixfieldParams& p, int qx, int qy, int Rx, int Ry) {
+    const QCol ca = qCol<kIn>(qx, -Rx, p.w), cc = qCol<kIn>(qx, Rx, p.w);
+    const int ya = qy + ((-Ry) >> 5), yc = qy + (Ry >> 5);
+    const uint32_t fa = (uint32_t)(-Ry) & 31u, fc = (uint32_t)Ry & 31u;
+    uint32_t oa = 4u * (uint32_t)((kIn ? ya : clampi(ya, 0, p.h - 1)) * p.w + ca.x);
+    uint32_t oc = 4u * (uint32_t)((kIn ? yc : clampi(yc, 0, p.h - 1)) * p.w + cc.x);
+    const uint32_t a0 = __dp2a_lo(ldPair(p.pa, oa), ca.w, 0u), c0 = __dp2a_lo(ldPair(p.pc, oc), cc.w, 0u);
+    if (kIn) {
+        oa += 4u * (uint32_t)p.w;
+        oc += 4u * (uint32_t)p.w;
+    } else {
+        oa = 4u * (uint32_t)(clampi(ya + 1, 0, p.h - 1) * p.w + ca.x);
+        oc = 4u * (uint32_t)(clampi(yc + 1, 0, p.h - 1) * p.w + cc.x);
+    }
+    const uint32_t a1 = __dp2a_lo(ldPair(p.pa, oa), ca.w, 0u), c1 = __dp2a_lo(ldPair(p.pc, oc), cc.w, 0u);
+    return __usad(a0 * (32u - fa) + a1 * fa, c0 * (32u - fc) + c1 * fc, 0u);
+}
+
+struct QfTile {
+    float2 bv[kQfBY][kQfBX];
+    int2 bR[kQfBY][kQfBX];                     // rne(32 v)
+    uint32_t above[kQfG + 1][2][kQfE];         // the errors of the 2 rows above each thread row (0: the apron's)
+    uint32_t below[kQfG + 1][2][kQfE];         // ... below thread row i - 1 (kQfG: the apron's)
+    alignas(16) uint32_t v[kQfTH][kQfVS];      // the vertical 5-sums
+    uint8_t pick[kQfTH][kQfE];
+};
+
+template <bool kIn>
+__device__ __forceinline__ void pixfieldQTile(const PixfieldParams& p, QfTile& t, int X0, int Y0) {
+    const int tid = threadIdx.x, ex = tid & (kQfE - 1), g = tid >> 6;
+    const int bx0 = (X0 >> 3) - 2, by0 = (Y0 >> 3) - 2;
+    // this thread's column; the columns and weights of cv2.resize x8 (weights (1, 0) beyond the borders)
+    const int qx = kIn ? X0 - kQfAp + ex : clampi(X0 - kQfAp + ex, 0, p.w - 1);
+    const int bx = (qx >> 3) - bx0;
+    int cx0;
+    float ca0, ca1;
+    {
+        const float f0 = __fsub_rn(__fmul_rn((float)qx + 0.5f, 0.125f), 0.5f);
+        const int s = (int)floorf(f0);
+        const bool edge = s < 0 || s >= p.bw - 1;
+        const float f = edge ? 0.0f : __fsub_rn(f0, (float)s);
+        cx0 = clampi(s, 0, p.bw - 1) - bx0;
+        ca0 = 1.0f - f;
+        ca1 = f;
+    }
+    // this thread's run: rows qy0 .. qy0 + 7 of block row br (rows past the frame repeat its last row below); its
+    // apron pixel: thread rows 0, 1 the 2 rows above the tile, 2, 3 the 2 below
+    const int qy0 = min(Y0 + 8 * g, p.h - 1), br = (qy0 >> 3) - by0;
+    const int ay = clampi(Y0 + (g < 2 ? g - 2 : kQfTH + g - 2), 0, p.h - 1), abr = (ay >> 3) - by0;
+    const int rows = p.h - qy0;   // rows of the run inside the frame, >= 1
+    // the bilinear block field in this column at region block row r (exact: dyadic values)
+    auto colField = [&](int r) {
+        return __ffma2_rn(t.bv[r][cx0 + 1], make_float2(ca1, ca1), pmul(t.bv[r][cx0], make_float2(ca0, ca0)));
+    };
+    // ... and at row qy of block row r: weights (2 (qy & 7) + 1) / 16 +- 1/2
+    auto rowField = [&](const float2& lo, const float2& mid, const float2& hi, int i) {
+        const float f = (float)(2 * i + 1) * 0.0625f + (i < 4 ? 0.5f : -0.5f);
+        const float2 a = i < 4 ? lo : mid, b = i < 4 ? mid : hi;
+        return __ffma2_rn(b, make_float2(f, f), pmul(a, make_float2(1.0f - f, 1.0f - f)));
+    };
+    const int r8 = tid & 31, c8 = (tid >> 5) * 8;   // the row run of the horizontal sums and the choice
+    float best[8];
+    int pk[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) { best[i] = FLT_MAX; pk[i] = 0; }
+    const uint32_t rowB = 4u * (uint32_t)p.w;
+    for (int k = 0; k < kQfNC; k++) {
+        uint32_t e[8], ea;   // the run's and the apron pixel's errors
+        if (k == 0) {   // the upsampled field: a vector per pixel
+            const float2 lo = colField(br - 1), mid = colField(br), hi = colField(br + 1);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float2 r = rne32bits(rowField(lo, mid, hi, j));
+                e[j] = qErr<kIn>(p, qx, qy0 + j, __float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
+            }
+            if (!kIn && (qy0 & 7)) {   // a run below the frame: its rows repeat row h - 1
+                const float2 r = rne32bits(rowField(lo, mid, hi, qy0 & 7));
+                e[0] = qErr<kIn>(p, qx, qy0, __float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
+            }
+            const float2 r = rne32bits(rowField(colField(abr - 1), colField(abr), colField(abr + 1), ay & 7));
+            ea = qErr<kIn>(p, qx, ay, __float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
+        } else if (k < kQfNC - 1) {   // the vector of the pixel's own block or of a 4-neighbour
+            const int dx = k == 4 ? -1 : (k == 5 ? 1 : 0), dy = k == 2 ? -1 : (k == 3 ? 1 : 0);
+            const int2 Ra = t.bR[abr + dy][bx + dx];
+            ea = qErr<kIn>(p, qx, ay, Ra.x, Ra.y);
+            const int2 R = t.bR[br + dy][bx + dx];
+            const QCol ca = qCol<kIn>(qx, -R.x, p.w), cc = qCol<kIn>(qx, R.x, p.w);
+            const uint32_t fa = (uint32_t)(-R.y) & 31u, fc = (uint32_t)R.y & 31u, ga = 32u - fa, gc = 32u - fc;
+            const int ya = qy0 + ((-R.y) >> 5), yc = qy0 + (R.y >> 5);
+            if (kIn || __all_sync(0xffffffffu, min(ya, yc) >= 0 && max(ya, yc) + 8 < p.h)) {
+                uint32_t oa = 4u * (uint32_t)(ya * p.w + ca.x), oc = 4u * (uint32_t)(yc * p.w + cc.x);
+                uint32_t ta = __dp2a_lo(ldPair(p.pa, oa), ca.w, 0u), tc = __dp2a_lo(ldPair(p.pc, oc), cc.w, 0u);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    oa += rowB;
+                    oc += rowB;
+                    const uint32_t ua = __dp2a_lo(ldPair(p.pa, oa), ca.w, 0u), uc = __dp2a_lo(ldPair(p.pc, oc), cc.w, 0u);
+                    e[j] = __usad(ta * ga + ua * fa, tc * gc + uc * fc, 0u);
+                    ta = ua;
+                    tc = uc;
+                }
+            } else {
+#pragma unroll 1
+                for (int j = 0; j < 8; j++) {
+                    const uint32_t v = qErr<kIn>(p, qx, qy0 + j, R.x, R.y);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) e[i] = i == j ? v : e[i];
+                }
+            }
+        } else {   // zero: the pixels themselves (weights 32 x 32)
+            auto err0 = [&](int y) {
+                const uint32_t o = 4u * (uint32_t)((kIn ? y : clampi(y, 0, p.h - 1)) * p.w + qx);
+                return __usad(ldPair(p.pa, o) & 0xFFFFu, ldPair(p.pc, o) & 0xFFFFu, 0u) << 10;
+            };
+#pragma unroll
+            for (int j = 0; j < 8; j++) e[j] = err0(qy0 + j);
+            ea = err0(ay);
+        }
+        if (!kIn && rows < 8) {   // the frame's last row stands for the rows below it
+#pragma unroll
+            for (int j = 1; j < 8; j++)
+                if (j >= rows) e[j] = e[j - 1];
+        }
+        // the vertical 5-sums of this run
+        t.below[g][0][ex] = e[0];
+        t.below[g][1][ex] = e[1];
+        t.above[g + 1][0][ex] = e[6];
+        t.above[g + 1][1][ex] = e[7];
+        if (g < 2) t.above[0][g][ex] = ea;
+        else t.below[kQfG][g - 2][ex] = ea;
+        __syncthreads();
+        const uint32_t a0 = t.above[g][0][ex], a1 = t.above[g][1][ex], b0 = t.below[g + 1][0][ex], b1 = t.below[g + 1][1][ex];
+        uint32_t S = a0 + a1 + e[0] + e[1] + e[2];
+        uint32_t* vo = &t.v[8 * g][ex];
+        vo[0] = S;
+        S += e[3] - a0; vo[kQfVS] = S;
+        S += e[4] - a1; vo[2 * kQfVS] = S;
+        S += e[5] - e[0]; vo[3 * kQfVS] = S;
+        S += e[6] - e[1]; vo[4 * kQfVS] = S;
+        S += e[7] - e[2]; vo[5 * kQfVS] = S;
+        S += b0 - e[3]; vo[6 * kQfVS] = S;
+        S += b1 - e[4]; vo[7 * kQfVS] = S;
+        __syncthreads();
+        // the horizontal 5-sums of a run of 8 output pixels, the cost (cv2's box scale with the 2^-14 units folded in,
+        // an exact scaling, in double as cv2), the running first minimum
+        const double C = 0x1p-14 * (1.0 / 25.0);
+        const float bonus = k == 0 ? p.smooth : (k == kQfNC - 1 ? p.zero : 0.0f);
+        uint32_t u[12];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const uint4 q = *reinterpret_cast<const uint4*>(&t.v[r8][c8 + 4 * i]);
+            u[4 * i] = q.x; u[4 * i + 1] = q.y; u[4 * i + 2] = q.z; u[4 * i + 3] = q.w;
+        }
+        uint32_t H = u[0] + u[1] + u[2] + u[3];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            H += u[i + 4];
+            const float c = __fsub_rn((float)(__dadd_rn(__hiloint2double(0x43300000, (int)H), -4503599627370496.0) * C), bonus);
+            if (c < best[i]) {
+                best[i] = c;
+                pk[i] = k;
+            }
+            H -= u[i];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) t.pick[r8][c8 + i] = (uint8_t)pk[i];
+    __syncthreads();
+    // the chosen candidate's vector
+    const int lx = ex - kQfAp;
+    if ((unsigned)lx >= (unsigned)kQfTW || X0 + lx >= p.w || Y0 + 8 * g >= p.h) return;
+    const float2 lo = colField(br - 1), mid = colField(br), hi = colField(br + 1);
+    float2* o = p.pf + (size_t)qy0 * p.w + X0 + lx;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        if (j >= rows) break;
+        const int k = t.pick[8 * g + j][lx];
+        float2 v = make_float2(0.0f, 0.0f);
+        if (k == 0) v = rowField(lo, mid, hi, j);
+        else if (k < kQfNC - 1) v = t.bv[br + (k == 2 ? -1 : (k == 3 ? 1 : 0))][bx + (k == 4 ? -1 : (k == 5 ? 1 : 0))];
+        o[(size_t)j * p.w] = v;
+    }
+}
+// CTA `cta` of an item: its tiles in raster order, then the CTAs that sum the leaves of the scene-cut mean, a warp each
+// (the sub-pixel launch before this one wrote the SADs)
+__device__ __forceinline__ void pixfieldQCta(const PixfieldParams& p, int cta) {
+    __shared__ QfTile t;
+    const int gx = (p.w + kQfTW - 1) / kQfTW, tiles = gx * ((p.h + kQfTH - 1) / kQfTH);
+    if (cta >= tiles) {
+        const int leaf = (cta - tiles) * 8 + (int)(threadIdx.x >> 5);
+        if (leaf < p.plan.nLeaves) cutMeanLeaf(p.plan, p.sads, p.bw * p.bh, p.cutSad, p.st, leaf, threadIdx.x & 31);
+        return;
+    }
+    const int X0 = cta % gx * kQfTW, Y0 = cta / gx * kQfTH;
+    // the block-field region, clamped to the field (a replicated entry stands for every block outside); the tile is
+    // interior if no vector of the region (nor any blend of them) takes a tap of the tile's pixels outside the frame
+    const int bx0 = (X0 >> 3) - 2, by0 = (Y0 >> 3) - 2;
+    bool out = false;
+    for (int i = threadIdx.x; i < kQfBX * kQfBY; i += 256) {
+        const float2 v = __ldg(p.v + clampi(by0 + i / kQfBX, 0, p.bh - 1) * p.bw + clampi(bx0 + i % kQfBX, 0, p.bw - 1));
+        t.bv[i / kQfBX][i % kQfBX] = v;
+        const float2 r = rne32bits(v);
+        const int2 R = make_int2(__float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
+        t.bR[i / kQfBX][i % kQfBX] = R;
+        const int dx = (abs(R.x) >> 5) + 2, dy = (abs(R.y) >> 5) + 2;
+        out |= X0 - kQfAp - dx < 0 || X0 + kQfTW + kQfAp + dx > p.w || Y0 - kQfAp - dy < 0 || Y0 + kQfTH + kQfAp + dy > p.h;
+    }
+    if (__syncthreads_or(out)) pixfieldQTile<false>(p, t, X0, Y0);
+    else pixfieldQTile<true>(p, t, X0, Y0);
+}
+__global__ void __launch_bounds__(256, 4) k_pixfield_q(const PixfieldParams p) {
+    pdlEnter();
+    pixfieldQCta(p, blockIdx.x);
+}
+__global__ void __launch_bounds__(256, 4) k_pixfield_q_m(const __grid_constant__ Merged<PixfieldParams> m) {
+    pdlEnter();
+    int bx, by;
+    const int i = mergedItem(m, bx, by);
+    pixfieldQCta(m.item[i], bx);
+}
+
+__global__ void __launch_bounds__(256) k_unpair(const uint32_t* pair, float* out, size_t n) {
+    pdlEnter();
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (i < n) out[i] = __fmul_rn(i2f((int)(__ldg(pair + i) & 0xFFFFu)), 1.0f / 16.0f);
+}
+
+// ============================================================================================== launchers
+cudaError_t launchUnpair(const uint32_t* pair, float* out, size_t n, cudaStream_t s) {
+    return launchPdl(k_unpair, dim3((unsigned int)((n + 255) / 256)), dim3(256), 0, s, pair, out, n);
+}
+cudaError_t launchSearchQ(const SearchParams& p, cudaStream_t s) {
+    const dim3 grid(divUp(p.bw, 4), p.bh);
+    if (p.R == 1) return launchPdl(p.pa ? k_search_q<1, true> : k_search_q<1, false>, grid, dim3(128), 0, s, p);
+    return launchPdl(p.pa ? k_search_q<2, true> : k_search_q<2, false>, grid, dim3(128), 0, s, p);
+}
+cudaError_t launchSearchQMerged(Merged<SearchParams>& m, cudaStream_t s) {
+    const int total = layoutMerged(m, [](const SearchParams& p, int& gx) {
+        gx = (int)divUp(p.bw, 4);
+        return gx * p.bh;
+    });
+    const bool pair = m.item[0].pa != nullptr;
+    if (m.item[0].R == 1) return launchPdl(pair ? k_search_q_m<1, true> : k_search_q_m<1, false>, dim3(total), dim3(128), 0, s, m);
+    return launchPdl(pair ? k_search_q_m<2, true> : k_search_q_m<2, false>, dim3(total), dim3(128), 0, s, m);
+}
+cudaError_t launchSubpixQ(const SubpixParams& p, cudaStream_t s) {
+    return launchPdl(k_subpix_q, dim3(divUp(p.bw, 4), p.bh), dim3(128), 0, s, p);
+}
+cudaError_t launchSubpixQMerged(Merged<SubpixParams>& m, cudaStream_t s) {
+    const int total = layoutMerged(m, [](const SubpixParams& p, int& gx) {
+        gx = (int)divUp(p.bw, 4);
+        return gx * p.bh;
+    });
+    return launchPdl(k_subpix_q_m, dim3(total), dim3(128), 0, s, m);
+}
+static int pixfieldQCtas(const PixfieldParams& p) {
+    return (int)(divUp(p.w, kQfTW) * divUp(p.h, kQfTH) + divUp(p.plan.nLeaves, 8));
+}
+cudaError_t launchPixfieldQ(const PixfieldParams& p, cudaStream_t s) {
+    return launchPdl(k_pixfield_q, dim3(pixfieldQCtas(p)), dim3(256), 0, s, p);
+}
+cudaError_t launchPixfieldQMerged(Merged<PixfieldParams>& m, cudaStream_t s) {
+    const int total = layoutMerged(m, [](const PixfieldParams& p, int& gx) { return gx = pixfieldQCtas(p); });
+    return launchPdl(k_pixfield_q_m, dim3(total), dim3(256), 0, s, m);
+}
+
+}  // namespace fgk

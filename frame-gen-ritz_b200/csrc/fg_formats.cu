@@ -225,13 +225,16 @@ __device__ __forceinline__ void lumaFmtCta(const LumaPyrParams& p, int bx, int b
             }
             va = __fmul_rn(i2f(rneDiv(4 * sa, n)), 1.0f / 16.0f);
             vc = __fmul_rn(i2f(rneDiv(4 * sc, n)), 1.0f / 16.0f);
-            p.la[0][(size_t)y * fw + x] = va;
-            p.lc[0][(size_t)y * fw + x] = vc;
+            if (p.la[0]) {
+                p.la[0][(size_t)y * fw + x] = va;
+                p.lc[0][(size_t)y * fw + x] = vc;
+            }
         }
         sl[0][i] = va;
         sl[1][i] = vc;
     }
     __syncthreads();
+    storePairs(p, sl, tx0, ty0);
     lumaTower<true>(p, sl, tx0, ty0);
 }
 template <int F>
@@ -1034,7 +1037,9 @@ __global__ void __launch_bounds__(64) k_ui_fill_fmt(const UiFillParams p) {
                 n++;
             }
         if (n > 0) {
-            (isC ? p.lc : p.la)[(size_t)cy * p.fw + cx] = __fmul_rn(i2f(rneDiv(4 * sum, n)), 1.0f / 16.0f);
+            const float v = __fmul_rn(i2f(rneDiv(4 * sum, n)), 1.0f / 16.0f);
+            (isC ? p.lc : p.la)[(size_t)cy * p.fw + cx] = v;
+            if (p.pa) storePairPx(isC ? p.pc : p.pa, p.fw, cx, cy, v);
             return;
         }
     }

@@ -22,7 +22,7 @@ namespace fgk {
 // below it, so the whole tower stays inside the tile. Mean of the valid pixels: sum * 1/n^2 when full, sum / count
 // at the frame's odd edges (cv2's INTER_AREA fast path).
 __device__ __forceinline__ void lumaPyrCta(const LumaPyrParams& p, int bx, int by) {
-    __shared__ float sl[2][kTowerFloats];
+    __shared__ __align__(8) float sl[2][kTowerFloats];
     const int tx0 = bx * 32, ty0 = by * 32;
     const int fw = p.lw[0], fh = p.lh[0], fs = p.fs;
     if (p.vec16 && tx0 + 32 <= fw && ty0 + 32 <= fh) {
@@ -43,11 +43,23 @@ __device__ __forceinline__ void lumaPyrCta(const LumaPyrParams& p, int bx, int b
             const int sc1 = gray8dp(c0.z, wlo, whi) + gray8dp(c0.w, wlo, whi) + gray8dp(c1.z, wlo, whi) + gray8dp(c1.w, wlo, whi);
             // sum * 0.25 (integer sums of 4 lumas: exact)
             const float2 va = make_float2(i2f(sa0) * 0.25f, i2f(sa1) * 0.25f), vc = make_float2(i2f(sc0) * 0.25f, i2f(sc1) * 0.25f);
-            *reinterpret_cast<float2*>(p.la[0] + (size_t)y * fw + tx0 + 2 * cg) = va;
-            *reinterpret_cast<float2*>(p.lc[0] + (size_t)y * fw + tx0 + 2 * cg) = vc;
-            sl[0][ly * 32 + 2 * cg] = va.x; sl[0][ly * 32 + 2 * cg + 1] = va.y;
-            sl[1][ly * 32 + 2 * cg] = vc.x; sl[1][ly * 32 + 2 * cg + 1] = vc.y;
+            const size_t px = (size_t)y * fw + tx0 + 2 * cg;
+            if (p.la[0]) {
+                *reinterpret_cast<float2*>(p.la[0] + px) = va;
+                *reinterpret_cast<float2*>(p.lc[0] + px) = vc;
+            }
+            *reinterpret_cast<float2*>(&sl[0][ly * 32 + 2 * cg]) = va;
+            *reinterpret_cast<float2*>(&sl[1][ly * 32 + 2 * cg]) = vc;
+            // the pair words (vec16 always has the planes): q = 16 x the mean; the right neighbour from the next lane,
+            // across the tile's right edge from the next tile, which writes that half itself (storePairs)
+            const uint32_t na = __shfl_down_sync(0xffffffffu, 4u * sa0, 1), nc = __shfl_down_sync(0xffffffffu, 4u * sc0, 1);
+            const bool last = tx0 + 2 * cg + 2 == fw;
+            storePairs2(p.pa + px, 4u * sa0, 4u * sa1, last ? 4u * sa1 : na, cg == 15 && !last, cg == 0 && tx0 > 0);
+            storePairs2(p.pc + px, 4u * sc0, 4u * sc1, last ? 4u * sc1 : nc, cg == 15 && !last, cg == 0 && tx0 > 0);
         }
+        __syncthreads();
+        lumaTower<false>(p, sl, tx0, ty0);
+        return;
     } else {
         for (int i = threadIdx.x; i < 1024; i += 256) {
             const int x = tx0 + (i & 31), y = ty0 + (i >> 5);
@@ -78,14 +90,17 @@ __device__ __forceinline__ void lumaPyrCta(const LumaPyrParams& p, int bx, int b
                     va = __fdiv_rn((float)sa, (float)n);
                     vc = __fdiv_rn((float)sc, (float)n);
                 }
-                p.la[0][(size_t)y * fw + x] = va;
-                p.lc[0][(size_t)y * fw + x] = vc;
+                if (p.la[0]) {
+                    p.la[0][(size_t)y * fw + x] = va;
+                    p.lc[0][(size_t)y * fw + x] = vc;
+                }
             }
             sl[0][i] = va;
             sl[1][i] = vc;
         }
     }
     __syncthreads();
+    if (p.pa) storePairs(p, sl, tx0, ty0);
     lumaTower<false>(p, sl, tx0, ty0);
 }
 __global__ void __launch_bounds__(256) k_luma_pyr(const LumaPyrParams p) {
@@ -698,87 +713,6 @@ __global__ void __launch_bounds__(256) k_cutmean(const CutMeanParams p) {
 // last leaf adds the inner nodes.
 constexpr int kSubT = 13, kSubO = 2, kSubL = 24, kSubRows = 10;   // tile, its margin, lattice side, tile rows used
 constexpr int kSubWarpFloats = 2 * kSubT * kSubT + 2 * kSubRows * kSubL + 72;
-
-// One leaf of the pairwise tree by one warp, in numpy's order: lanes 0..7 are its 8 accumulators (independent loads),
-// combined as ((r0 + r1) + (r2 + r3)) + ((r4 + r5) + (r6 + r7)), then the tail; leaves under 8 elements by lane 0
-// alone. Also returns (in every lane) the leaf's sum of roundEven(sad * 256), the debug counter's share.
-__device__ __forceinline__ float warpLeafSum(const float* a, int n, int lane, unsigned int& s256) {
-    unsigned int s = 0;
-    for (int i = lane; i < n; i += 32) s += (unsigned int)__float2int_rn(__fmul_rn(__ldcg(a + i), 256.0f));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    s256 = s;
-    float res = 0.0f;
-    if (n < 8) {
-        if (lane == 0)
-            for (int i = 0; i < n; i++) res = __fadd_rn(res, __ldcg(a + i));
-        return __shfl_sync(0xffffffffu, res, 0);
-    }
-    const int body = n - (n % 8);
-    float r = 0.0f;
-    if (lane < 8) {
-        r = __ldcg(a + lane);
-        for (int i = 8 + lane; i < body; i += 8) r = __fadd_rn(r, __ldcg(a + i));
-    }
-    const float r1 = __shfl_down_sync(0xffffffffu, r, 1);   // lane 2k: r[2k] + r[2k+1]
-    const float p2 = __fadd_rn(r, r1);
-    const float p2b = __shfl_down_sync(0xffffffffu, p2, 2);  // lane 4k: (r0 + r1) + (r2 + r3)
-    const float p4 = __fadd_rn(p2, p2b);
-    const float p4b = __shfl_down_sync(0xffffffffu, p4, 4);
-    if (lane == 0) {
-        res = __fadd_rn(p4, p4b);
-        for (int i = body; i < n; i++) res = __fadd_rn(res, __ldcg(a + i));
-    }
-    return __shfl_sync(0xffffffffu, res, 0);
-}
-
-// the scene-cut mean's share of the warp that wrote the SAD of block b (warp-uniform call)
-__device__ __forceinline__ void cutMeanShare(const SubpixParams& p, int b, int nb, int lane) {
-    const CutPlan& pl = p.plan;
-    const int leaf = pl.leafOf[b];
-    unsigned int old = 0;
-    if (lane == 0) {
-        __threadfence();   // this warp's SAD before its arrival
-        old = atomicAdd(pl.leafCnt + leaf, 1u);
-    }
-    old = __shfl_sync(0xffffffffu, old, 0);
-    const int2 lf = pl.leaves[leaf];
-    if (old != (unsigned int)lf.y - 1u) return;
-    __threadfence();
-    unsigned int s256;
-    const float v = warpLeafSum(p.sads + lf.x, lf.y, lane, s256);
-    unsigned int done = 0;
-    if (lane == 0) {
-        pl.gvals[leaf] = v;
-        pl.leafS256[leaf] = s256;
-        pl.leafCnt[leaf] = 0;
-        __threadfence();
-        done = atomicAdd(&p.st->subDone, 1u);
-    }
-    done = __shfl_sync(0xffffffffu, done, 0);
-    if (done != (unsigned int)pl.nLeaves - 1u) return;
-    // the last leaf: the inner nodes, one height per step, then the mean and the debug counter
-    __threadfence();
-    for (int d = 0; d < pl.nSteps; d++) {
-        for (int j = pl.depthStart[d] + lane; j < pl.depthStart[d + 1]; j += 32) {
-            const int2 c = pl.inner[j];
-            pl.gvals[pl.nLeaves + j] = __fadd_rn(__ldcg(pl.gvals + c.x), __ldcg(pl.gvals + c.y));
-        }
-        __threadfence_block();
-        __syncwarp();
-    }
-    unsigned int tot = 0;
-    for (int i = lane; i < pl.nLeaves; i += 32) tot += __ldcg(pl.leafS256 + i);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    if (lane == 0) {
-        const float mean = __fdiv_rn(__ldcg(pl.gvals + pl.root), (float)nb);
-        p.st->sadMean = mean;
-        p.st->cut = mean > p.cutSad ? 1u : 0u;
-        p.st->sadSum256 = tot;
-        p.st->subDone = 0;
-    }
-}
 
 __device__ __forceinline__ void subpixCta(const SubpixParams& p, int cta) {
     extern __shared__ float smem[];
@@ -1523,7 +1457,12 @@ static cudaError_t launchSearchR(const SearchParams& p, cudaStream_t s) {
     if (p.bw * p.bh <= kSearchLatBlocks) return launchPdl(k_search_r<R, true>, grid, dim3(128), smem, s, p);
     return launchPdl(k_search_r<R, false>, grid, dim3(128), smem, s, p);
 }
+// Searches on integer luma (fg_estimate_q.cu): radii 1 and 2 (a warp reduction per candidate, one lane each: at most 32)
+// at levels of more than kSearchLatBlocks blocks (k_search_r<2, false> 41.4 us, k_search_q<2> 28.6 us on a 4K frame's
+// level 0); wider radii keep k_search_r, whose lanes hold whole rows, and small levels its latency form.
+bool searchIsQ(const SearchParams& p) { return (p.pa || p.qscale > 0.0f) && p.R <= 2 && p.bw * p.bh > kSearchLatBlocks; }
 cudaError_t launchSearch(const SearchParams& p, cudaStream_t s) {
+    if (searchIsQ(p)) return launchSearchQ(p, s);
     switch (p.R) {
         case 1: return launchSearchR<1>(p, s);
         case 2: return launchSearchR<2>(p, s);
@@ -1546,19 +1485,6 @@ cudaError_t launchMedian3(const Median3Params& p, cudaStream_t s) {
     return launchPdl(k_median3, dim3(divUp(p.bw * p.bh, 256)), dim3(256), 0, s, p);
 }
 // ---- merged launches: the items' CTA ranges, then one launch (every item of m takes the same kernel variant)
-template <class P, class F>
-static int layoutMerged(Merged<P>& m, F ctasOf) {   // ctasOf(item, gx&) -> the item's CTA count
-    int total = 0;
-    for (int i = 0; i < m.n; i++) {
-        int gx = 1;
-        const int c = ctasOf(m.item[i], gx);
-        m.first[i] = total;
-        m.gx[i] = gx;
-        total += c;
-    }
-    m.first[m.n] = total;
-    return total;
-}
 cudaError_t launchLumaPyrMerged(Merged<LumaPyrParams>& m, cudaStream_t s) {
     if (m.n < 1 || m.n > kMergeMax) return cudaErrorInvalidValue;
     const int total = layoutMerged(m, [](const LumaPyrParams& p, int& gx) {
@@ -1568,6 +1494,7 @@ cudaError_t launchLumaPyrMerged(Merged<LumaPyrParams>& m, cudaStream_t s) {
     return launchPdl(k_luma_pyr_m, dim3(total), dim3(256), 0, s, m);
 }
 int searchVariant(const SearchParams& p) {
+    if (searchIsQ(p)) return 200 + 2 * p.R + (p.pa ? 1 : 0);
     if (p.R >= 1 && p.R <= 6) return 2 * p.R + (p.bw * p.bh <= kSearchLatBlocks ? 1 : 0);
     return 100 + p.R;
 }
@@ -1583,6 +1510,7 @@ cudaError_t launchSearchMerged(Merged<SearchParams>& m, cudaStream_t s) {
     const int v = searchVariant(m.item[0]);
     for (int i = 1; i < m.n; i++)
         if (searchVariant(m.item[i]) != v) return cudaErrorInvalidValue;
+    if (v >= 200) return launchSearchQMerged(m, s);
     const int total = layoutMerged(m, [](const SearchParams& p, int& gx) {
         gx = (int)divUp(p.bw * p.bh, 4);
         return gx;
@@ -1630,6 +1558,7 @@ cudaError_t launchMedian3Merged(Merged<Median3Params>& m, cudaStream_t s) {
 }
 cudaError_t launchSubpixMerged(Merged<SubpixParams>& m, cudaStream_t s) {
     if (m.n < 1 || m.n > kMergeMax) return cudaErrorInvalidValue;
+    if (m.item[0].pa) return launchSubpixQMerged(m, s);   // every item of a launch has pair planes, or none
     const int total = layoutMerged(m, [](const SubpixParams& p, int& gx) {
         gx = (int)divUp(p.bw * p.bh, 4);
         return gx;
@@ -1638,6 +1567,7 @@ cudaError_t launchSubpixMerged(Merged<SubpixParams>& m, cudaStream_t s) {
 }
 cudaError_t launchPixfieldMerged(Merged<PixfieldParams>& m, cudaStream_t s) {
     if (m.n < 1 || m.n > kMergeMax) return cudaErrorInvalidValue;
+    if (m.item[0].pa) return launchPixfieldQMerged(m, s);   // every item of a launch has pair planes, or none
     const int total = layoutMerged(m, [](const PixfieldParams& p, int& gx) {
         gx = (int)divUp(p.w, kPfTW);
         return gx * (int)divUp(p.h, kPfTH);
@@ -1676,6 +1606,7 @@ cudaError_t prepareKernels() {
     return e;
 }
 cudaError_t launchSubpix(const SubpixParams& p, cudaStream_t s) {
+    if (p.pa) return launchSubpixQ(p, s);
     const size_t smem = (size_t)4 * kSubWarpFloats * sizeof(float);
     return launchPdl(k_subpix, dim3(divUp(p.bw * p.bh, 4)), dim3(128), smem, s, p);
 }
@@ -1683,6 +1614,7 @@ cudaError_t launchCutMean(const CutMeanParams& p, cudaStream_t s) {
     return launchPdl(k_cutmean, dim3(1), dim3(256), planBytes(p.plan), s, p);
 }
 cudaError_t launchPixfield(const PixfieldParams& p, cudaStream_t s) {
+    if (p.pa) return launchPixfieldQ(p, s);
     return launchPdl(k_pixfield, dim3(divUp(p.w, kPfTW), divUp(p.h, kPfTH)), dim3(256), 0, s, p);
 }
 size_t synthSmemBytes(int fs) {  // declared in fg_params.h

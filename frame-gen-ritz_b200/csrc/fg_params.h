@@ -50,9 +50,12 @@ struct LumaPyrParams {
     int vec16;             // flowScale 2 with 16-byte aligned frames and rows: the uint4 path
     const float* pq;       // RgbaF16 linear: the PQ level (fmtPq255) of every half value, indexed by its bits, or null
     int lw[kPyrInKernel], lh[kPyrInKernel];
-    float* la[kPyrInKernel];
+    float* la[kPyrInKernel];   // [0] null: no pass reads level 0 as float
     float* lc[kPyrInKernel];
     FmtConst f;            // the luma kernel of the other formats (k_luma_fmt)
+    // level 0 again as pair planes, or null: word (x, y) = q(x) | q(min(x + 1, w - 1)) << 16 with q = 16 x luma, the two
+    // horizontal taps of a bilinear sample in one load (fg_estimate_q.cu)
+    uint32_t* pa; uint32_t* pc;
 };
 
 struct DownParams {         // one further pyramid level (INTER_AREA 0.5)
@@ -74,6 +77,10 @@ struct SearchParams {
     float2* out;
     float* sadOut;             // optional: the winner's SAD (finest level when sub-pixel refinement is off)
     const float* cnn;          // optional: the seed net's output at this level (kSeedNetOut floats per block)
+    // integer luma: the level's pair planes (LumaPyrParams; level 0), or la / lc as multiples of 1 / qscale, at most
+    // 2^23 of them; null and 0: float
+    const uint32_t* pa; const uint32_t* pc;
+    float qscale;
 };
 
 struct Median3Params {
@@ -104,10 +111,11 @@ struct SubpixParams {
     const float2* in; float2* out; float* sads;
     float2* out0;              // optional: the vectors after the 0.5 px step
     float pen[2][3];           // fl32(lambda * step * n), step 0.5 / 0.25, n = 0..2
-    // scene-cut mean in the last block
+    // the float kernel's share of the scene-cut mean
     CutPlan plan;
     float cutSad;
     DevState* st;
+    const uint32_t* pa; const uint32_t* pc;   // level 0's pair planes (LumaPyrParams), or null: the float kernel
 };
 
 struct CutMeanParams {         // the same scene-cut reduction as a separate pass (sub-pixel refinement off)
@@ -122,6 +130,12 @@ struct PixfieldParams {
     const float2* v; int bw, bh;   // the finest block field
     float smooth, zero;            // bonuses (interp.py:181-182)
     float2* pf;
+    const uint32_t* pa; const uint32_t* pc;   // level 0's pair planes (LumaPyrParams), or null: the float kernel
+    // on pair planes with sub-pixel refinement: the scene-cut mean of its SADs (plan.nLeaves 0: not here)
+    const float* sads;
+    CutPlan plan;
+    float cutSad;
+    DevState* st;
 };
 
 struct SynthParams {
@@ -229,6 +243,16 @@ cudaError_t launchSearchMerged(Merged<SearchParams>& m, cudaStream_t s);
 cudaError_t launchMedian3Merged(Merged<Median3Params>& m, cudaStream_t s);
 cudaError_t launchSubpixMerged(Merged<SubpixParams>& m, cudaStream_t s);
 cudaError_t launchPixfieldMerged(Merged<PixfieldParams>& m, cudaStream_t s);
+// the estimate's level-0 passes on the pair planes (fg_estimate_q.cu); the launchers above choose them
+bool searchIsQ(const SearchParams& p);
+// level 0 as float (n pixels of prev, then of curr) from the pair planes
+cudaError_t launchUnpair(const uint32_t* pair, float* out, size_t n, cudaStream_t s);
+cudaError_t launchSearchQ(const SearchParams& p, cudaStream_t s);
+cudaError_t launchSearchQMerged(Merged<SearchParams>& m, cudaStream_t s);
+cudaError_t launchSubpixQ(const SubpixParams& p, cudaStream_t s);
+cudaError_t launchSubpixQMerged(Merged<SubpixParams>& m, cudaStream_t s);
+cudaError_t launchPixfieldQ(const PixfieldParams& p, cudaStream_t s);
+cudaError_t launchPixfieldQMerged(Merged<PixfieldParams>& m, cudaStream_t s);
 // one pass of a motion blur, 8-bit RGBA frames: the main pass (fix = 0), then the fix-up (fix = 1)
 cudaError_t launchSynthBlur(const BlurParams& bp, int fix, cudaStream_t s);
 int synthBatchCtasPerSm(size_t smem);
@@ -292,6 +316,7 @@ struct UiFillParams {
     int W, H, ri, gi, bi, fs, fw, fh;
     const uint32_t* ma; const uint32_t* mc;
     float* la; float* lc;
+    uint32_t* pa; uint32_t* pc;    // the pair planes of level 0 (LumaPyrParams), or null
     int cx0, cy0, ncx, ncy;
     FmtConst f;                    // Rgb10 / RgbaF16 (launchUiFillFmt): the format's luma
     const float* pq;

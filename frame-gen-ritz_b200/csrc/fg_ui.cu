@@ -270,7 +270,9 @@ __global__ void __launch_bounds__(64) k_ui_v2_fill(const UiFillParams p) {
             }
         if (n > 0) {
             const int s2 = fs * fs;
-            (isC ? p.lc : p.la)[(size_t)cy * p.fw + cx] = (float)((2 * sum * s2 + n) / (2 * n)) / (float)s2;
+            const float v = (float)((2 * sum * s2 + n) / (2 * n)) / (float)s2;
+            (isC ? p.lc : p.la)[(size_t)cy * p.fw + cx] = v;
+            if (p.pa) storePairPx(isC ? p.pc : p.pa, p.fw, cx, cy, v);
             return;
         }
     }

@@ -225,6 +225,8 @@ struct Interpolator::Impl {
     float* luma = nullptr;
     float2* pqSeg = nullptr;  // linear RgbaF16: the PQ segment table of the synthesis
     float* pqTab = nullptr;   // linear RgbaF16: the PQ level of every half value (the luma pass looks them up)
+    bool lumaF0 = true;         // the latest estimate wrote level 0 as float too
+    uint32_t* pair = nullptr;   // level 0's pair planes (prev, then curr; fg_params.h LumaPyrParams), or null
     float2* field = nullptr;
     float* sads = nullptr;
     float2* pf = nullptr;
@@ -504,6 +506,10 @@ struct Interpolator::Impl {
         CutPlanHost P = buildCutPlan(nb0);
         size_t off = 0;
         auto take = [&](size_t bytes) { size_t o = off; off = alignUp(off + bytes, 256); return o; };
+        // level-0 luma is a multiple of 1/16 but for flowScale 4 cells of 3 px a side (means of 12, 9, 6, 3 px), whose
+        // estimates run the float kernels
+        const bool pairs = fmt != Format::Rgba8 || set.flowScale != 4 || (w % 4 != 3 && h % 4 != 3);
+        const size_t oPair = take(pairs ? (size_t)2 * L.fw * L.fh * 4 : 0);
         const size_t oLuma = take(L.lumaFloats * 4), oField = take(L.fieldF2 * 8), oSads = take((size_t)nb0 * 4);
         const size_t oPf = take((size_t)L.fw * L.fh * 8), oHist = take((size_t)2 * (2 * histB + 1) * 4);
         const size_t oSt = take(sizeof(fgk::DevState)), oEmap = take((size_t)((w + 3) & ~3u) * h);
@@ -519,6 +525,7 @@ struct Interpolator::Impl {
         arenaBytes = off;
         cudaMemset(arena, 0, off);
         luma = (float*)(arena + oLuma);
+        pair = pairs ? (uint32_t*)(arena + oPair) : nullptr;
         field = (float2*)(arena + oField);
         sads = (float*)(arena + oSads);
         pf = (float2*)(arena + oPf);
@@ -619,6 +626,8 @@ struct Interpolator::Impl {
         lp.nlev = std::min(e.top + 1, fgk::kPyrInKernel);
         lp.f = fc;
         lp.pq = pqTab;
+        lp.pa = pair;
+        lp.pc = pair ? pair + (size_t)L.fw * L.fh : nullptr;
         lp.vec16 = fmt == Format::Rgba8 && set.flowScale == 2 && prev.pitch % 16 == 0 && ((uintptr_t)prev.data & 15) == 0 && ((uintptr_t)curr.data & 15) == 0 &&
                    W % 4 == 0 && H % 2 == 0;   // complete 2x2 cells in every full tile, 8-byte aligned level-0 rows
         for (int l = 0; l < lp.nlev; l++) {
@@ -639,6 +648,10 @@ struct Interpolator::Impl {
             sp.w = l.w; sp.h = l.h; sp.bw = l.bw; sp.bh = l.bh;
             sp.top = i == n - 1 && snK < 0;
             sp.cnn = i == snK ? snOut : nullptr;
+            if (pair && i == 0) { sp.pa = lp.pa; sp.pc = lp.pc; }
+            // luma of level i is a multiple of 1 / (16 4^i), in the other formats of 2^-10 at most: the scale the sums
+            // of the integer search need to stay exact in float, up to level 3
+            if (pair && i <= 3) sp.qscale = (float)(16 << (2 * i));
             sp.R = (int)(sp.top ? set.searchRadiusTop : set.searchRadius);
             if (!sp.top && !sp.cnn) {
                 const Level& pl = L.lv[i + 1];
@@ -658,6 +671,9 @@ struct Interpolator::Impl {
             }
             mp.err = &st->err;
         }
+        // level 0 as float only for the passes that read it so: the float kernels, the estimate fill's pyramid rebuild, a
+        // seed net on level 0 (recordTrace makes it from the pair planes)
+        if (pair && !fill && snK != 0 && fgk::searchIsQ(e.search[0])) lp.la[0] = lp.lc[0] = nullptr;
         // 6. sub-pixel refinement + the scene-cut mean
         const Level& l0 = L.lv[0];
         const float2* vfin = field + l0.fM;
@@ -671,13 +687,15 @@ struct Interpolator::Impl {
             for (int p = 0; p < 2; p++)
                 for (int k = 0; k < 3; k++) sp.pen[p][k] = (float)((double)lam * (double)steps[p] * (double)k);
             sp.plan = plan; sp.cutSad = set.sceneCutSad; sp.st = st;
+            sp.pa = lp.pa; sp.pc = lp.pc;
             vfin = field + L.sub1;
         } else {
             e.cut = fgk::CutMeanParams{sads, l0.bw * l0.bh, plan, set.sceneCutSad, st};
         }
         // 8. per-pixel vector choice
         e.pix = fgk::PixfieldParams{luma + l0.lumaA, luma + l0.lumaC, l0.w, l0.h, vfin, l0.bw, l0.bh, set.smoothBonus,
-                                    set.hudBonus, pf};
+                                    set.hudBonus, pf, lp.pa, lp.pc, sads, fgk::CutPlan{}, set.sceneCutSad, st};
+        if (pair && set.subpixel) e.pix.plan = plan;
     }
 
     bool estimate(cudaStream_t s, const Frame& prev, const Frame& curr) {
@@ -686,6 +704,7 @@ struct Interpolator::Impl {
         const bool fill = fillMask[0] && fillMask[1];
         EstPlan e;
         planEstimate(prev, curr, fill, e);
+        lumaF0 = e.luma.la[0] != nullptr;
         const fgk::LumaPyrParams& lp = e.luma;
         if (!check(fmt == Format::Rgba8 ? fgk::launchLumaPyr(lp, s) : fgk::launchLumaFmt(lp, s))) return false;
         stamp(s, "luma");
@@ -696,6 +715,7 @@ struct Interpolator::Impl {
             fp.fw = L.lv[0].w; fp.fh = L.lv[0].h;
             fp.ma = fillMask[0]; fp.mc = fillMask[1];
             fp.la = luma + L.lv[0].lumaA; fp.lc = luma + L.lv[0].lumaC;
+            fp.pa = lp.pa; fp.pc = lp.pc;
             fp.cx0 = uiWork[0] / fp.fs; fp.cy0 = uiWork[1] / fp.fs;
             fp.ncx = (uiWork[0] + uiWork[2] - 1) / fp.fs - fp.cx0 + 1;
             fp.ncy = (uiWork[1] + uiWork[3] - 1) / fp.fs - fp.cy0 + 1;
@@ -1349,6 +1369,8 @@ bool Interpolator::recordTrace(cudaStream_t stream, void* dst) {
     DeviceGuard g(m->device);
     char* d = (char*)dst;
     const auto D2D = cudaMemcpyDeviceToDevice;
+    // an estimate that kept level 0 as pair planes only left its float form to this call
+    if (!m->lumaF0 && fgk::launchUnpair(m->pair, m->luma + m->L.lv[0].lumaA, (size_t)2 * l.fw * l.fh, stream) != cudaSuccess) return false;
     bool ok = cudaMemcpyAsync(d + l.lumaOff, m->luma, l.lumaBytes, D2D, stream) == cudaSuccess &&
               cudaMemcpyAsync(d + l.fieldOff, m->field, l.fieldBytes, D2D, stream) == cudaSuccess &&
               cudaMemcpyAsync(d + l.medOff, m->st->med, (size_t)l.nLevels * 8, D2D, stream) == cudaSuccess &&
@@ -1530,6 +1552,7 @@ bool Batch::Impl::mergedEstimates(cudaStream_t s, const Frame* prev, const Frame
         im.estSets++;
         im.haveEst = im.estUi = false;
         im.planEstimate(prev[i], curr[i], false, plans[j]);
+        im.lumaF0 = plans[j].luma.la[0] != nullptr;
         maxTop = std::max(maxTop, plans[j].top);
     }
     auto fail = [&](cudaError_t e) {
@@ -1569,15 +1592,19 @@ bool Batch::Impl::mergedEstimates(cudaStream_t s, const Frame* prev, const Frame
     }
     std::vector<fgk::SubpixParams> sub;
     std::vector<fgk::PixfieldParams> pix;
+    std::vector<int> subKeys, pixKeys;   // with pair planes or without
     for (int j = 0; j < ns; j++) {
         const int i = idx[j];
-        if (slots[i]->m->set.subpixel) sub.push_back(plans[j].sub);
-        else if (fail(fgk::launchCutMean(plans[j].cut, s))) return false;
+        if (slots[i]->m->set.subpixel) {
+            sub.push_back(plans[j].sub);
+            subKeys.push_back(plans[j].sub.pa != nullptr);
+        } else if (fail(fgk::launchCutMean(plans[j].cut, s))) return false;
         pix.push_back(plans[j].pix);
+        pixKeys.push_back(plans[j].pix.pa != nullptr);
     }
-    if (fail(launchMergedGroups(sub, std::vector<int>(sub.size(), 0),
+    if (fail(launchMergedGroups(sub, subKeys,
                                 [&](fgk::Merged<fgk::SubpixParams>& mg, int) { return fgk::launchSubpixMerged(mg, s); })) ||
-        fail(launchMergedGroups(pix, std::vector<int>(pix.size(), 0),
+        fail(launchMergedGroups(pix, pixKeys,
                                 [&](fgk::Merged<fgk::PixfieldParams>& mg, int) { return fgk::launchPixfieldMerged(mg, s); })))
         return false;
     for (int j = 0; j < ns; j++) {

@@ -261,7 +261,13 @@ __device__ __forceinline__ void storePairPx(uint32_t* plane, int fw, int x, int 
 
 // ============================================================================================== synthesis tile
 // 64 x 64 mismatch region -> 58 x 58 output tile: the square tile recomputes the least halo (1.22 region pixels per
-// output pixel, against 1.29 for 128 x 32) within the shared memory of 3 CTAs per SM
+// output pixel, against 1.29 for 128 x 32) within the shared memory of 3 CTAs per SM.
+//
+// The synthesis kernels are bound by instruction issue and by the latency of the sample loads (8-bit RGBA at 3840x2160,
+// t = 1/2: 74 % issue, 62 M warp instructions, 78 us in a graph; 91 us before the rows of a thread became consecutive with
+// the upsampled field in registers, interior tiles went without clamps, the row sums became byte dot products and fully
+// trusted warps only blend; t = 1/4 105 -> 88 us). Other shapes measured within 3 % of it (64 x 60 with 4 x 384 threads,
+// 64 x 72) or slower (64 x 40, 64 x 48).
 constexpr int kSyE = 64, kSyEH = 64, kSyAp = 3;
 constexpr int kSyT = kSyE - 2 * kSyAp, kSyTH = kSyEH - 2 * kSyAp;
 constexpr int kSyThreads = 512, kSyK = kSyEH / (kSyThreads / kSyE);   // region rows per thread (512 = 64 columns x 8)
@@ -274,7 +280,8 @@ __device__ __forceinline__ int syOutRow(int ey0, int k) { return ey0 * kSyK + k;
 constexpr int kSyES = kSyE + 4, kSyHS = kSyE + 2;
 
 // cv2.remap INTER_LINEAR / BORDER_REPLICATE of the 2-channel float field at (x, y): quantisation and weights paired
-// (exact), the taps' weighted sum as cv2 rounds it, ((p00 w00 + p01 w01) + p10 w10) + p11 w11 per channel
+// (exact), the taps' weighted sum as cv2 rounds it, ((p00 w00 + p01 w01) + p10 w10) + p11 w11 per channel (paired
+// products, scalar sums: never fused). One address where the four taps lie inside the field.
 __device__ __forceinline__ float2 remapF2m(const float2* __restrict__ F, int w, int h, float x, float y) {
     const float2 bits = rne32bits(make_float2(x, y));
     const int X = __float_as_int(bits.x) - 0x4B400000, Y = __float_as_int(bits.y) - 0x4B400000;
@@ -283,29 +290,43 @@ __device__ __forceinline__ float2 remapF2m(const float2* __restrict__ F, int w, 
     const float2 g = padd(make_float2(1.0f, 1.0f), make_float2(-f.x, -f.y));
     const float2 wA = pmul(make_float2(g.y, g.y), make_float2(g.x, f.x));   // (w00, w01)
     const float2 wB = pmul(make_float2(f.y, f.y), make_float2(g.x, f.x));   // (w10, w11)
-    const int x0 = clampi(ix, 0, w - 1), x1 = clampi(ix + 1, 0, w - 1);
-    const size_t r0 = (size_t)clampi(iy, 0, h - 1) * w, r1 = (size_t)clampi(iy + 1, 0, h - 1) * w;
-    const float2 p00 = __ldg(F + r0 + x0), p01 = __ldg(F + r0 + x1), p10 = __ldg(F + r1 + x0), p11 = __ldg(F + r1 + x1);
-    float2 r;
-    r.x = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(p00.x, wA.x), __fmul_rn(p01.x, wA.y)), __fmul_rn(p10.x, wB.x)), __fmul_rn(p11.x, wB.y));
-    r.y = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(p00.y, wA.x), __fmul_rn(p01.y, wA.y)), __fmul_rn(p10.y, wB.x)), __fmul_rn(p11.y, wB.y));
-    return r;
+    float2 p00, p01, p10, p11;
+    if ((unsigned)ix < (unsigned)(w - 1) && (unsigned)iy < (unsigned)(h - 1)) {
+        const float2* q = F + (iy * w + ix);
+        p00 = __ldg(q);
+        p01 = __ldg(q + 1);
+        p10 = __ldg(q + w);
+        p11 = __ldg(q + w + 1);
+    } else {
+        const int x0 = clampi(ix, 0, w - 1), x1 = clampi(ix + 1, 0, w - 1);
+        const size_t r0 = (size_t)clampi(iy, 0, h - 1) * w, r1 = (size_t)clampi(iy + 1, 0, h - 1) * w;
+        p00 = __ldg(F + r0 + x0); p01 = __ldg(F + r0 + x1); p10 = __ldg(F + r1 + x0); p11 = __ldg(F + r1 + x1);
+    }
+    const float2 m00 = pmul(p00, make_float2(wA.x, wA.x)), m01 = pmul(p01, make_float2(wA.y, wA.y));
+    const float2 m10 = pmul(p10, make_float2(wB.x, wB.x)), m11 = pmul(p11, make_float2(wB.y, wB.y));
+    return make_float2(__fadd_rn(__fadd_rn(__fadd_rn(m00.x, m01.x), m10.x), m11.x),
+                       __fadd_rn(__fadd_rn(__fadd_rn(m00.y, m01.y), m10.y), m11.y));
 }
 
 struct SyCoef {   // one region column (or row): upsampling taps (relative to the tile's field region) and weights
     int i0, i1;
     float a0, a1;   // rows: already x fs (scaling by a power of 2 commutes with the rounding)
     float pos;      // the clamped pixel coordinate
-    int pi;
 };
 
-__device__ __forceinline__ SyCoef syCoef(int e, int origin, int n, int un, int fn, int g0, float invfs, float wscale, bool xaxis) {
+// the clamped pixel of region column (or row) e, and cv2 resize's left tap and fraction of it, (d + 1/2) / fs - 1/2 in
+// units of 1 / (2 fs): s = floor, rem the remainder (d: the crop [:H, :W] / edge pad of the upsampled field)
+__device__ __forceinline__ int syPx(int e, int origin, int n) { return clampi(origin - kSyAp + e, 0, n - 1); }
+__device__ __forceinline__ int syTap(int p, int un, int fs, int sh, int& rem) {
+    const int num = 2 * min(p, un - 1) + 1 - fs;
+    rem = num & (2 * fs - 1);
+    return num >> sh;
+}
+__device__ __forceinline__ SyCoef syCoef(int e, int origin, int n, int un, int fn, int g0, int fs, float wscale, bool xaxis) {
     SyCoef c;
-    const int p = clampi(origin - kSyAp + e, 0, n - 1);
-    const int d = min(p, un - 1);   // crop [:H, :W] / edge pad of the upsampled field
-    float f = __fsub_rn(__fmul_rn((float)d + 0.5f, invfs), 0.5f);   // exact for fs = 1, 2, 4
-    int s = (int)floorf(f);
-    f = __fsub_rn(f, (float)s);
+    const int p = syPx(e, origin, n), sh = fs == 1 ? 1 : (fs == 2 ? 2 : 3);
+    int rem, s = syTap(p, un, fs, sh, rem);
+    float f = __fmul_rn(i2f(rem), fs == 1 ? 0.5f : (fs == 2 ? 0.25f : 0.125f));   // exact
     if (xaxis) {   // cv2 resize: x weights forced to (1, 0) beyond the borders; y rows clamped, weights kept
         if (s < 0) { s = 0; f = 0.0f; }
         if (s >= fn - 1) { s = fn - 1; f = 0.0f; }
@@ -315,35 +336,53 @@ __device__ __forceinline__ SyCoef syCoef(int e, int origin, int n, int un, int f
     c.a0 = __fmul_rn(1.0f - f, wscale);
     c.a1 = __fmul_rn(f, wscale);
     c.pos = (float)p;
-    c.pi = p;
     return c;
 }
 
-// Stages 0-1b of a synthesis tile, shared by the kernels of every format: the tile's field region, the row
-// coefficients (rowc) and this thread's column coefficients (returned); the field at t on the region (interp.field_at:
-// g <- pf(q - s g), twice, from g = pf(q)); the horizontal stage of its upsampling (cv2 resize: h = S0 a0 + S1 a1 per
-// row) into hrow. Carves the dynamic shared memory sm into the field region, hrow, the mismatch plane e and the row
-// sums hsum. Ends with a barrier.
-__device__ __forceinline__ SyCoef syFieldStage(const SynthParams& p, int X0, int Y0, int tid, int ex, int ey0, SyCoef* rowc,
-                                               int* gReg, unsigned char* sm, float2*& hrow, uint8_t*& e,
-                                               unsigned short*& hsum) {
-    const int fs = p.fs, uw = p.fw * fs, uh = p.fh * fs;
-    const float invfs = 1.0f / (float)fs, fsf = (float)fs;
-    if (tid == 0) {
-        const SyCoef lo = syCoef(0, X0, p.W, uw, p.fw, 0, invfs, 1.0f, true);
-        const SyCoef hi = syCoef(kSyE - 1, X0, p.W, uw, p.fw, 0, invfs, 1.0f, true);
-        const SyCoef rlo = syCoef(0, Y0, p.H, uh, p.fh, 0, invfs, 1.0f, false);
-        const SyCoef rhi = syCoef(kSyEH - 1, Y0, p.H, uh, p.fh, 0, invfs, 1.0f, false);
-        gReg[0] = lo.i0; gReg[1] = hi.i1 - lo.i0 + 1; gReg[2] = rlo.i0; gReg[3] = rhi.i1 - rlo.i0 + 1;
-    }
-    __syncthreads();
-    const int gx0 = gReg[0], GW = gReg[1], gy0 = gReg[2], GH = gReg[3];
-    if (tid < kSyEH) rowc[tid] = syCoef(tid, Y0, p.H, uh, p.fh, gy0, invfs, fsf, false);
-    const SyCoef cx = syCoef(ex, X0, p.W, uw, p.fw, gx0, invfs, 1.0f, true);
+// One region row of a synthesis tile: (upsampling taps i0 | i1 << 16 relative to the tile's field region, weights x fs,
+// the clamped pixel coordinate)
+__device__ __forceinline__ float4 syRow(const SyCoef& c) { return make_float4(__int_as_float(c.i0 | (c.i1 << 16)), c.a0, c.a1, c.pos); }
+
+// The field stage of a synthesis tile, shared by the kernels of every format: the tile's field region g (GW columns),
+// the row coefficients (rowc) and this thread's column coefficients; the field at t on the region (interp.field_at:
+// g <- pf(q - s g), twice, from g = pf(q)). Carves the dynamic shared memory sm into the field region, the mismatch
+// plane e and the row sums hsum. Ends with a barrier.
+//
+// `in` (uniform over the CTA): flowScale 2, no coordinate of the tile clamped, and no warp of the tile, whatever blend of
+// the region's vectors it takes, reaches within 2 px of the frame's border: the rows then follow a fixed pattern and
+// the samples need no clamps. On a 4K frame 92 % of the tiles.
+struct SyField {
+    const float2* g;
+    int GW, gx0;
+    SyCoef cx;
+    bool in;
+};
+__device__ __forceinline__ SyField syFieldStage(const SynthParams& p, int X0, int Y0, int tid, int ex, float4* rowc,
+                                                unsigned char* sm, uint8_t*& e, unsigned short*& hsum) {
+    const int fs = p.fs, uw = p.fw * fs, uh = p.fh * fs, sh = fs == 1 ? 1 : (fs == 2 ? 2 : 3);
+    int rem;
+    // the field region: from the first pixel's left tap to the last one's right tap (every thread, no barrier)
+    const int gx0 = clampi(syTap(syPx(0, X0, p.W), uw, fs, sh, rem), 0, p.fw - 1);
+    const int gy0 = clampi(syTap(syPx(0, Y0, p.H), uh, fs, sh, rem), 0, p.fh - 1);
+    const int GW = clampi(syTap(syPx(kSyE - 1, X0, p.W), uw, fs, sh, rem) + 1, 0, p.fw - 1) - gx0 + 1;
+    const int GH = clampi(syTap(syPx(kSyEH - 1, Y0, p.H), uh, fs, sh, rem) + 1, 0, p.fh - 1) - gy0 + 1;
+    const float fsf = (float)fs;
+    if (tid < kSyEH) rowc[tid] = syRow(syCoef(tid, Y0, p.H, uh, p.fh, gy0, fs, fsf, false));
+    SyField f;
+    f.cx = syCoef(ex, X0, p.W, uw, p.fw, gx0, fs, 1.0f, true);
     float2* g = reinterpret_cast<float2*>(sm);             // GH x GW
-    hrow = g + GW * GH;                                    // GH x kSyE
-    e = reinterpret_cast<uint8_t*>(hrow + GH * kSyE);      // kSyEH rows of kSyES bytes
+    f.g = g;
+    f.GW = GW;
+    f.gx0 = gx0;
+    e = reinterpret_cast<uint8_t*>(g + GW * GH);           // kSyEH rows of kSyES bytes
     hsum = reinterpret_cast<unsigned short*>(e + kSyEH * kSyES);   // kSyEH rows of kSyHS (columns < kSyT used)
+    // the room for |(2t) h|, |2(1 - t) h| (h: fs x a vector of the region) on each axis, negative where none is left
+    const float kf = p.mid ? fsf : __fmul_rn(fmaxf(p.ka, p.kc), fsf);
+    const int Ht = min(p.H, uh), Wt = min(p.W, uw);
+    const bool wide = fs != 2 || (uint64_t)p.H * (p.pitch >> 2) >= 0xF0000000u;
+    const float mx = wide ? -1.0f : (float)(min(X0 - kSyAp, Wt - (X0 - kSyAp + kSyE)) - 3);
+    const float my = wide ? -1.0f : (float)(min(Y0 - kSyAp, Ht - (Y0 - kSyAp + kSyEH)) - 3);
+    bool out = false;
     // the region's GW x GH samples spread over all threads (GW is about half the CTA's width at flowScale 2): row
     // r = floor((i + 0.5) / GW), exact in float for these sizes (the quotient stays >= 0.5 / GW from an integer)
     const float invGW = 1.0f / (float)GW;
@@ -357,38 +396,80 @@ __device__ __forceinline__ SyCoef syFieldStage(const SynthParams& p, int X0, int
             for (int it = 0; it < 2; it++)
                 v = remapF2m(p.pf, p.fw, p.fh, __fsub_rn(fx, __fmul_rn(p.s, v.x)), __fsub_rn(fy, __fmul_rn(p.s, v.y)));
         }
-        g[r * GW + c] = v;
+        g[i] = v;
+        out |= !(fabsf(v.x) * kf <= mx) || !(fabsf(v.y) * kf <= my);   // (a NaN is out too)
     }
-    __syncthreads();
-    for (int r = ey0; r < GH; r += kSyThreads / kSyE) {
-        const float2 s0 = g[r * GW + cx.i0], s1 = g[r * GW + cx.i1];
-        hrow[r * kSyE + ex] = make_float2(__fadd_rn(__fmul_rn(s0.x, cx.a0), __fmul_rn(s1.x, cx.a1)),
-                                          __fadd_rn(__fmul_rn(s0.y, cx.a0), __fmul_rn(s1.y, cx.a1)));
+    f.in = !__syncthreads_or(out);
+    return f;
+}
+
+// this thread's column of the horizontally upsampled field (cv2 resize: h = S0 a0 + S1 a1) at region row r
+__device__ __forceinline__ float2 syColField(const SyField& f, int r) {
+    const float2 s0 = f.g[r * f.GW + f.cx.i0], s1 = f.g[r * f.GW + f.cx.i1];
+    return make_float2(__fadd_rn(__fmul_rn(s0.x, f.cx.a0), __fmul_rn(s1.x, f.cx.a1)),
+                       __fadd_rn(__fmul_rn(s0.y, f.cx.a0), __fmul_rn(s1.y, f.cx.a1)));
+}
+// the vertical stage (x fs folded into the weights): the half-vector between two rows of it
+__device__ __forceinline__ float2 syLerp(float2 h0, float2 h1, float a0, float a1) {
+    return make_float2(__fadd_rn(__fmul_rn(h0.x, a0), __fmul_rn(h1.x, a1)), __fadd_rn(__fmul_rn(h0.y, a0), __fmul_rn(h1.y, a1)));
+}
+
+// Walks this thread's kSyK consecutive region rows (ey0 kSyK ..) top down and hands each to f(k, ey, posy, h). kIn (SyField
+// ::in): rows follow flowScale 2's pattern, the tile's first row odd: two rows share their pair of field rows, weights
+// (3/4, 1/4) and (1/4, 3/4) x 2. Else from the row coefficients, a field row loaded when the pair moves on. kRows rows
+// per loop round: the 8-bit kernels stay rolled (2) where many CTAs share an SM (a 4K synthesis at t = 1/2: 78 us rolled,
+// 83 us unrolled) and unroll (8) for grids of about one CTA per SM.
+template <bool kIn, int kRows, class F>
+__device__ __forceinline__ void syWalk(const SyField& f, const float4* rowc, int ey0, F&& fn) {
+    if (kIn) {
+        const float y0 = rowc[ey0 * kSyK].w;
+        float2 h0 = syColField(f, ey0 * (kSyK / 2));
+#pragma unroll (kRows / 2)
+        for (int k = 0; k < kSyK; k += 2) {
+            const float2 h1 = syColField(f, ey0 * (kSyK / 2) + k / 2 + 1);
+            fn(k, ey0 * kSyK + k, y0 + (float)k, syLerp(h0, h1, 1.5f, 0.5f));
+            fn(k + 1, ey0 * kSyK + k + 1, y0 + (float)(k + 1), syLerp(h0, h1, 0.5f, 1.5f));
+            h0 = h1;
+        }
+    } else {
+        int c0 = -1, c1 = -1;
+        float2 h0 = make_float2(0.0f, 0.0f), h1 = h0;
+#pragma unroll kRows
+        for (int k = 0; k < kSyK; k++) {
+            const float4 r = rowc[ey0 * kSyK + k];
+            const int i0 = __float_as_int(r.x) & 0xFFFF, i1 = __float_as_int(r.x) >> 16;
+            if (i0 != c0) {   // uniform over the warp
+                h0 = i0 == c1 ? h1 : syColField(f, i0);
+                c0 = i0;
+            }
+            if (i1 != c1) {
+                h1 = syColField(f, i1);
+                c1 = i1;
+            }
+            fn(k, ey0 * kSyK + k, r.w, syLerp(h0, h1, r.y, r.z));
+        }
     }
-    __syncthreads();
-    return cx;
 }
 
 // Stage 3 of a synthesis tile: the horizontal 7-sums of the mismatch plane, one region row and 8 output columns per
-// thread (a running window); the lanes of a warp take the 32 rows of one column group (conflict-free strides)
+// thread, as byte dot products with masks of ones (words w0 .. w3 hold columns c0 .. c0 + 15; the last group's columns
+// past the region belong to outputs that no one reads); the lanes of a warp take the 32 rows of one column group
+// (conflict-free strides)
 __device__ __forceinline__ void syRowSums(const uint8_t* e, unsigned short* hsum, int tid) {
     const int r = tid & (kSyEH - 1), c0 = (tid / kSyEH) * 8;
-    const uint8_t* q = e + r * kSyES + c0;
-    unsigned short* o = hsum + r * kSyHS + c0;
-    unsigned int sum = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6];
-    o[0] = (unsigned short)sum;
-#pragma unroll
-    for (int c = 1; c < 8; c++) {
-        if (c0 + c + 6 < kSyE) sum += q[c + 6] - q[c - 1];
-        o[c] = (unsigned short)sum;
-    }
-}
-
-// the half-vector of region row ey in this thread's column (vertical stage of the upsampling, x fs folded in)
-__device__ __forceinline__ float2 syHalfVec(const SyCoef& cy, const float2* hrow, int ex) {
-    const float2 h0 = hrow[cy.i0 * kSyE + ex], h1 = hrow[cy.i1 * kSyE + ex];
-    return make_float2(__fadd_rn(__fmul_rn(h0.x, cy.a0), __fmul_rn(h1.x, cy.a1)),
-                       __fadd_rn(__fmul_rn(h0.y, cy.a0), __fmul_rn(h1.y, cy.a1)));
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(e + r * kSyES + c0);
+    const bool more = c0 + 8 < kSyE;
+    const uint32_t w0 = q[0], w1 = q[1], w2 = more ? q[2] : 0u, w3 = more ? q[3] : 0u;
+    const uint32_t m1 = __dp4a(w1, 0x01010101u, 0u), m2 = __dp4a(w2, 0x01010101u, 0u);
+    const uint32_t s0 = __dp4a(w0, 0x01010101u, __dp4a(w1, 0x00010101u, 0u)), s1 = __dp4a(w0, 0x01010100u, m1);
+    const uint32_t s2 = __dp4a(w0, 0x01010000u, __dp4a(w2, 0x00000001u, m1)), s3 = __dp4a(w0, 0x01000000u, __dp4a(w2, 0x00000101u, m1));
+    const uint32_t s4 = __dp4a(w2, 0x00010101u, m1), s5 = __dp4a(w1, 0x01010100u, m2);
+    const uint32_t s6 = __dp4a(w1, 0x01010000u, __dp4a(w3, 0x00000001u, m2)), s7 = __dp4a(w1, 0x01000000u, __dp4a(w3, 0x00000101u, m2));
+    uint32_t* o = reinterpret_cast<uint32_t*>(hsum + r * kSyHS + c0);   // sums below 2^11: two per word
+    o[0] = s0 | (s1 << 16);
+    o[1] = s2 | (s3 << 16);
+    o[2] = s4 | (s5 << 16);
+    o[3] = s6 | (s7 << 16);
 }
 
 // ============================================================================================== scene-cut mean, spread

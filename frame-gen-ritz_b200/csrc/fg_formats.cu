@@ -12,8 +12,8 @@
 //     bilinear tap ((p00 w00 + p01 w01) + p10 w10) + p11 w11 in float, clamped to the edge; the mismatch, blend and
 //     stores of format.glsl / resolve.comp with a fixed operation order (round-to-nearest intrinsics, no fusion);
 //   - PQ (SMPTE ST 2084) via the log2 / exp2 series below, built from IEEE float operations only.
-// Synthesis tiles are the 8-bit path's (kSyE x kSyEH mismatch region, 3-pixel halo); the warps of the output
-// pixels are taken again after the 7x7 box instead of being held in registers (up to 3 floats per channel).
+// Synthesis tiles are the 8-bit path's (kSyE x kSyEH mismatch region, 3-pixel halo); the blend inputs of the output
+// pixels wait in shared memory for the 7x7 box.
 #include <cuda_fp16.h>
 
 #include "fg_device.h"
@@ -257,7 +257,7 @@ struct Taps {
 };
 
 // the texels and cv2's float weights of the sample point (X, Y) in 1/2^BITS texel units, clamped to w x h
-template <int BITS>
+template <int BITS, bool kIn = false>
 __device__ __forceinline__ Taps mkTaps(int X, int Y, int w, int h) {
     Taps t;
     constexpr int mask = (1 << BITS) - 1;
@@ -269,8 +269,8 @@ __device__ __forceinline__ Taps mkTaps(int X, int Y, int w, int h) {
     t.w01 = __fmul_rn(gy, fx);
     t.w10 = __fmul_rn(fy, gx);
     t.w11 = __fmul_rn(fy, fx);
-    t.x0 = clampi(ix, 0, w - 1); t.x1 = clampi(ix + 1, 0, w - 1);
-    t.y0 = clampi(iy, 0, h - 1); t.y1 = clampi(iy + 1, 0, h - 1);
+    t.x0 = kIn ? ix : clampi(ix, 0, w - 1); t.x1 = kIn ? ix + 1 : clampi(ix + 1, 0, w - 1);
+    t.y0 = kIn ? iy : clampi(iy, 0, h - 1); t.y1 = kIn ? iy + 1 : clampi(iy + 1, 0, h - 1);
     return t;
 }
 
@@ -287,18 +287,21 @@ __device__ __forceinline__ float bil(const Taps& t, float p00, float p01, float 
 // position is clamped to [0, 2^B (n - 1)] and the left tap is min(X >> B, n - 2) with the right weight X - 2^B ix: at
 // the right edge the taps (n - 2, n - 1) with weights (0, 2^B) give mkTaps' clamped (n - 1, n - 1) value, below zero
 // the taps (0, 1) with weights (2^B, 0) its (0, 0) value (frames are at least 16 x 16, so n >= 2).
+// kIn: the four taps are known to lie inside the plane (SyField::in): no clamps.
 struct ITaps {
     int x, y;                 // the top-left tap
     uint32_t w0, w1;          // 16-bit lanes: (w00, w01) and (w10, w11)
 };
-template <int B>
+template <int B, bool kIn>
 __device__ __forceinline__ ITaps mkITaps(int X, int Y, int w, int h) {
     constexpr int one = 1 << B;
-    X = clampi(X, 0, one * (w - 1));
-    Y = clampi(Y, 0, one * (h - 1));
     ITaps t;
-    t.x = min(X >> B, w - 2);
-    t.y = min(Y >> B, h - 2);
+    if (!kIn) {
+        X = clampi(X, 0, one * (w - 1));
+        Y = clampi(Y, 0, one * (h - 1));
+    }
+    t.x = kIn ? X >> B : min(X >> B, w - 2);
+    t.y = kIn ? Y >> B : min(Y >> B, h - 2);
     const uint32_t fx = (uint32_t)(X - one * t.x), fy = (uint32_t)(Y - one * t.y);
     const uint32_t wx = ((uint32_t)one - fx) | (fx << 16);   // lanes <= 2^B: the products below stay under 2^16
     t.w0 = wx * ((uint32_t)one - fy);
@@ -320,28 +323,27 @@ __device__ __noinline__ float2 warpChromaP010Off(const uint8_t* cbase, size_t cp
 }
 
 // the chroma (Cb, Cr) levels warped to the point whose 1/32-px coordinates are (X, Y)
-template <int F>
+template <int F, bool kIn>
 __device__ __forceinline__ float2 warpChroma(const uint8_t* cbase, size_t cpitch, int W, int H, int X, int Y) {
     if (F == kFmtNv12) {   // byte pairs (Cb, Cr): gathered as (Cb00, Cb01, Cr00, Cr01), two dp2a per channel, exact
-        const ITaps t = mkITaps<6>(X - 16, Y - 16, (W + 1) >> 1, (H + 1) >> 1);
+        const ITaps t = mkITaps<6, kIn>(X - 16, Y - 16, (W + 1) >> 1, (H + 1) >> 1);
         const unsigned short* q0 = reinterpret_cast<const unsigned short*>(cbase + (size_t)t.y * cpitch) + t.x;
         const unsigned short* q1 = reinterpret_cast<const unsigned short*>(cbase + (size_t)(t.y + 1) * cpitch) + t.x;
         const uint32_t c0 = __byte_perm((uint32_t)__ldg(q0), (uint32_t)__ldg(q0 + 1), 0x5140);
         const uint32_t c1 = __byte_perm((uint32_t)__ldg(q1), (uint32_t)__ldg(q1 + 1), 0x5140);
         const uint32_t cb = __dp2a_lo(t.w1, c1, __dp2a_lo(t.w0, c0, 0u)), cr = __dp2a_hi(t.w1, c1, __dp2a_hi(t.w0, c0, 0u));
-        return make_float2(__fmul_rn(i2f((int)cb), 0x1p-12f), __fmul_rn(i2f((int)cr), 0x1p-12f));
+        return make_float2(__fmul_rn((float)cb, 0x1p-12f), __fmul_rn((float)cr, 0x1p-12f));
     }
     if (F == kFmtP010) {   // 10-bit codes in the high bits of 16-bit samples: integer taps when the low 6 bits are zero
-        const ITaps t = mkITaps<6>(X - 16, Y - 16, (W + 1) >> 1, (H + 1) >> 1);
+        const ITaps t = mkITaps<6, kIn>(X - 16, Y - 16, (W + 1) >> 1, (H + 1) >> 1);
         const uint32_t* q0 = reinterpret_cast<const uint32_t*>(cbase + (size_t)t.y * cpitch) + t.x;
         const uint32_t* q1 = reinterpret_cast<const uint32_t*>(cbase + (size_t)(t.y + 1) * cpitch) + t.x;
         const uint32_t p00 = __ldg(q0), p01 = __ldg(q0 + 1), p10 = __ldg(q1), p11 = __ldg(q1 + 1);
         if (((p00 | p01 | p10 | p11) & 0x003F003Fu) == 0u) {   // codes x 64: every float step exact (ITaps)
             const uint32_t w00 = t.w0 & 0xFFFFu, w01 = t.w0 >> 16, w10 = t.w1 & 0xFFFFu, w11 = t.w1 >> 16;
-            const uint32_t cb = ((p00 >> 6) & 1023u) * w00 + ((p01 >> 6) & 1023u) * w01 + ((p10 >> 6) & 1023u) * w10 +
-                                ((p11 >> 6) & 1023u) * w11;
+            const uint32_t cb = ((p00 & 0xFFFFu) * w00 + (p01 & 0xFFFFu) * w01 + (p10 & 0xFFFFu) * w10 + (p11 & 0xFFFFu) * w11) >> 6;
             const uint32_t cr = (p00 >> 22) * w00 + (p01 >> 22) * w01 + (p10 >> 22) * w10 + (p11 >> 22) * w11;
-            return make_float2(__fmul_rn(i2f((int)cb), 0x1p-14f), __fmul_rn(i2f((int)cr), 0x1p-14f));
+            return make_float2(__fmul_rn((float)cb, 0x1p-14f), __fmul_rn((float)cr, 0x1p-14f));
         }
         return warpChromaP010Off(cbase, cpitch, W, H, X, Y);
     }
@@ -355,72 +357,57 @@ __device__ __noinline__ float warpYP010Off(const uint8_t* base, size_t pitch, in
     return bil(t, v(t.x0, t.y0), v(t.x1, t.y0), v(t.x0, t.y1), v(t.x1, t.y1));
 }
 
-// the warped sample at (px, py): Rgb10 RGB levels, F16 values, YUV (Y, Cb, Cr) levels
-template <int F>
-__device__ __forceinline__ void warp(const SynthParams& p, const uint8_t* base, const uint8_t* cbase, float px, float py,
-                                     float out[3]) {
-    const int X = rne32(px), Y = rne32(py);
+// the warped sample at the 1/32-px position (X, Y): Rgb10 levels (channels by bit position), F16 values, YUV (Y, Cb, Cr)
+// levels
+template <int F, bool kIn>
+__device__ __forceinline__ void warp(const SynthParams& p, const uint8_t* base, const uint8_t* cbase, int X, int Y, float out[3]) {
     if (F == kFmtRgb10) {   // 10-bit codes: integer taps, exact (ITaps)
-        const ITaps t = mkITaps<5>(X, Y, p.W, p.H);
+        const ITaps t = mkITaps<5, kIn>(X, Y, p.W, p.H);
         const uint32_t* q0 = reinterpret_cast<const uint32_t*>(base + (size_t)t.y * p.pitch) + t.x;
         const uint32_t* q1 = reinterpret_cast<const uint32_t*>(base + (size_t)(t.y + 1) * p.pitch) + t.x;
         const uint32_t p00 = __ldg(q0), p01 = __ldg(q0 + 1), p10 = __ldg(q1), p11 = __ldg(q1 + 1);
         const uint32_t w00 = t.w0 & 0xFFFFu, w01 = t.w0 >> 16, w10 = t.w1 & 0xFFFFu, w11 = t.w1 >> 16;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const int sh = p.f.rHigh ? 20 - 10 * k : 10 * k;
-            const uint32_t S = ((p00 >> sh) & 1023u) * w00 + ((p01 >> sh) & 1023u) * w01 + ((p10 >> sh) & 1023u) * w10 +
-                               ((p11 >> sh) & 1023u) * w11;
-            out[k] = __fmul_rn(__fmul_rn(i2f((int)S), 0x1p-10f), p.f.k10);
-        }
-        return;
-    }
-    if (F == kFmtNv12) {    // 8-bit luma: integer taps, two dp2a (as the 8-bit RGBA sampler), exact
-        const ITaps t = mkITaps<5>(X, Y, p.W, p.H);
+        // the middle field is weighted in place (30 bits); each sum times a power of two is exact in float
+        constexpr uint32_t M = 1023u, G = 1023u << 10;
+        const uint32_t s0 = (p00 & M) * w00 + (p01 & M) * w01 + (p10 & M) * w10 + (p11 & M) * w11;
+        const uint32_t s1 = (p00 & G) * w00 + (p01 & G) * w01 + (p10 & G) * w10 + (p11 & G) * w11;
+        const uint32_t s2 = ((p00 >> 20) & M) * w00 + ((p01 >> 20) & M) * w01 + ((p10 >> 20) & M) * w10 + ((p11 >> 20) & M) * w11;
+        out[0] = __fmul_rn(__fmul_rn((float)s0, 0x1p-10f), p.f.k10);
+        out[1] = __fmul_rn(__fmul_rn((float)s1, 0x1p-20f), p.f.k10);
+        out[2] = __fmul_rn(__fmul_rn((float)s2, 0x1p-10f), p.f.k10);
+    } else if (F == kFmtNv12) {    // 8-bit luma: integer taps, two dp2a (as the 8-bit RGBA sampler), exact
+        const ITaps t = mkITaps<5, kIn>(X, Y, p.W, p.H);
         const uint8_t* q0 = base + (size_t)t.y * p.pitch + t.x;
         const uint8_t* q1 = q0 + p.pitch;
         const uint32_t r0 = (uint32_t)__ldg(q0) | ((uint32_t)__ldg(q0 + 1) << 8);
         const uint32_t r1 = (uint32_t)__ldg(q1) | ((uint32_t)__ldg(q1 + 1) << 8);
-        out[0] = __fmul_rn(i2f((int)__dp2a_lo(t.w1, r1, __dp2a_lo(t.w0, r0, 0u))), 0x1p-10f);
-        const float2 c = warpChroma<F>(cbase, p.cpitch, p.W, p.H, X, Y);
+        out[0] = __fmul_rn((float)__dp2a_lo(t.w1, r1, __dp2a_lo(t.w0, r0, 0u)), 0x1p-10f);
+        const float2 c = warpChroma<F, kIn>(cbase, p.cpitch, p.W, p.H, X, Y);
         out[1] = c.x;
         out[2] = c.y;
-        return;
-    }
-    if (F == kFmtP010) {    // integer taps when the four samples' low 6 bits are zero (then every float step is exact)
-        const ITaps t = mkITaps<5>(X, Y, p.W, p.H);
+    } else if (F == kFmtP010) {    // integer taps when the four samples' low 6 bits are zero (then every float step is exact)
+        const ITaps t = mkITaps<5, kIn>(X, Y, p.W, p.H);
         const unsigned short* q0 = reinterpret_cast<const unsigned short*>(base + (size_t)t.y * p.pitch) + t.x;
         const unsigned short* q1 = reinterpret_cast<const unsigned short*>(base + (size_t)(t.y + 1) * p.pitch) + t.x;
         const uint32_t s00 = __ldg(q0), s01 = __ldg(q0 + 1), s10 = __ldg(q1), s11 = __ldg(q1 + 1);
-        if (((s00 | s01 | s10 | s11) & 63u) == 0u) {
-            const uint32_t S = (s00 >> 6) * (t.w0 & 0xFFFFu) + (s01 >> 6) * (t.w0 >> 16) + (s10 >> 6) * (t.w1 & 0xFFFFu) +
-                               (s11 >> 6) * (t.w1 >> 16);
-            out[0] = __fmul_rn(i2f((int)S), 0x1p-12f);   // codes / 4 = the levels
+        if (((s00 | s01 | s10 | s11) & 63u) == 0u) {   // codes x 64, weighted as they are (26 bits, 20 significant)
+            const uint32_t S = s00 * (t.w0 & 0xFFFFu) + s01 * (t.w0 >> 16) + s10 * (t.w1 & 0xFFFFu) + s11 * (t.w1 >> 16);
+            out[0] = __fmul_rn((float)S, 0x1p-18f);   // codes / 4 = the levels
         } else {
             out[0] = warpYP010Off(base, p.pitch, p.W, p.H, X, Y);
         }
-        const float2 c = warpChroma<F>(cbase, p.cpitch, p.W, p.H, X, Y);
-        out[1] = c.x;
-        out[2] = c.y;
-        return;
-    }
-    const Taps t = mkTaps<5>(X, Y, p.W, p.H);
-    float r00[3], r01[3], r10[3], r11[3];
-    texel<F>(p.f, base, p.pitch, t.x0, t.y0, r00);
-    texel<F>(p.f, base, p.pitch, t.x1, t.y0, r01);
-    texel<F>(p.f, base, p.pitch, t.x0, t.y1, r10);
-    texel<F>(p.f, base, p.pitch, t.x1, t.y1, r11);
-    if (F == kFmtNv12 || F == kFmtP010) {
-        out[0] = bil(t, r00[0], r01[0], r10[0], r11[0]);
-        const float2 c = warpChroma<F>(cbase, p.cpitch, p.W, p.H, X, Y);
+        const float2 c = warpChroma<F, kIn>(cbase, p.cpitch, p.W, p.H, X, Y);
         out[1] = c.x;
         out[2] = c.y;
     } else {
+        const Taps t = mkTaps<5, kIn>(X, Y, p.W, p.H);
+        float r00[3], r01[3], r10[3], r11[3];
+        texel<F>(p.f, base, p.pitch, t.x0, t.y0, r00);
+        texel<F>(p.f, base, p.pitch, t.x1, t.y0, r01);
+        texel<F>(p.f, base, p.pitch, t.x0, t.y1, r10);
+        texel<F>(p.f, base, p.pitch, t.x1, t.y1, r11);
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const float r = bil(t, r00[k], r01[k], r10[k], r11[k]);
-            out[k] = F == kFmtRgb10 ? __fmul_rn(r, p.f.k10) : r;
-        }
+        for (int k = 0; k < 3; k++) out[k] = bil(t, r00[k], r01[k], r10[k], r11[k]);
     }
 }
 
@@ -446,7 +433,7 @@ __device__ __forceinline__ int mismatch(const FmtConst& f, const float wa[3], co
             m = fmaxf(m, d);
         }
     }
-    return (int)fminf(m, 255.0f);
+    return floorPos(fminf(m, 255.0f));   // (a NaN takes the minimum's other operand)
 }
 
 // linear RgbaF16: the same from the segment table; false where the table leaves two integers possible
@@ -492,6 +479,17 @@ __device__ __forceinline__ void copyNear(const SynthParams& p, int x, int y) {
     }
 }
 
+// CTAs per SM a format's synthesis is compiled for, and region rows per loop round (syWalk), measured at 3840x2160, t = 1/2:
+// three CTAs (40 registers, rolled) are ahead of two (64 registers) where their shared memory fits and the taps are few
+// (Rgb10 129 against 143 us, P010 190 against 207); RgbaF16's table and blend planes leave room for two (211 -> 195),
+// and Nv12's 16 loads a pixel gain more from the registers (156 -> 152).
+__host__ __device__ constexpr int fmtCtas(int F) { return F == kFmtF16 || F == kFmtNv12 ? 2 : 3; }
+__host__ __device__ constexpr int fmtRows(int F) { return F == kFmtF16 ? 4 : (F == kFmtNv12 ? 8 : 2); }
+
+// compile-time flags of the synthesis tile's lambdas: the tile is inside the frame (SyField::in), or not known to be
+struct SyTrue { static constexpr bool value = true; };
+struct SyFalse { static constexpr bool value = false; };
+
 // ============================================================================================== synthesis
 // interp.synth for one t in the other formats: the 8-bit path's tile (k_synth) with each format's warp, mismatch,
 // blend and store (resolve.comp:48-83). YUV: the chroma of each 2x2 block is written with its even-even pixel, warped
@@ -508,9 +506,8 @@ __device__ __forceinline__ void copyNear(const SynthParams& p, int x, int y) {
 template <int F, bool kCut, bool kUi = false, class Sink>
 __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int by, Sink& sink) {
     extern __shared__ __align__(16) unsigned char sm[];
-    __shared__ SyCoef rowc[kSyEH];
+    __shared__ float4 rowc[kSyEH];
     __shared__ unsigned int cnt, nSlow;
-    __shared__ int gReg[4];
     const int X0 = bx * kSyT, Y0 = by * kSyTH;
     const int tid = threadIdx.x, ex = tid & (kSyE - 1), ey0 = tid / kSyE;
     if (kCut && p.st->cut) {   // scene cut (interp.py:225-226): the nearer real frame
@@ -521,12 +518,13 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
         return;
     }
     if (tid == 0) cnt = nSlow = 0;
-    float2* hrow;
     uint8_t* e;
     unsigned short* hsum;
-    const SyCoef cx = syFieldStage(p, X0, Y0, tid, ex, ey0, rowc, gReg, sm, hrow, e, hsum);
+    const SyField f = syFieldStage(p, X0, Y0, tid, ex, rowc, sm, e, hsum);
+    const SyCoef& cx = f.cx;
     const float kA = p.mid ? 1.0f : p.ka, kC = p.mid ? 1.0f : p.kc;
     constexpr bool kYuv = F == kFmtNv12 || F == kFmtP010;
+    constexpr int kRows = fmtRows(F);
     // the blend inputs m of the output pixels, kept from stage 2 for stage 4 (the warps are computed once): per channel
     // planes of kSyTH x kSyE floats (YUV: the luma plane, then the block-centre chroma (Cb, Cr) of the even-even
     // pixels, (kSyTH / 2) x (kSyE / 2))
@@ -543,14 +541,18 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
     }
     const int lx = ex - kSyAp, x = X0 + lx;
     // both warps of a region pixel (at pos, with half-vector h), the tap rejection applied
-    auto warps = [&](float posx, float posy, float2 h, float wa[3], float wc[3]) {
-        const float pax = __fsub_rn(posx, __fmul_rn(kA, h.x)), pay = __fsub_rn(posy, __fmul_rn(kA, h.y));
-        const float pcx = __fadd_rn(posx, __fmul_rn(kC, h.x)), pcy = __fadd_rn(posy, __fmul_rn(kC, h.y));
-        warp<F>(p, p.a, p.ac, pax, pay, wa);
-        warp<F>(p, p.c, p.cc, pcx, pcy, wc);
+    auto warps = [&](auto in, float posx, float posy, float2 h, float wa[3], float wc[3]) {
+        constexpr bool kIn = decltype(in)::value;
+        const float2 ha = pmul(h, make_float2(kA, kA)), hc = pmul(h, make_float2(kC, kC));
+        const float2 ba = rne32bits(make_float2(__fsub_rn(posx, ha.x), __fsub_rn(posy, ha.y)));
+        const float2 bc = rne32bits(make_float2(__fadd_rn(posx, hc.x), __fadd_rn(posy, hc.y)));
+        const int Xa = __float_as_int(ba.x) - 0x4B400000, Ya = __float_as_int(ba.y) - 0x4B400000;
+        const int Xc = __float_as_int(bc.x) - 0x4B400000, Yc = __float_as_int(bc.y) - 0x4B400000;
+        warp<F, kIn>(p, p.a, p.ac, Xa, Ya, wa);
+        warp<F, kIn>(p, p.c, p.cc, Xc, Yc, wc);
         if (kUi) {
-            const bool ha = p.uiA && (kYuv ? uiHitMaskYuv(p.uiA, rne32(pax), rne32(pay)) : uiHitMask(p.uiA, rne32(pax), rne32(pay)));
-            const bool hc = p.uiC && (kYuv ? uiHitMaskYuv(p.uiC, rne32(pcx), rne32(pcy)) : uiHitMask(p.uiC, rne32(pcx), rne32(pcy)));
+            const bool ha = p.uiA && (kYuv ? uiHitMaskYuv(p.uiA, Xa, Ya) : uiHitMask(p.uiA, Xa, Ya));
+            const bool hc = p.uiC && (kYuv ? uiHitMaskYuv(p.uiC, Xc, Yc) : uiHitMask(p.uiC, Xc, Yc));
             if (ha != hc) {
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
@@ -561,12 +563,10 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
         }
     };
     // 2. the mismatch over the region, and the blend inputs of the output pixels
-    for (int k = 0; k < kSyK; k++) {
-        const int ey = ey0 + (kSyThreads / kSyE) * k;
-        const SyCoef cy = rowc[ey];
-        const float2 h = syHalfVec(cy, hrow, ex);
+    auto stage2 = [&](auto in, int ey, float posy, float2 h) {
+        constexpr bool kIn = decltype(in)::value;
         float wa[3], wc[3];
-        warps(cx.pos, cy.pos, h, wa, wc);
+        warps(in, cx.pos, posy, h, wa, wc);
         if (pq) {
             int m;
             if (!mismatchPq(p.f, seg, wa, wc, m)) slow[atomicAdd(&nSlow, 1u)] = (unsigned short)(ey * kSyE + ex);
@@ -575,40 +575,44 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
             e[ey * kSyES + ex] = (uint8_t)mismatch<F>(p.f, wa, wc);
         }
         const int ly = ey - kSyAp;
-        if ((unsigned)ly < (unsigned)kSyTH) {   // warp-uniform
-            if (kYuv) {
-                mix[ly * kSyE + ex] = mixF(wa[0], wc[0], p);
-                if ((((lx | ly) & 1) == 0) && (unsigned)lx < (unsigned)kSyT && x < p.W && Y0 + ly < p.H) {
-                    // the chroma of this 2x2 block, warped from its centre with this pixel's half-vector
-                    const float bx = __fadd_rn(cx.pos, 0.5f), by = __fadd_rn(cy.pos, 0.5f);
-                    const float qax = __fsub_rn(bx, __fmul_rn(kA, h.x)), qay = __fsub_rn(by, __fmul_rn(kA, h.y));
-                    const float qcx = __fadd_rn(bx, __fmul_rn(kC, h.x)), qcy = __fadd_rn(by, __fmul_rn(kC, h.y));
-                    float2 ca = warpChroma<F>(p.ac, p.cpitch, p.W, p.H, rne32(qax), rne32(qay));
-                    float2 cc = warpChroma<F>(p.cc, p.cpitch, p.W, p.H, rne32(qcx), rne32(qcy));
-                    if (kUi) {   // uiRejectC: the block-centre taps, with their own footprints
-                        const bool ha = p.uiA && uiHitMaskYuv(p.uiA, rne32(qax), rne32(qay));
-                        const bool hc = p.uiC && uiHitMaskYuv(p.uiC, rne32(qcx), rne32(qcy));
-                        if (ha != hc) {
-                            if (ha) ca = cc;
-                            else cc = ca;
-                        }
+        if ((unsigned)ly >= (unsigned)kSyTH) return;   // warp-uniform
+        if (kYuv) {
+            mix[ly * kSyE + ex] = mixF(wa[0], wc[0], p);
+            if ((((lx | ly) & 1) == 0) && (unsigned)lx < (unsigned)kSyT && x < p.W && Y0 + ly < p.H) {
+                // the chroma of this 2x2 block, warped from its centre with this pixel's half-vector
+                const float bx = __fadd_rn(cx.pos, 0.5f), by = __fadd_rn(posy, 0.5f);
+                const float qax = __fsub_rn(bx, __fmul_rn(kA, h.x)), qay = __fsub_rn(by, __fmul_rn(kA, h.y));
+                const float qcx = __fadd_rn(bx, __fmul_rn(kC, h.x)), qcy = __fadd_rn(by, __fmul_rn(kC, h.y));
+                float2 ca = warpChroma<F, kIn>(p.ac, p.cpitch, p.W, p.H, rne32(qax), rne32(qay));
+                float2 cc = warpChroma<F, kIn>(p.cc, p.cpitch, p.W, p.H, rne32(qcx), rne32(qcy));
+                if (kUi) {   // uiRejectC: the block-centre taps, with their own footprints
+                    const bool ha = p.uiA && uiHitMaskYuv(p.uiA, rne32(qax), rne32(qay));
+                    const bool hc = p.uiC && uiHitMaskYuv(p.uiC, rne32(qcx), rne32(qcy));
+                    if (ha != hc) {
+                        if (ha) ca = cc;
+                        else cc = ca;
                     }
-                    mixc[(ly >> 1) * (kSyE / 2) + (lx >> 1)] = make_float2(mixF(ca.x, cc.x, p), mixF(ca.y, cc.y, p));
                 }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 3; c++) mix[(c * kSyTH + ly) * kSyE + ex] = mixF(wa[c], wc[c], p);
+                mixc[(ly >> 1) * (kSyE / 2) + (lx >> 1)] = make_float2(mixF(ca.x, cc.x, p), mixF(ca.y, cc.y, p));
             }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; c++) mix[(c * kSyTH + ly) * kSyE + ex] = mixF(wa[c], wc[c], p);
         }
-    }
+    };
+    if (!kUi && f.in) syWalk<true, kRows>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) { stage2(SyTrue(), ey, posy, h); });
+    else syWalk<false, kRows>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) { stage2(SyFalse(), ey, posy, h); });
     __syncthreads();
     if (pq) {   // the undecided pixels (about 1.6 % on natural content), dealt out over all threads: warped again, exact
         const int n = (int)nSlow;
         for (int i = tid; i < n; i += kSyThreads) {
             const int sx = slow[i] & (kSyE - 1), sy = slow[i] / kSyE;
-            const SyCoef cy = rowc[sy];
+            const float4 r = rowc[sy];
+            SyField fc = f;
+            fc.cx = syCoef(sx, X0, p.W, p.fw * p.fs, p.fw, f.gx0, p.fs, 1.0f, true);
+            const float2 h = syLerp(syColField(fc, __float_as_int(r.x) & 0xFFFF), syColField(fc, __float_as_int(r.x) >> 16), r.y, r.z);
             float wa[3], wc[3];
-            warps((float)clampi(X0 - kSyAp + sx, 0, p.W - 1), cy.pos, syHalfVec(cy, hrow, sx), wa, wc);
+            warps(SyFalse(), fc.cx.pos, r.w, h, wa, wc);
             e[sy * kSyES + sx] = (uint8_t)mismatch<F>(p.f, wa, wc);
         }
         __syncthreads();
@@ -620,12 +624,13 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
     unsigned int myCnt = 0;
     if ((unsigned)lx < (unsigned)kSyT && x < p.W) {
         const uint8_t* nearF = p.nearC ? p.c : p.a;
+        const unsigned short* q = hsum + syOutRow(ey0, 0) * kSyHS + lx;
+        int S = q[0] + q[kSyHS] + q[2 * kSyHS] + q[3 * kSyHS] + q[4 * kSyHS] + q[5 * kSyHS];
 #pragma unroll
         for (int k = 0; k < kSyK; k++) {
-            const int ey = ey0 + (kSyThreads / kSyE) * k, ly = ey - kSyAp, y = Y0 + ly;
-            if ((unsigned)ly >= (unsigned)kSyTH || y >= p.H) continue;
-            const unsigned short* q = hsum + ly * kSyHS + lx;
-            const int S = q[0] + q[kSyHS] + q[2 * kSyHS] + q[3 * kSyHS] + q[4 * kSyHS] + q[5 * kSyHS] + q[6 * kSyHS];
+            const int ly = syOutRow(ey0, k), y = Y0 + ly;
+            if (ly >= kSyTH || y >= p.H) break;   // uniform over the warp; later rows are out too
+            S += q[(k + 6) * kSyHS] - (k ? q[(k - 1) * kSyHS] : 0);
             float u, iu;
             if (S <= p.sZero) {          // the ramp is exactly 0 (host-derived threshold)
                 u = 0.0f;
@@ -644,10 +649,10 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
                 uint32_t ow = nw & 0xC0000000u;
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
-                    const float nl = __fmul_rn(i2f(rgb10(p.f, nw, c)), p.f.k10);
+                    const float nl = __fmul_rn(i2f((int)((nw >> (10 * c)) & 1023u)), p.f.k10);
                     const float v = clampF(blendM(mix[(c * kSyTH + ly) * kSyE + ex], nl, u, iu), 0.0f, 255.0f);
                     const int code = clampi((int)floorf(__fadd_rn(__fmul_rn(v, p.f.k10i), 0.5f)), 0, 1023);
-                    ow |= (uint32_t)code << (p.f.rHigh ? 20 - 10 * c : 10 * c);
+                    ow |= (uint32_t)code << (10 * c);
                 }
                 sink.word(k, x, y, ow);
             } else if (F == kFmtF16) {
@@ -672,7 +677,7 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
                     sink.chroma(k, x, y, cb, cr);
                 }
             }
-            if (p.emap) p.emap[(size_t)y * ((p.W + 3) & ~3) + x] = e[ey * kSyES + ex];
+            if (p.emap) p.emap[(size_t)y * ((p.W + 3) & ~3) + x] = e[(ly + kSyAp) * kSyES + ex];
         }
     }
     if (myCnt) atomicAdd(&cnt, myCnt);
@@ -703,14 +708,14 @@ struct FmtStore {
 };
 
 template <int F>
-__global__ void __launch_bounds__(kSyThreads, 3) k_synth_fmt(const SynthParams p) {
+__global__ void __launch_bounds__(kSyThreads, fmtCtas(F)) k_synth_fmt(const SynthParams p) {
     pdlEnter();
     FmtStore<F> store{p};
     synthFmtTile<F, true>(p, blockIdx.x, blockIdx.y, store);
 }
 // the same with CrosshairV2's tap rejection (Rgb10 / RgbaF16); a separate kernel so the plain one is unchanged
 template <int F>
-__global__ void __launch_bounds__(kSyThreads, 3) k_synth_fmt_ui(const SynthParams p) {
+__global__ void __launch_bounds__(kSyThreads, fmtCtas(F)) k_synth_fmt_ui(const SynthParams p) {
     pdlEnter();
     FmtStore<F> store{p};
     synthFmtTile<F, true, true>(p, blockIdx.x, blockIdx.y, store);
@@ -720,7 +725,7 @@ __global__ void __launch_bounds__(kSyThreads, 3) k_synth_fmt_ui(const SynthParam
 // tile of the work list from an atomic counter until the list is exhausted; an item's parameters are staged in shared
 // memory per tile.
 template <int F>
-__global__ void __launch_bounds__(kSyThreads, 3) k_synth_fmt_batch(const SynthBatchArgs b) {
+__global__ void __launch_bounds__(kSyThreads, fmtCtas(F)) k_synth_fmt_batch(const SynthBatchArgs b) {
     pdlEnter();
     __shared__ int work, item;
     __shared__ __align__(16) SynthParams sp;
@@ -849,8 +854,8 @@ __global__ void __launch_bounds__(kSyThreads, 1) k_synth_blur_fmt(const BlurPara
             if (colOk) {
 #pragma unroll
                 for (int k = 0; k < kSyK; k++) {
-                    const int ly = ey0 + (kSyThreads / kSyE) * k - kSyAp, y = blockIdx.y * kSyTH + ly;
-                    if ((unsigned)ly < (unsigned)kSyTH && y < b.H) frameValues<F>(b, nc ? b.c : b.a, nc ? b.cc : b.ac, k, x, y, acc);
+                    const int ly = syOutRow(ey0, k), y = blockIdx.y * kSyTH + ly;
+                    if (ly < kSyTH && y < b.H) frameValues<F>(b, nc ? b.c : b.a, nc ? b.cc : b.ac, k, x, y, acc);
                 }
             }
             continue;
@@ -874,8 +879,8 @@ __global__ void __launch_bounds__(kSyThreads, 1) k_synth_blur_fmt(const BlurPara
     const uint32_t wap = sWap, wac = 65536u - wap;
 #pragma unroll
     for (int k = 0; k < kSyK; k++) {
-        const int ly = ey0 + (kSyThreads / kSyE) * k - kSyAp, y = blockIdx.y * kSyTH + ly;
-        if ((unsigned)ly >= (unsigned)kSyTH || y >= b.H) continue;
+        const int ly = syOutRow(ey0, k), y = blockIdx.y * kSyTH + ly;
+        if (ly >= kSyTH || y >= b.H) break;
         uint8_t* orow = b.out + (size_t)y * b.outPitch;
         if (F == kFmtRgb10) {
             const uint32_t pa = ldw(b.a, b.pitch, x, y) >> 30, pc = ldw(b.c, b.pitch, x, y) >> 30;

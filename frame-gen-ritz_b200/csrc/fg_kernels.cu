@@ -1096,15 +1096,14 @@ __global__ void __launch_bounds__(256) k_pixfield_m(const __grid_constant__ Merg
 // t = 0.5 blend use byte-SIMD instructions.
 
 // one cv2.remap INTER_LINEAR / BORDER_REPLICATE sample of a 4-byte-per-pixel 8-bit frame of at least 2 x 2 pixels
-// at the position whose rne32 bits are (bx, by): channels 0..2 of the result (byte 3 = 0; also unpacked in ch).
+// at the position whose rne32 bits are (bx, by): channels 0..2 of the result (byte 3 = 0).
 // Borders: the 1/32-pixel position is clamped to [0, 32 (W - 1)], the left tap is min(X >> 5, W - 2) and the right
 // weight X - 32 ix (0..32): at the right edge the taps (W - 2, W - 1) with weights (0, 32), the same products as cv2's
 // (W - 1, W - 1) pair, so the four taps are always (ix, iy) + {0, 1}^2 (one address, fixed offsets). Filter: cv2's
 // 15-bit weights of 5-bit bilinear fractions are 32 wx wy, and (sum p 32 wx wy + 2^14) >> 15 == (sum p wx wy + 512) >> 10
 // with wx wy <= 1024; per channel two 16-bit x 8-bit dot products (dp2a) on tap bytes gathered by byte permutes, exact
 // in 32 bits.
-__device__ __forceinline__ uint32_t sampleU8(const uint32_t* __restrict__ img, uint32_t pw, int W, int H, float bxf, float byf,
-                                             int ch[3]) {
+__device__ __forceinline__ uint32_t sampleU8(const uint32_t* __restrict__ img, uint32_t pw, int W, int H, float bxf, float byf) {
     const int X = clampi(__float_as_int(bxf) - 0x4B400000, 0, 32 * (W - 1));
     const int Y = clampi(__float_as_int(byf) - 0x4B400000, 0, 32 * (H - 1));
     const int ix = min(X >> 5, W - 2), iy = min(Y >> 5, H - 2);
@@ -1118,24 +1117,42 @@ __device__ __forceinline__ uint32_t sampleU8(const uint32_t* __restrict__ img, u
     const uint32_t c0 = __dp2a_lo(w1, rg1, __dp2a_lo(w0, rg0, 512u)) >> 10;
     const uint32_t c1 = __dp2a_hi(w1, rg1, __dp2a_hi(w0, rg0, 512u)) >> 10;
     const uint32_t c2 = __dp2a_hi(w1, b1, __dp2a_lo(w0, b0, 512u)) >> 10;
-    ch[0] = (int)c0;
-    ch[1] = (int)c1;
-    ch[2] = (int)c2;
     return c2 * 65536u + (c1 * 256u + c0);
 }
 
-// one output tile (bx, by) of one synthesis; all threads of the CTA take part. Each output pixel goes to
-// sink(k, x, y, ly, o): k = this thread's region-row slot, (x, y) the pixel, ly its tile row, o the packed result
-// (alpha = the nearer frame's). The untrusted count is added to *p.untrusted unless that is null. kCut: under a scene
-// cut the tile is a copy of the nearer frame to p.out (and the core returns at once); without kCut the caller has
-// taken the cut into account.
-template <bool kCut, bool kUi = false, class Sink>
-__device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int by, Sink&& sink) {
+// the same inside the frame by at least 2 px (SyField::in): no clamps; the rne32 bits are those of integers in [0, 2^22)
+__device__ __forceinline__ uint32_t sampleU8In(const uint32_t* __restrict__ img, uint32_t pw, float bxf, float byf) {
+    const uint32_t X = __float_as_uint(bxf), Y = __float_as_uint(byf);   // 0x4B400000 + the 1/32-px position
+    const uint32_t fx = X & 31u, fy = Y & 31u;
+    const uint32_t* q = img + (((Y >> 5) - 0x25A0000u) * pw + ((X >> 5) - 0x25A0000u));
+    const uint32_t p00 = __ldg(q), p01 = __ldg(q + 1), p10 = __ldg(q + pw), p11 = __ldg(q + pw + 1);
+    const uint32_t wx = fx * 65535u + 32u;                  // (32 - fx) | fx << 16
+    const uint32_t w0 = wx * (32u - fy), w1 = wx * fy;
+    const uint32_t rg0 = __byte_perm(p00, p01, 0x5140), rg1 = __byte_perm(p10, p11, 0x5140);
+    const uint32_t b0 = __byte_perm(p00, p01, 0x0062), b1 = __byte_perm(p10, p11, 0x6200);
+    const uint32_t c0 = __dp2a_lo(w1, rg1, __dp2a_lo(w0, rg0, 512u)) >> 10;
+    const uint32_t c1 = __dp2a_hi(w1, rg1, __dp2a_hi(w0, rg0, 512u)) >> 10;
+    const uint32_t c2 = __dp2a_hi(w1, b1, __dp2a_lo(w0, b0, 512u)) >> 10;
+    return c2 * 65536u + (c1 * 256u + c0);
+}
+
+// the largest of the 3 channel differences of two packed samples (byte 3 zero in both)
+__device__ __forceinline__ uint32_t maxDiffU8(uint32_t a, uint32_t c) {
+    const uint32_t d = __vabsdiffu4(a, c);
+    return max(max(d & 255u, (d >> 8) & 255u), d >> 16);
+}
+
+// one output tile (bx, by) of one synthesis; all threads of the CTA take part. Each thread hands its output pixels, a
+// column of up to kSyK rows, to the sink: begin(x, y0) (their first pixel), then put(k, o) per row k = 0, 1, .. (o packed,
+// alpha = the nearer frame's). The untrusted count is added to *p.untrusted unless that is null. kCut: under a scene cut
+// the tile is a copy of the nearer frame to p.out (and the core returns at once); without kCut the caller has taken the
+// cut into account. kLat: the unrolled form for grids of about one CTA per SM.
+template <bool kCut, bool kUi, bool kLat, class Sink>
+__device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int by, Sink& sink) {
     extern __shared__ __align__(16) unsigned char sm[];
-    __shared__ SyCoef rowc[kSyEH];
+    __shared__ float4 rowc[kSyEH];
     __shared__ float TA[256], TC[256];
     __shared__ unsigned int cnt;
-    __shared__ int gReg[4];
     const int X0 = bx * kSyT, Y0 = by * kSyTH;
     const int tid = threadIdx.x, ex = tid & (kSyE - 1), ey0 = tid / kSyE;
     const uint8_t* nearF = p.nearC ? p.c : p.a;
@@ -1152,50 +1169,53 @@ __device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int 
         return;
     }
     if (tid == 0) cnt = 0;
-    if (tid < 256) {
+    if (!p.mid && tid < 256) {
         TA[tid] = __fmul_rn(p.wA, (float)tid);
         TC[tid] = __fmul_rn(p.wC, (float)tid);
     }
-    float2* hrow;
     uint8_t* e;
     unsigned short* hsum;
-    const SyCoef cx = syFieldStage(p, X0, Y0, tid, ex, ey0, rowc, gReg, sm, hrow, e, hsum);
-    // 2. this thread's region column: half-vector (vertical stage, x fs folded in), both warps, mismatch. The warps
-    //    wait in shared memory for the blend (in registers they would leave too few for the sample loads in flight).
+    const SyField f = syFieldStage(p, X0, Y0, tid, ex, rowc, sm, e, hsum);
+    // 2. this thread's region column and kSyK rows: half-vector, both warps, mismatch. The warps wait in shared memory
+    //    for the blend (in registers they would leave too few for the sample loads in flight).
     uint32_t* sWA = reinterpret_cast<uint32_t*>(hsum + kSyEH * kSyHS);   // the output rows: kSyTH x kSyE
     uint32_t* sWC = sWA + kSyTH * kSyE;
     const float kA = p.mid ? 1.0f : p.ka, kC = p.mid ? 1.0f : p.kc;   // t = 0.5: the products by 1 are exact
-#pragma unroll
-    for (int k = 0; k < kSyK; k++) {
-        const int ey = ey0 + (kSyThreads / kSyE) * k;
-        const SyCoef cy = rowc[ey];
-        const float2 h0 = hrow[cy.i0 * kSyE + ex], h1 = hrow[cy.i1 * kSyE + ex];
-        const float hx = __fadd_rn(__fmul_rn(h0.x, cy.a0), __fmul_rn(h1.x, cy.a1));
-        const float hy = __fadd_rn(__fmul_rn(h0.y, cy.a0), __fmul_rn(h1.y, cy.a1));
-        // a(q - 2t h), c(q + 2(1 - t) h): float32 products, then the sums (numpy's order)
-        const float2 ba = rne32bits(make_float2(__fsub_rn(cx.pos, __fmul_rn(kA, hx)), __fsub_rn(cy.pos, __fmul_rn(kA, hy))));
-        const float2 bc = rne32bits(make_float2(__fadd_rn(cx.pos, __fmul_rn(kC, hx)), __fadd_rn(cy.pos, __fmul_rn(kC, hy))));
-        int ca[3], cc[3];
-        uint32_t A = sampleU8(fa32, pw, p.W, p.H, ba.x, ba.y, ca), C = sampleU8(fc32, pw, p.W, p.H, bc.x, bc.y, cc);
-        if (kUi) {   // CrosshairV2: a tap on its own frame's UI takes the other frame's tap (both or neither: kept)
-            const bool ha = p.uiA && uiHitMask(p.uiA, __float_as_int(ba.x) - 0x4B400000, __float_as_int(ba.y) - 0x4B400000);
-            const bool hc = p.uiC && uiHitMask(p.uiC, __float_as_int(bc.x) - 0x4B400000, __float_as_int(bc.y) - 0x4B400000);
-            if (ha != hc) {
-                if (ha) {
-                    A = C;
-                    ca[0] = cc[0]; ca[1] = cc[1]; ca[2] = cc[2];
-                } else {
-                    C = A;
-                    cc[0] = ca[0]; cc[1] = ca[1]; cc[2] = ca[2];
-                }
-            }
-        }
+    // a(q - 2t h), c(q + 2(1 - t) h): float32 products, then the sums (numpy's order), rounded to 1/32 px
+    auto positions = [&](float posy, float2 h, float2& ba, float2& bc) {
+        const float2 ha = pmul(h, make_float2(kA, kA)), hc = pmul(h, make_float2(kC, kC));
+        ba = rne32bits(make_float2(__fsub_rn(f.cx.pos, ha.x), __fsub_rn(posy, ha.y)));
+        bc = rne32bits(make_float2(__fadd_rn(f.cx.pos, hc.x), __fadd_rn(posy, hc.y)));
+    };
+    auto keep = [&](int ey, uint32_t A, uint32_t C, uint32_t m) {
         if ((unsigned)(ey - kSyAp) < (unsigned)kSyTH) {   // warp-uniform
             sWA[(ey - kSyAp) * kSyE + ex] = A;
             sWC[(ey - kSyAp) * kSyE + ex] = C;
         }
-        const int m = max(max(abs(ca[0] - cc[0]), abs(ca[1] - cc[1])), abs(ca[2] - cc[2]));
         e[ey * kSyES + ex] = (uint8_t)m;
+    };
+    if (!kUi && f.in) {
+        syWalk<true, kLat ? kSyK : 2>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) {
+            float2 ba, bc;
+            positions(posy, h, ba, bc);
+            const uint32_t A = sampleU8In(fa32, pw, ba.x, ba.y), C = sampleU8In(fc32, pw, bc.x, bc.y);
+            keep(ey, A, C, maxDiffU8(A, C));
+        });
+    } else {
+        syWalk<false, 2>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) {
+            float2 ba, bc;
+            positions(posy, h, ba, bc);
+            uint32_t A = sampleU8(fa32, pw, p.W, p.H, ba.x, ba.y), C = sampleU8(fc32, pw, p.W, p.H, bc.x, bc.y);
+            if (kUi) {   // CrosshairV2: a tap on its own frame's UI takes the other frame's tap (both or neither: kept)
+                const bool ha = p.uiA && uiHitMask(p.uiA, __float_as_int(ba.x) - 0x4B400000, __float_as_int(ba.y) - 0x4B400000);
+                const bool hc = p.uiC && uiHitMask(p.uiC, __float_as_int(bc.x) - 0x4B400000, __float_as_int(bc.y) - 0x4B400000);
+                if (ha != hc) {
+                    if (ha) A = C;
+                    else C = A;
+                }
+            }
+            keep(ey, A, C, maxDiffU8(A, C));
+        });
     }
     const int lx = ex - kSyAp, x = X0 + lx;
     const bool colOk = (unsigned)lx < (unsigned)kSyT && x < p.W;   // this thread's output column
@@ -1203,46 +1223,71 @@ __device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int 
     // 3. horizontal 7-sums: one region row and 8 output columns per thread, a running window
     syRowSums(e, hsum, tid);
     __syncthreads();
-    // 4. this thread's output pixels: vertical 7-sum (a running window), trust, blend, store
+    // 4. this thread's output pixels: the vertical 7-sums (a running window), trust, blend, store. A warp whose pixels
+    //    are all fully trusted (most are) only blends.
     unsigned int myCnt = 0;
-    // Weights that are multiples of 1/256 (t = k/256: 1/4, 3/4, ...) make every step of the blend exact (8-bit x 8-bit
-    // products, sums below 2^17), so fl(fl(wA a) + fl(wC c)) + 0.5 floored is (WA a + WC c + 128) >> 8 with WA = 256 wA,
-    // WC = 256 wC: two channels per 32-bit multiply-add (16-bit lanes, no carry while WA + WC <= 256)
-    const float wa256 = __fmul_rn(p.wA, 256.0f), wc256 = __fmul_rn(p.wC, 256.0f);
-    const bool dyad = !p.mid && wa256 == truncf(wa256) && wc256 == truncf(wc256) && wa256 >= 0.0f && wc256 >= 0.0f &&
-                      __fadd_rn(wa256, wc256) <= 256.0f;
-    const uint32_t WA = dyad ? (uint32_t)wa256 : 0u, WC = dyad ? (uint32_t)wc256 : 0u;
-    if (colOk) {
-        const unsigned short* q = hsum + syOutRow(ey0, 0) * kSyHS + lx;
+    const uint32_t WA = (uint32_t)p.wA256, WC = (uint32_t)p.wC256;
+    const int ly0 = syOutRow(ey0, 0), rows = colOk ? min(kSyK, min(kSyTH - ly0, p.H - (Y0 + ly0))) : 0;
+    const uint32_t* wa = sWA + ly0 * kSyE + ex;
+    const uint32_t* wc = sWC + ly0 * kSyE + ex;
+    const uint32_t* nf = reinterpret_cast<const uint32_t*>(nearF + (size_t)(Y0 + ly0) * pitch) + x;
+    const unsigned short* q = hsum + ly0 * kSyHS + lx;
+    int top = -1;   // the largest 7x7 sum of this thread's pixels
+    if (rows > 0) {
         int S = q[0] + q[kSyHS] + q[2 * kSyHS] + q[3 * kSyHS] + q[4 * kSyHS] + q[5 * kSyHS];
 #pragma unroll
         for (int k = 0; k < kSyK; k++) {
-            const int ly = syOutRow(ey0, k), y = Y0 + ly;
-            if (ly >= kSyTH || y >= p.H) break;   // uniform over the warp; later rows are out too
-            S += q[(k + 6) * kSyHS] - (k ? q[(k - 1) * kSyHS] : 0);
-            const uint32_t nq = __ldg(reinterpret_cast<const uint32_t*>(nearF + (size_t)y * pitch) + x);
-            const uint32_t wak = sWA[ly * kSyE + ex], wck = sWC[ly * kSyE + ex];
+            if (k >= rows) break;   // uniform over the warp's valid columns, as below
+            S += q[(k + 6) * kSyHS];
+            top = max(top, S);
+            S -= q[k * kSyHS];
+        }
+        sink.begin(x, Y0 + ly0);
+    }
+    // the blend rounded (u = 0)
+    auto blendMid = [](uint32_t A, uint32_t C) {   // floor(0.5 (a + c) + 0.5) per byte, no borrow between bytes
+        return (A | C) - (((A ^ C) >> 1) & 0x7F7F7F7Fu);
+    };
+    auto blendWhole = [&](uint32_t A, uint32_t C) {   // whole 256ths (blendDyadic)
+        const uint32_t M = 0x00FF00FFu;
+        const uint32_t rb = (A & M) * WA + ((C & M) * WC + 0x00800080u);
+        const uint32_t g = ((A >> 8) & M) * WA + (((C >> 8) & M) * WC + 0x00800080u);
+        return __byte_perm(rb, g, 0x0351);
+    };
+    auto blendTable = [&](uint32_t A, uint32_t C) {
+        // fl32(fl32((1 - t) a) + fl32(t c)) + 0.5, floored (never above 255.5 here, so no clamp is needed): the products
+        // come from the tables, the adds are paired (adds alone cannot be fused), the floor is a round-toward-zero add
+        // of 2^23 whose low mantissa byte is the result
+        const float2 m01 = padd(make_float2(TA[A & 255u], TA[(A >> 8) & 255u]), make_float2(TC[C & 255u], TC[(C >> 8) & 255u]));
+        const float m2 = __fadd_rn(TA[(A >> 16) & 255u], TC[(C >> 16) & 255u]);
+        const float2 f01 = __ffma2_rz(padd(m01, make_float2(0.5f, 0.5f)), make_float2(1.0f, 1.0f), make_float2(8388608.0f, 8388608.0f));
+        const float f2 = __fadd_rz(__fadd_rn(m2, 0.5f), 8388608.0f);
+        return __byte_perm(__byte_perm(__float_as_uint(f01.x), __float_as_uint(f01.y), 0x0040), __float_as_uint(f2), 0x0410);
+    };
+    auto trusted = [&](auto&& blend) {
+#pragma unroll
+        for (int k = 0; k < kSyK; k++) {
+            if (k >= rows) break;
+            // alpha (byte 3 in both pixel orders): the nearer frame's
+            sink.put(k, __byte_perm(blend(wa[k * kSyE], wc[k * kSyE]), __ldg(nf), 0x7210));
+            nf += pw;
+        }
+    };
+    if (!__any_sync(0xffffffffu, top > p.sZero)) {
+        if (p.mid) trusted(blendMid);
+        else if (p.wA256 >= 0) trusted(blendWhole);
+        else trusted(blendTable);
+    } else {
+#pragma unroll(Sink::kUnroll)
+        for (int k = 0; k < kSyK; k++) {
+            if (k >= rows) break;
+            const uint32_t nq = __ldg(nf), wak = wa[k * kSyE], wck = wc[k * kSyE];
+            nf += pw;
+            const int S = q[k * kSyHS] + q[(k + 1) * kSyHS] + q[(k + 2) * kSyHS] + q[(k + 3) * kSyHS] + q[(k + 4) * kSyHS] +
+                          q[(k + 5) * kSyHS] + q[(k + 6) * kSyHS];
             uint32_t o;
-            if (S <= p.sZero) {   // u = 0: out = the blend rounded
-                if (p.mid) {
-                    // floor(0.5 (a + c) + 0.5) per byte: (a | c) - ((a ^ c) >> 1), no borrow between bytes
-                    o = (wak | wck) - (((wak ^ wck) >> 1) & 0x7F7F7F7Fu);
-                } else if (dyad) {
-                    const uint32_t M = 0x00FF00FFu;
-                    const uint32_t rb = (wak & M) * WA + ((wck & M) * WC + 0x00800080u);
-                    const uint32_t g = ((wak >> 8) & M) * WA + (((wck >> 8) & M) * WC + 0x00800080u);
-                    o = ((rb >> 8) & M) | (g & 0x0000FF00u);
-                } else {
-                    // fl32(fl32((1 - t) a) + fl32(t c)) + 0.5, floored (never above 255.5 here, so no clamp is needed): the
-                    // products come from the tables, the adds are paired (adds alone cannot be fused), the floor is a
-                    // round-toward-zero add of 2^23 whose low mantissa byte is the result
-                    const uint32_t A = wak, C = wck;
-                    const float2 m01 = padd(make_float2(TA[A & 255u], TA[(A >> 8) & 255u]), make_float2(TC[C & 255u], TC[(C >> 8) & 255u]));
-                    const float m2 = __fadd_rn(TA[(A >> 16) & 255u], TC[(C >> 16) & 255u]);
-                    const float2 f01 = __ffma2_rz(padd(m01, make_float2(0.5f, 0.5f)), make_float2(1.0f, 1.0f), make_float2(8388608.0f, 8388608.0f));
-                    const float f2 = __fadd_rz(__fadd_rn(m2, 0.5f), 8388608.0f);
-                    o = __byte_perm(__byte_perm(__float_as_uint(f01.x), __float_as_uint(f01.y), 0x0040), __float_as_uint(f2), 0x0410);
-                }
+            if (S <= p.sZero) {   // u = 0
+                o = p.mid ? blendMid(wak, wck) : (p.wA256 >= 0 ? blendWhole(wak, wck) : blendTable(wak, wck));
             } else if (S >= p.sOne) {   // u = 1: the nearer frame
                 o = nq;
                 myCnt++;
@@ -1263,27 +1308,57 @@ __device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int 
                     o |= (uint32_t)floorPos(fminf(fmaxf(v, 0.0f), 255.0f)) << sh;
                 }
             }
-            o = (o & 0x00FFFFFFu) | (nq & 0xFF000000u);   // alpha (byte 3 in both pixel orders): the nearer frame's
-            sink(k, x, y, ly, o);
-            if (p.emap) p.emap[(size_t)y * ((p.W + 3) & ~3) + x] = e[(ly + kSyAp) * kSyES + ex];
+            sink.put(k, __byte_perm(o, nq, 0x7210));
         }
     }
+    if (p.emap)
+        for (int k = 0; k < rows; k++)
+            p.emap[(size_t)(Y0 + ly0 + k) * ((p.W + 3) & ~3) + x] = e[(ly0 + k + kSyAp) * kSyES + ex];
     if (myCnt) atomicAdd(&cnt, myCnt);
     __syncthreads();
     if (tid == 0 && cnt && p.untrusted) atomicAdd(p.untrusted, cnt);
 }
 
+// the store of a synthesis: rows of p.out from (x, y0) down
+struct SynthStore {
+    static constexpr int kUnroll = 1;
+    const SynthParams& p;
+    uint8_t* o;
+    __device__ __forceinline__ void begin(int x, int y0) { o = p.out + (size_t)y0 * p.outPitch + (size_t)x * 4; }
+    __device__ __forceinline__ void put(int, uint32_t v) {
+        *reinterpret_cast<uint32_t*>(o) = v;
+        o += p.outPitch;
+    }
+};
+
+// a blur's sample: acc += q x the pixel
+struct BlurAdd {
+    static constexpr int kUnroll = kSyK;   // acc stays in registers
+    uint32_t (&acc)[kSyK][3];
+    uint32_t q;
+    __device__ __forceinline__ void begin(int, int) {}
+    __device__ __forceinline__ void put(int k, uint32_t o) {
+        acc[k][0] += q * (o & 255u);
+        acc[k][1] += q * ((o >> 8) & 255u);
+        acc[k][2] += q * ((o >> 16) & 255u);
+    }
+};
+
 // one output tile of one synthesis, stored to p.out
-template <bool kUi = false>
+template <bool kUi = false, bool kLat = false>
 __device__ __forceinline__ void synthTile(const SynthParams& p, int bx, int by) {
-    synthTileCore<true, kUi>(p, bx, by, [&](int, int x, int y, int, uint32_t o) {
-        reinterpret_cast<uint32_t*>(p.out + (size_t)y * p.outPitch)[x] = o;
-    });
+    SynthStore store{p, nullptr};
+    synthTileCore<true, kUi, kLat>(p, bx, by, store);
 }
 
 __global__ void __launch_bounds__(kSyThreads, 3) k_synth(const SynthParams p) {
     pdlEnter();
     synthTile(p, blockIdx.x, blockIdx.y);
+}
+// grids of at most 2 CTAs per SM: more registers and the unrolled rows in place of a third CTA
+__global__ void __launch_bounds__(kSyThreads, 2) k_synth_lat(const SynthParams p) {
+    pdlEnter();
+    synthTile<false, true>(p, blockIdx.x, blockIdx.y);
 }
 
 // the same with CrosshairV2's warp-tap rejection (p.uiA / p.uiC); a separate kernel so the plain one is unchanged
@@ -1346,16 +1421,14 @@ __global__ void __launch_bounds__(kSyThreads, 2) k_synth_blur_t(const BlurParams
             const BlurSample& m = bp.smp[j];
             sp.lookup = m.lookup; sp.mid = m.mid; sp.nearC = m.nearC;
             sp.s = m.s; sp.ka = m.ka; sp.kc = m.kc; sp.wA = m.wA; sp.wC = m.wC;
+            sp.wA256 = m.wA256; sp.wC256 = m.wC256;
             sp.untrusted = bp.fix ? nullptr : bp.cnt + j;
             sp.emap = nullptr;
         }
         __syncthreads();
         const uint32_t q = bp.smp[j].q;
-        synthTileCore<false, kUi>(sp, blockIdx.x, blockIdx.y, [&](int k, int, int, int, uint32_t o) {
-            acc[k][0] += q * (o & 255u);
-            acc[k][1] += q * ((o >> 8) & 255u);
-            acc[k][2] += q * ((o >> 16) & 255u);
-        });
+        BlurAdd add{acc, q};
+        synthTileCore<false, kUi, false>(sp, blockIdx.x, blockIdx.y, add);
         __syncthreads();   // the tile's shared memory and sp are free again
     }
     // the output: the synthesized samples' sums plus the replaced samples' real pixels, rounded once
@@ -1593,6 +1666,8 @@ cudaError_t prepareKernels() {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_synth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(synthSmemBytes(1) + kSyWarpBytes));
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_synth_lat, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(synthSmemBytes(1) + kSyWarpBytes));
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_synth_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(synthSmemBytes(1) + kSyWarpBytes));
     if (e == cudaSuccess)
@@ -1618,9 +1693,9 @@ cudaError_t launchPixfield(const PixfieldParams& p, cudaStream_t s) {
     return launchPdl(k_pixfield, dim3(divUp(p.w, kPfTW), divUp(p.h, kPfTH)), dim3(256), 0, s, p);
 }
 size_t synthSmemBytes(int fs) {  // declared in fg_params.h
-    // worst-case field region of a tile (GW x GH float2) + its horizontal stage + mismatch + row sums
+    // worst-case field region of a tile (GW x GH float2) + mismatch + row sums
     const int gw = (kSyE + fs - 1) / fs + 3, gh = (kSyEH + fs - 1) / fs + 3;
-    return (size_t)gw * gh * 8 + (size_t)gh * kSyE * 8 + (size_t)kSyEH * kSyES + (size_t)kSyEH * kSyHS * 2;
+    return (size_t)gw * gh * 8 + (size_t)kSyEH * kSyES + (size_t)kSyEH * kSyHS * 2;
 }
 size_t synthKernelSmem(int fs) { return synthSmemBytes(fs) + kSyWarpBytes; }
 int synthTilesX(int W) { return (int)divUp(W, kSyT); }
@@ -1629,6 +1704,8 @@ cudaError_t launchSynth(const SynthParams& p, cudaStream_t s) {
     const size_t smem = synthSmemBytes(p.fs) + kSyWarpBytes;
     const dim3 grid(divUp(p.W, kSyT), divUp(p.H, kSyTH));
     if (p.uiA || p.uiC) return launchPdl(k_synth_ui, grid, dim3(kSyThreads), smem, s, p);
+    // one wave of 2 CTAs per SM (a 640x360 frame: 14.6 -> 11 us, 1280x720 and up about even): the latency form
+    if ((int)(grid.x * grid.y) <= 2 * smCount()) return launchPdl(k_synth_lat, grid, dim3(kSyThreads), smem, s, p);
     return launchPdl(k_synth, grid, dim3(kSyThreads), smem, s, p);
 }
 cudaError_t launchSynthBlur(const BlurParams& bp, int fix, cudaStream_t s) {

@@ -194,6 +194,7 @@ extern "C" int fg_record_synth_noalloc(void* stream, uint32_t view_format, uint3
     sp.kc = (float)(2.0 * (1.0 - td));
     sp.wA = (float)(1.0 - td);
     sp.wC = t;
+    fgk::blendDyadic(sp.wA, sp.wC, sp.wA256, sp.wC256);
     sp.trust0 = set.trustLow;
     sp.trustSpan = (float)((double)set.trustHigh - (double)set.trustLow);
     fgk::trustShortcuts(set.trustLow, set.trustHigh, sp.sZero, sp.sOne);

@@ -148,6 +148,7 @@ struct SynthParams {
     int mid;                       // t == 0.5: blend 0.5 * (wa + wc)
     int nearC;                     // t > 0.5: the nearer frame is curr
     float s, ka, kc, wA, wC;       // fl32(2t - 1), fl32(2t), fl32(2(1 - t)), fl32(1 - t), fl32(t)
+    int wA256, wC256;              // 256 wA, 256 wC where both are whole numbers, at most 256 in all (blendDyadic), else -1
     float trust0, trustSpan;       // trustLow, fl32(trustHigh - trustLow)
     int sZero, sOne;               // 7x7 sums S <= sZero give u = 0, S >= sOne give u = 1 (host-derived shortcuts)
     DevState* st;
@@ -192,6 +193,7 @@ struct BlurSample {
     int mode;                      // 0: a synthesis at t_k; 1: the real frame prev (t_k <= 0); 2: curr (t_k >= 1)
     int lookup, mid, nearC;        // recordSynth(t_k)'s SynthParams fields
     float s, ka, kc, wA, wC;
+    int wA256, wC256;
     uint32_t q;                    // weight, units of 2^-16
 };
 struct BlurParams {
@@ -345,6 +347,16 @@ inline void trustShortcuts(float trustLow, float trustHigh, int& sZero, int& sOn
     for (int S = 0; S <= 49 * 255 && u(S) == 0.0f; S++) sZero = S;
     sOne = 49 * 255 + 1;
     for (int S = 49 * 255; S >= 0 && u(S) == 1.0f; S--) sOne = S;
+}
+
+// Weights that are multiples of 1/256 (t = k/256: 1/4, 3/4, ...) make every step of the 8-bit blend exact (8-bit x 8-bit
+// products, sums below 2^17), so fl(fl(wA a) + fl(wC c)) + 0.5 floored is (WA a + WC c + 128) >> 8 with WA = 256 wA, WC =
+// 256 wC: two channels per 32-bit multiply-add (16-bit lanes, no carry while WA + WC <= 256)
+inline void blendDyadic(float wA, float wC, int& WA, int& WC) {
+    const float a = wA * 256.0f, c = wC * 256.0f;   // exact
+    const bool ok = a >= 0.0f && c >= 0.0f && a + c <= 256.0f && a == (float)(int)a && c == (float)(int)c;
+    WA = ok ? (int)a : -1;
+    WC = ok ? (int)c : -1;
 }
 
 }  // namespace fgk

@@ -764,6 +764,7 @@ struct Interpolator::Impl {
         sp.kc = (float)(2.0 * (1.0 - td));
         sp.wA = (float)(1.0 - td);
         sp.wC = t;
+        fgk::blendDyadic(sp.wA, sp.wC, sp.wA256, sp.wC256);
         sp.trust0 = set.trustLow;
         sp.trustSpan = (float)((double)set.trustHigh - (double)set.trustLow);
         sp.sZero = sZero; sp.sOne = sOne;
@@ -817,6 +818,7 @@ struct Interpolator::Impl {
             const fgk::SynthParams sp = synthParams(prev, curr, out, tk[k], nullptr);
             m.lookup = sp.lookup; m.mid = sp.mid; m.nearC = sp.nearC;
             m.s = sp.s; m.ka = sp.ka; m.kc = sp.kc; m.wA = sp.wA; m.wC = sp.wC;
+            m.wA256 = sp.wA256; m.wC256 = sp.wC256;
         }
         bp.n = n;
         bp.frac = (double)set.globalFallback;

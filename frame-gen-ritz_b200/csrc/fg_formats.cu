@@ -165,32 +165,65 @@ __device__ __forceinline__ float levelOf(const FmtConst& f, float r) {
 }
 
 // ============================================================================================== luma
-// the motion estimate's luma of pixel (x, y) in quarter levels (luma.comp:9-27, format.glsl fgLuma)
-// pq: linear RgbaF16's table of fmtPq255 by half bits (the same function, evaluated once per value), or null
+// a luma level in quarter levels: rint(4 clamp(y, 0, 255)), a NaN 0
+__device__ __forceinline__ int quarters(float y) {
+    return __float_as_int(__fadd_rn(__fmul_rn(fminf(fmaxf(y, 0.0f), 255.0f), 4.0f), 12582912.0f)) - 0x4B400000;
+}
+// the luma of three channel levels (luma.comp:9-27, format.glsl fgLuma)
+__device__ __forceinline__ int quartersRgb(float lr, float lg, float lb) {
+    float d = __fmul_rn(4899.0f, lr);
+    d = __fadd_rn(d, __fmul_rn(9617.0f, lg));
+    d = __fadd_rn(d, __fmul_rn(1868.0f, lb));
+    return quarters(__fmul_rn(d, 1.0f / 16384.0f));
+}
+__device__ __forceinline__ int quartersY(const FmtConst& f, float y) { return quarters(__fmul_rn(__fsub_rn(y, f.black), f.ys)); }
+// ... of an Rgb10 word, of an RgbaF16 pixel. pq: linear RgbaF16's table of fmtPq255 by half bits (the same function,
+// evaluated once per value), or null
+__device__ __forceinline__ int quartersRgb10(const FmtConst& f, uint32_t w) {
+    const float l0 = __fmul_rn((float)(w & 1023u), f.k10), l1 = __fmul_rn((float)((w >> 10) & 1023u), f.k10);
+    const float l2 = __fmul_rn((float)((w >> 20) & 1023u), f.k10);
+    return f.rHigh ? quartersRgb(l2, l1, l0) : quartersRgb(l0, l1, l2);
+}
+__device__ __forceinline__ int quartersF16(const FmtConst& f, const float* pq, uint32_t rg, uint32_t b) {
+    if (pq) return quartersRgb(__ldg(pq + (rg & 0xFFFFu)), __ldg(pq + (rg >> 16)), __ldg(pq + (b & 0xFFFFu)));
+    return quartersRgb(levelOf<kFmtF16>(f, h2f(rg & 0xFFFFu)), levelOf<kFmtF16>(f, h2f(rg >> 16)), levelOf<kFmtF16>(f, h2f(b & 0xFFFFu)));
+}
+
+// the motion estimate's luma of pixel (x, y) in quarter levels
 template <int F>
 __device__ __forceinline__ int lumaQ(const FmtConst& f, const uint8_t* base, size_t pitch, int x, int y, const float* pq) {
+    const uint8_t* row = base + (size_t)y * pitch;
+    if (F == kFmtRgb10) return quartersRgb10(f, __ldg(reinterpret_cast<const uint32_t*>(row) + x));
+    if (F == kFmtF16) {
+        const uint2 q = __ldg(reinterpret_cast<const uint2*>(row) + x);
+        return quartersF16(f, pq, q.x, q.y);
+    }
     float r[3];
-    float yl;
-    if (F == kFmtF16 && pq) {   // the three channels' PQ levels looked up by their bits
-        const uint2 q = __ldg(reinterpret_cast<const uint2*>(base + (size_t)y * pitch) + x);
-        const float lr = __ldg(pq + (q.x & 0xFFFFu)), lg = __ldg(pq + (q.x >> 16)), lb = __ldg(pq + (q.y & 0xFFFFu));
-        float d = __fmul_rn(4899.0f, lr);
-        d = __fadd_rn(d, __fmul_rn(9617.0f, lg));
-        d = __fadd_rn(d, __fmul_rn(1868.0f, lb));
-        yl = __fmul_rn(d, 1.0f / 16384.0f);
-        return __float2int_rn(__fmul_rn(clampF(yl, 0.0f, 255.0f), 4.0f));
-    }
     texel<F>(f, base, pitch, x, y, r);
-    if (F == kFmtNv12 || F == kFmtP010) {
-        yl = __fmul_rn(__fsub_rn(r[0], f.black), f.ys);
+    return quartersY(f, r[0]);
+}
+
+// ... of the 4 pixels from x on of an aligned row, added up in pairs
+template <int F>
+__device__ __forceinline__ void lumaQ4(const FmtConst& f, const uint8_t* row, int x, const float* pq, int& s0, int& s1) {
+    if (F == kFmtRgb10) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(row + (size_t)x * 4));
+        s0 += quartersRgb10(f, q.x) + quartersRgb10(f, q.y);
+        s1 += quartersRgb10(f, q.z) + quartersRgb10(f, q.w);
+    } else if (F == kFmtF16) {
+        const uint4 q0 = __ldg(reinterpret_cast<const uint4*>(row + (size_t)x * 8)), q1 = __ldg(reinterpret_cast<const uint4*>(row + (size_t)x * 8) + 1);
+        s0 += quartersF16(f, pq, q0.x, q0.y) + quartersF16(f, pq, q0.z, q0.w);
+        s1 += quartersF16(f, pq, q1.x, q1.y) + quartersF16(f, pq, q1.z, q1.w);
+    } else if (F == kFmtNv12) {
+        const uint32_t q = __ldg(reinterpret_cast<const uint32_t*>(row + x));
+        s0 += quartersY(f, (float)(q & 255u)) + quartersY(f, (float)((q >> 8) & 255u));
+        s1 += quartersY(f, (float)((q >> 16) & 255u)) + quartersY(f, (float)(q >> 24));
     } else {
-        const float lr = levelOf<F>(f, r[0]), lg = levelOf<F>(f, r[1]), lb = levelOf<F>(f, r[2]);
-        float d = __fmul_rn(4899.0f, lr);
-        d = __fadd_rn(d, __fmul_rn(9617.0f, lg));
-        d = __fadd_rn(d, __fmul_rn(1868.0f, lb));
-        yl = __fmul_rn(d, 1.0f / 16384.0f);
+        const uint2 q = __ldg(reinterpret_cast<const uint2*>(row + (size_t)x * 2));
+        auto lv = [](uint32_t v) { return __fmul_rn((float)v, 0x1p-8f); };
+        s0 += quartersY(f, lv(q.x & 0xFFFFu)) + quartersY(f, lv(q.x >> 16));
+        s1 += quartersY(f, lv(q.y & 0xFFFFu)) + quartersY(f, lv(q.y >> 16));
     }
-    return __float2int_rn(__fmul_rn(clampF(yl, 0.0f, 255.0f), 4.0f));
 }
 
 // integer num / n rounded half to even (num >= 0, n > 0)
@@ -201,12 +234,44 @@ __device__ __forceinline__ int rneDiv(int num, int n) {
     return q;
 }
 
-// interp.flow + pyramid for the other formats: one CTA = a 32x32 level-0 tile and its tower (as k_luma_pyr)
+// interp.flow + pyramid for the other formats: one CTA = a 32x32 level-0 tile and its tower (as k_luma_pyr). Whole tiles of
+// aligned frames at flowScale 2 (p.vec16) take 4 frame pixels x 2 rows per thread and load (4K: Rgb10 49 -> 31 us, linear
+// RgbaF16 78 -> 66, Nv12 35 -> 20, P010 37 -> 21): bound by instruction issue, linear RgbaF16 by its table gathers.
 template <int F>
 __device__ __forceinline__ void lumaFmtCta(const LumaPyrParams& p, int bx, int by) {
-    __shared__ float sl[2][kTowerFloats];
+    __shared__ __align__(8) float sl[2][kTowerFloats];
     const int tx0 = bx * 32, ty0 = by * 32;
     const int fw = p.lw[0], fh = p.lh[0], fs = p.fs;
+    if (p.vec16 && tx0 + 32 <= fw && ty0 + 32 <= fh) {
+        const int cg = threadIdx.x & 15, rp = threadIdx.x >> 4;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int ly = rp + 16 * j, y = ty0 + ly, x = 2 * tx0 + 4 * cg;
+            const uint8_t* ra = p.a + (size_t)(2 * y) * p.pitch;
+            const uint8_t* rc = p.c + (size_t)(2 * y) * p.pitch;
+            int sa0 = 0, sa1 = 0, sc0 = 0, sc1 = 0;   // 4 quarter levels a cell: 16 x the mean
+            lumaQ4<F>(p.f, ra, x, p.pq, sa0, sa1);
+            lumaQ4<F>(p.f, ra + p.pitch, x, p.pq, sa0, sa1);
+            lumaQ4<F>(p.f, rc, x, p.pq, sc0, sc1);
+            lumaQ4<F>(p.f, rc + p.pitch, x, p.pq, sc0, sc1);
+            const float2 va = make_float2(__fmul_rn((float)sa0, 1.0f / 16.0f), __fmul_rn((float)sa1, 1.0f / 16.0f));
+            const float2 vc = make_float2(__fmul_rn((float)sc0, 1.0f / 16.0f), __fmul_rn((float)sc1, 1.0f / 16.0f));
+            const size_t px = (size_t)y * fw + tx0 + 2 * cg;
+            if (p.la[0]) {
+                *reinterpret_cast<float2*>(p.la[0] + px) = va;
+                *reinterpret_cast<float2*>(p.lc[0] + px) = vc;
+            }
+            *reinterpret_cast<float2*>(&sl[0][ly * 32 + 2 * cg]) = va;
+            *reinterpret_cast<float2*>(&sl[1][ly * 32 + 2 * cg]) = vc;
+            const int na = __shfl_down_sync(0xffffffffu, sa0, 1), nc = __shfl_down_sync(0xffffffffu, sc0, 1);
+            const bool last = tx0 + 2 * cg + 2 == fw;
+            storePairs2(p.pa + px, sa0, sa1, last ? sa1 : na, cg == 15 && !last, cg == 0 && tx0 > 0);
+            storePairs2(p.pc + px, sc0, sc1, last ? sc1 : nc, cg == 15 && !last, cg == 0 && tx0 > 0);
+        }
+        __syncthreads();
+        lumaTower<true>(p, sl, tx0, ty0);
+        return;
+    }
     for (int i = threadIdx.x; i < 1024; i += 256) {
         const int x = tx0 + (i & 31), y = ty0 + (i >> 5);
         float va = 0.0f, vc = 0.0f;
@@ -1017,45 +1082,27 @@ cudaError_t launchLumaFmtMerged(Merged<LumaPyrParams>& m, int format, cudaStream
 // widened by fs px per step up to 8 px while it has none, formed as the luma pass forms a cell (quarter levels summed,
 // rneDiv(4 sum, n) / 16, so the estimate's sums stay exact)
 template <int F>
-__global__ void __launch_bounds__(64) k_ui_fill_fmt(const UiFillParams p) {
+__global__ void __launch_bounds__(128) k_ui_fill_fmt(const UiFillParams p) {   // a warp per cell
     pdlEnter();
-    const int cx = p.cx0 + (int)(blockIdx.x * 8 + (threadIdx.x & 7)), cy = p.cy0 + (int)(blockIdx.y * 8 + (threadIdx.x >> 3));
-    if (cx >= p.cx0 + p.ncx || cy >= p.cy0 + p.ncy || cx >= p.fw || cy >= p.fh) return;
-    const bool isC = blockIdx.z != 0;
-    const uint32_t* __restrict__ m = isC ? p.mc : p.ma;
+    const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int cx = p.cx0 + i % p.ncx, cy = p.cy0 + i / p.ncx;
+    if (i >= p.ncx * p.ncy || cx >= p.fw || cy >= p.fh) return;
+    const bool isC = blockIdx.y != 0;
     const uint8_t* f = isC ? p.c : p.a;
-    const int fs = p.fs, px = cx * fs, py = cy * fs;
-    bool has = false;
-    for (int j = 0; j < fs && !has; j++)
-        for (int i = 0; i < fs; i++)
-            if (px + i < p.W && py + j < p.H && uiPx(m, px + i, py + j)) {
-                has = true;
-                break;
-            }
-    if (!has) return;
-    for (int k = 0; k <= 8; k += fs) {
-        int sum = 0, n = 0;
-        for (int y = py - k; y < py + fs + k; y++)
-            for (int x = px - k; x < px + fs + k; x++) {
-                if (x < 0 || y < 0 || x >= p.W || y >= p.H || uiPx(m, x, y)) continue;
-                sum += lumaQ<F>(p.f, f, p.pitch, x, y, p.pq);
-                n++;
-            }
-        if (n > 0) {
-            const float v = __fmul_rn(i2f(rneDiv(4 * sum, n)), 1.0f / 16.0f);
-            (isC ? p.lc : p.la)[(size_t)cy * p.fw + cx] = v;
-            if (p.pa) storePairPx(isC ? p.pc : p.pa, p.fw, cx, cy, v);
-            return;
-        }
-    }
+    int sum, n;
+    if (!uiFillWindow(isC ? p.mc : p.ma, p.W, p.H, p.fs, cx * p.fs, cy * p.fs, lane,
+                      [&](int x, int y) { return lumaQ<F>(p.f, f, p.pitch, x, y, p.pq); }, sum, n) || lane) return;
+    const float v = __fmul_rn(i2f(rneDiv(4 * sum, n)), 1.0f / 16.0f);
+    (isC ? p.lc : p.la)[(size_t)cy * p.fw + cx] = v;
+    storePairPx(isC ? p.pc : p.pa, p.fw, cx, cy, v);
 }
 cudaError_t launchUiFillFmt(const UiFillParams& p, cudaStream_t s) {
-    const dim3 grid(divUp(p.ncx, 8), divUp(p.ncy, 8), 2);
+    const dim3 grid(divUp(p.ncx * p.ncy, 4), 2);
     switch (p.f.format) {
-        case kFmtRgb10: return launchPdl(k_ui_fill_fmt<kFmtRgb10>, grid, dim3(64), 0, s, p);
-        case kFmtF16: return launchPdl(k_ui_fill_fmt<kFmtF16>, grid, dim3(64), 0, s, p);
-        case kFmtNv12: return launchPdl(k_ui_fill_fmt<kFmtNv12>, grid, dim3(64), 0, s, p);
-        case kFmtP010: return launchPdl(k_ui_fill_fmt<kFmtP010>, grid, dim3(64), 0, s, p);
+        case kFmtRgb10: return launchPdl(k_ui_fill_fmt<kFmtRgb10>, grid, dim3(128), 0, s, p);
+        case kFmtF16: return launchPdl(k_ui_fill_fmt<kFmtF16>, grid, dim3(128), 0, s, p);
+        case kFmtNv12: return launchPdl(k_ui_fill_fmt<kFmtNv12>, grid, dim3(128), 0, s, p);
+        case kFmtP010: return launchPdl(k_ui_fill_fmt<kFmtP010>, grid, dim3(128), 0, s, p);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -47,7 +47,7 @@ struct LumaPyrParams {
     int W, H, fs;          // frame size, flow scale (1, 2, 4)
     int ri, gi, bi;        // byte offsets of R, G, B in a 4-byte pixel
     int nlev;              // levels written here (<= kPyrInKernel)
-    int vec16;             // flowScale 2 with 16-byte aligned frames and rows: the uint4 path
+    int vec16;             // flowScale 2, rows aligned to a load of 4 pixels, the pair planes kept: the vector path
     const float* pq;       // RgbaF16 linear: the PQ level (fmtPq255) of every half value, indexed by its bits, or null
     int lw[kPyrInKernel], lh[kPyrInKernel];
     float* la[kPyrInKernel];   // [0] null: no pass reads level 0 as float

@@ -244,44 +244,27 @@ __global__ void __launch_bounds__(kUiTX * kUiTY) k_ui_patch_chroma(const UiPatch
 // 1 curr: a cell holding a UI pixel takes the mean gray level (cv2's weights, the library's level-0 source) of its
 // not-UI pixels, the window widened by fs px per side per step up to 8 px while there are none, rounded half up to the
 // level-0 grid (multiples of 1 / fs^2) so the estimate's sums stay exact.
-__global__ void __launch_bounds__(64) k_ui_v2_fill(const UiFillParams p) {
+__global__ void __launch_bounds__(128) k_ui_v2_fill(const UiFillParams p) {   // a warp per cell
     pdlEnter();
-    const int cx = p.cx0 + (int)(blockIdx.x * 8 + (threadIdx.x & 7)), cy = p.cy0 + (int)(blockIdx.y * 8 + (threadIdx.x >> 3));
-    if (cx >= p.cx0 + p.ncx || cy >= p.cy0 + p.ncy || cx >= p.fw || cy >= p.fh) return;
-    const bool isC = blockIdx.z != 0;
-    const uint32_t* __restrict__ m = isC ? p.mc : p.ma;
+    const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int cx = p.cx0 + i % p.ncx, cy = p.cy0 + i / p.ncx;
+    if (i >= p.ncx * p.ncy || cx >= p.fw || cy >= p.fh) return;
+    const bool isC = blockIdx.y != 0;
     const uint8_t* f = isC ? p.c : p.a;
-    const int fs = p.fs, px = cx * fs, py = cy * fs;
-    bool has = false;
-    for (int j = 0; j < fs && !has; j++)
-        for (int i = 0; i < fs; i++)
-            if (px + i < p.W && py + j < p.H && uiPx(m, px + i, py + j)) {
-                has = true;
-                break;
-            }
-    if (!has) return;
-    for (int k = 0; k <= 8; k += fs) {
-        int sum = 0, n = 0;
-        for (int y = py - k; y < py + fs + k; y++)
-            for (int x = px - k; x < px + fs + k; x++) {
-                if (x < 0 || y < 0 || x >= p.W || y >= p.H || uiPx(m, x, y)) continue;
-                sum += gray8(__ldg(reinterpret_cast<const uint32_t*>(f + (size_t)y * p.pitch) + x), p.ri, p.gi, p.bi);
-                n++;
-            }
-        if (n > 0) {
-            const int s2 = fs * fs;
-            const float v = (float)((2 * sum * s2 + n) / (2 * n)) / (float)s2;
-            (isC ? p.lc : p.la)[(size_t)cy * p.fw + cx] = v;
-            if (p.pa) storePairPx(isC ? p.pc : p.pa, p.fw, cx, cy, v);
-            return;
-        }
-    }
+    int sum, n;
+    if (!uiFillWindow(isC ? p.mc : p.ma, p.W, p.H, p.fs, cx * p.fs, cy * p.fs, lane, [&](int x, int y) {
+            return gray8(__ldg(reinterpret_cast<const uint32_t*>(f + (size_t)y * p.pitch) + x), p.ri, p.gi, p.bi);
+        }, sum, n) || lane) return;
+    const int s2 = p.fs * p.fs;
+    const float v = (float)((2 * sum * s2 + n) / (2 * n)) / (float)s2;
+    (isC ? p.lc : p.la)[(size_t)cy * p.fw + cx] = v;
+    if (p.pa) storePairPx(isC ? p.pc : p.pa, p.fw, cx, cy, v);
 }
 
 }  // namespace
 
 cudaError_t launchUiFill(const UiFillParams& p, cudaStream_t s) {
-    return launchPdl(k_ui_v2_fill, dim3(divUp(p.ncx, 8), divUp(p.ncy, 8), 2), dim3(64), 0, s, p);
+    return launchPdl(k_ui_v2_fill, dim3(divUp(p.ncx * p.ncy, 4), 2), dim3(128), 0, s, p);
 }
 
 cudaError_t launchUiV2Update(const UiV2Params& p, cudaStream_t s) {

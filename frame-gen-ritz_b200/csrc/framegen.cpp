@@ -628,8 +628,11 @@ struct Interpolator::Impl {
         lp.pq = pqTab;
         lp.pa = pair;
         lp.pc = pair ? pair + (size_t)L.fw * L.fh : nullptr;
-        lp.vec16 = fmt == Format::Rgba8 && set.flowScale == 2 && prev.pitch % 16 == 0 && ((uintptr_t)prev.data & 15) == 0 && ((uintptr_t)curr.data & 15) == 0 &&
-                   W % 4 == 0 && H % 2 == 0;   // complete 2x2 cells in every full tile, 8-byte aligned level-0 rows
+        // complete 2x2 cells in every full tile, 8-byte aligned level-0 rows, and rows aligned to a load of 4 pixels (RgbaF16:
+        // of 2)
+        const size_t al = fmt == Format::Nv12 ? 4 : (fmt == Format::P010 ? 8 : 16);
+        lp.vec16 = pair && set.flowScale == 2 && prev.pitch % al == 0 && (uintptr_t)prev.data % al == 0 && (uintptr_t)curr.data % al == 0 &&
+                   W % 4 == 0 && H % 2 == 0;
         for (int l = 0; l < lp.nlev; l++) {
             lp.lw[l] = L.lv[l].w; lp.lh[l] = L.lv[l].h;
             lp.la[l] = luma + L.lv[l].lumaA; lp.lc[l] = luma + L.lv[l].lumaC;

@@ -220,8 +220,25 @@ __device__ __forceinline__ void subpixQCta(const SubpixParams& p, int ctaX, int 
     const int bx = ctaX * 4 + warp;
     if (bx >= p.bw) return;
     const int b = by * p.bw + bx, b0x = bx * kBlock, b0y = by * kBlock;
-    const float2 v0 = __ldg(p.in + b);
-    const int sx = __float2int_rn(v0.x), sy = __float2int_rn(v0.y);
+    // interp.median3 :127-128 of the search's field at this block (level 0's medians feed nothing else: a launch of their own
+    // cost more): lanes 0..8 hold the neighbours' x, 16..24 their y; the median is the one of rank 4
+    int sx, sy;
+    {
+        const int i = lane & 15, j = min(i, 8);
+        const float v = __ldg(reinterpret_cast<const float*>(p.in + clampi(by + j / 3 - 1, 0, p.bh - 1) * p.bw + clampi(bx + j % 3 - 1, 0, p.bw - 1)) +
+                              (lane >> 4));
+        int rank = i > 8 ? 16 : 0;
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            const float u = __shfl_sync(0xffffffffu, v, (lane & 16) + k);
+            rank += u < v || (u == v && k < i);
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, rank == 4);
+        const float mx = __shfl_sync(0xffffffffu, v, __ffs(m & 0xffffu) - 1), my = __shfl_sync(0xffffffffu, v, 15 + __ffs(m >> 16));
+        if (lane == 0) p.med[b] = make_float2(mx, my);
+        sx = __float2int_rn(mx);
+        sy = __float2int_rn(my);
+    }
     uint32_t* wa = tile[warp][0];
     uint32_t* wc = tile[warp][1];
     const int ax0 = b0x - sx - 1, ay0 = b0y - sy - 1, cx0 = b0x + sx - 1, cy0 = b0y + sy - 1;
@@ -293,54 +310,26 @@ __global__ void __launch_bounds__(128) k_subpix_q_m(const __grid_constant__ Merg
 // bilinear block field, own block, block above / below / left / right, zero; each scored by the 5x5 replicate-border
 // box of |a(q - h) - c(q + h)| where every window pixel uses its own candidate; the first minimum wins.
 //
-// One CTA = 60 x 32 outputs (4 block rows) with a 2 px apron, one candidate at a time. A thread owns a region column
-// and the 8 rows of one block row, so a block candidate has one vector, one set of weights and two row pointers per
-// run: per row and frame one load and one dp2a, the lower tap row reused as the next row's upper one. The 2 + 2 apron rows take one more pixel per thread. Errors
-// stay in registers: the vertical 5-sums run down the thread's rows (2 rows above and below from the neighbours through
-// shared memory), the horizontal 5-sums and the choice along rows, 8 pixels per thread. Tiles whose vectors take no tap
-// outside the frame run without any clamp (kIn).
+// One CTA = 60 x 32 outputs (4 block rows) with a 2 px apron, one candidate at a time. The vectors of a tile's blocks
+// differ little, so the window of each frame that they reach is staged in shared memory first, clamped there to the frame
+// (kWin): every tap after that is a shared load at a fixed offset, and frame edges cost nothing more. A thread owns a
+// region column and the 8 rows of one block row, so a block candidate has one vector and one set of weights per run: per
+// row and frame one load and one dp2a, the lower tap row reused as the next row's upper one. The 2 + 2 apron rows take one
+// more pixel per thread. Errors stay in registers: the vertical 5-sums run down the thread's rows (2 rows above and below
+// from the neighbours through shared memory), the horizontal 5-sums and the choice along rows, 8 pixels per thread. Tiles
+// whose vectors differ by more than the window allows load their taps from the planes, clamped one by one.
 constexpr int kQfE = 64, kQfAp = 2, kQfTW = kQfE - 2 * kQfAp, kQfTH = 32, kQfNC = 7;
 constexpr int kQfG = kQfTH / 8;                             // block rows (thread rows) of a tile
 constexpr int kQfBX = kQfE / 8 + 4, kQfBY = kQfG + 4;       // block-field region: the tile's, the apron's, +-1 around
+constexpr int kQfWX = 80, kQfWY = 46;   // the windows: vectors of a tile within 16 px of each other across, 9 down
 constexpr int kQfVS = kQfE + 4;   // row stride of the vertical sums: 16-byte loads down 8 rows hit all banks once
 
-// the horizontal stage of a bilinear tap at 1/32 position 32 q + X: column and byte weights (left, right). kIn: the tap
-// is known to lie inside the frame; else clamped
-struct QCol {
-    int x;
-    uint32_t w;
-};
-template <bool kIn>
-__device__ __forceinline__ QCol qCol(int q, int X, int w) {
-    const int i = q + (X >> 5);
-    const uint32_t wt = ((uint32_t)X & 31u) * 255u + 32u;   // (32 - f) | f << 8
-    QCol c;
-    c.x = kIn ? i : clampi(i, 0, w - 1);      // the last column's word repeats its pixel
-    c.w = kIn || i >= 0 ? wt : 32u;           // left of the frame: pixel 0 alone
-    return c;
-}
-// a pair-plane word at a byte offset (planes are below 4 GiB)
-__device__ __forceinline__ uint32_t ldPair(const uint32_t* plane, uint32_t off) {
-    return __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(plane) + off));
-}
-// |a(q - h) - c(q + h)| in units of 2^-14 at pixel (qx, qy) for R = rne(32 h)
-template <bool kIn>
-__device__ __forceinline__ uint32_t qErr(const PixfieldParams& p, int qx, int qy, int Rx, int Ry) {
-    const QCol ca = qCol<kIn>(qx, -Rx, p.w), cc = qCol<kIn>(qx, Rx, p.w);
-    const int ya = qy + ((-Ry) >> 5), yc = qy + (Ry >> 5);
-    const uint32_t fa = (uint32_t)(-Ry) & 31u, fc = (uint32_t)Ry & 31u;
-    uint32_t oa = 4u * (uint32_t)((kIn ? ya : clampi(ya, 0, p.h - 1)) * p.w + ca.x);
-    uint32_t oc = 4u * (uint32_t)((kIn ? yc : clampi(yc, 0, p.h - 1)) * p.w + cc.x);
-    const uint32_t a0 = __dp2a_lo(ldPair(p.pa, oa), ca.w, 0u), c0 = __dp2a_lo(ldPair(p.pc, oc), cc.w, 0u);
-    if (kIn) {
-        oa += 4u * (uint32_t)p.w;
-        oc += 4u * (uint32_t)p.w;
-    } else {
-        oa = 4u * (uint32_t)(clampi(ya + 1, 0, p.h - 1) * p.w + ca.x);
-        oc = 4u * (uint32_t)(clampi(yc + 1, 0, p.h - 1) * p.w + cc.x);
-    }
-    const uint32_t a1 = __dp2a_lo(ldPair(p.pa, oa), ca.w, 0u), c1 = __dp2a_lo(ldPair(p.pc, oc), cc.w, 0u);
-    return __usad(a0 * (32u - fa) + a1 * fa, c0 * (32u - fc) + c1 * fc, 0u);
+// (32 - f) | f << 8, f = X & 31: a tap pair's byte weights (left, right) at 1/32 position X
+__device__ __forceinline__ uint32_t qWeights(int X) { return ((uint32_t)X & 31u) * 255u + 32u; }
+// a pair-plane word, clamped (the last column's word repeats its pixel; left of the frame both halves are pixel 0)
+__device__ __forceinline__ uint32_t ldPairClamped(const uint32_t* plane, int w, int h, int x, int y) {
+    const uint32_t v = __ldg(plane + (size_t)clampi(y, 0, h - 1) * w + clampi(x, 0, w - 1));
+    return x < 0 ? __byte_perm(v, v, 0x1010) : v;
 }
 
 struct QfTile {
@@ -350,14 +339,43 @@ struct QfTile {
     uint32_t below[kQfG + 1][2][kQfE];         // ... below thread row i - 1 (kQfG: the apron's)
     alignas(16) uint32_t v[kQfTH][kQfVS];      // the vertical 5-sums
     uint8_t pick[kQfTH][kQfE];
+    int4 range[4];                             // per warp: the least and largest R (x, y) of its block vectors
+    uint32_t differ;                           // bit k: candidate k (2 .. 5) is not the own block's everywhere
+    alignas(8) uint32_t win[2][kQfWY * kQfWX];   // pair words of a and c
 };
+// the windows' origins
+struct QfWin {
+    int ax, ay, cx, cy;
+};
+// |a(q - h) - c(q + h)| in units of 2^-14 at pixel (qx, qy) for R = rne(32 h)
+template <bool kWin>
+__device__ __forceinline__ uint32_t qErr(const PixfieldParams& p, const QfTile& t, const QfWin& o, int qx, int qy, int Rx, int Ry) {
+    const int xa = qx + ((-Rx) >> 5), ya = qy + ((-Ry) >> 5), xc = qx + (Rx >> 5), yc = qy + (Ry >> 5);
+    const uint32_t wa = qWeights(-Rx), wc = qWeights(Rx), fa = (uint32_t)(-Ry) & 31u, fc = (uint32_t)Ry & 31u;
+    uint32_t a0, a1, c0, c1;
+    if (kWin) {
+        const uint32_t* qa = t.win[0] + (ya - o.ay) * kQfWX + xa - o.ax;
+        const uint32_t* qc = t.win[1] + (yc - o.cy) * kQfWX + xc - o.cx;
+        a0 = qa[0];
+        a1 = qa[kQfWX];
+        c0 = qc[0];
+        c1 = qc[kQfWX];
+    } else {
+        a0 = ldPairClamped(p.pa, p.w, p.h, xa, ya);
+        a1 = ldPairClamped(p.pa, p.w, p.h, xa, ya + 1);
+        c0 = ldPairClamped(p.pc, p.w, p.h, xc, yc);
+        c1 = ldPairClamped(p.pc, p.w, p.h, xc, yc + 1);
+    }
+    return __usad(__dp2a_lo(a0, wa, 0u) * (32u - fa) + __dp2a_lo(a1, wa, 0u) * fa,
+                  __dp2a_lo(c0, wc, 0u) * (32u - fc) + __dp2a_lo(c1, wc, 0u) * fc, 0u);
+}
 
-template <bool kIn>
-__device__ __forceinline__ void pixfieldQTile(const PixfieldParams& p, QfTile& t, int X0, int Y0) {
+template <bool kWin>
+__device__ __forceinline__ void pixfieldQTile(const PixfieldParams& p, QfTile& t, const QfWin& o, int X0, int Y0) {
     const int tid = threadIdx.x, ex = tid & (kQfE - 1), g = tid >> 6;
     const int bx0 = (X0 >> 3) - 2, by0 = (Y0 >> 3) - 2;
     // this thread's column; the columns and weights of cv2.resize x8 (weights (1, 0) beyond the borders)
-    const int qx = kIn ? X0 - kQfAp + ex : clampi(X0 - kQfAp + ex, 0, p.w - 1);
+    const int qx = clampi(X0 - kQfAp + ex, 0, p.w - 1);
     const int bx = (qx >> 3) - bx0;
     int cx0;
     float ca0, ca1;
@@ -390,38 +408,37 @@ __device__ __forceinline__ void pixfieldQTile(const PixfieldParams& p, QfTile& t
     int pk[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) { best[i] = FLT_MAX; pk[i] = 0; }
-    const uint32_t rowB = 4u * (uint32_t)p.w;
+    const uint32_t cands = t.differ | 0x43u;   // the bilinear, own-block and zero candidates always
     for (int k = 0; k < kQfNC; k++) {
+        if (!((cands >> k) & 1u)) continue;
         uint32_t e[8], ea;   // the run's and the apron pixel's errors
         if (k == 0) {   // the upsampled field: a vector per pixel
             const float2 lo = colField(br - 1), mid = colField(br), hi = colField(br + 1);
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 const float2 r = rne32bits(rowField(lo, mid, hi, j));
-                e[j] = qErr<kIn>(p, qx, qy0 + j, __float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
+                e[j] = qErr<kWin>(p, t, o, qx, qy0 + j, __float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
             }
-            if (!kIn && (qy0 & 7)) {   // a run below the frame: its rows repeat row h - 1
+            if (qy0 & 7) {   // a run below the frame: its rows repeat row h - 1
                 const float2 r = rne32bits(rowField(lo, mid, hi, qy0 & 7));
-                e[0] = qErr<kIn>(p, qx, qy0, __float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
+                e[0] = qErr<kWin>(p, t, o, qx, qy0, __float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
             }
             const float2 r = rne32bits(rowField(colField(abr - 1), colField(abr), colField(abr + 1), ay & 7));
-            ea = qErr<kIn>(p, qx, ay, __float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
+            ea = qErr<kWin>(p, t, o, qx, ay, __float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
         } else if (k < kQfNC - 1) {   // the vector of the pixel's own block or of a 4-neighbour
             const int dx = k == 4 ? -1 : (k == 5 ? 1 : 0), dy = k == 2 ? -1 : (k == 3 ? 1 : 0);
             const int2 Ra = t.bR[abr + dy][bx + dx];
-            ea = qErr<kIn>(p, qx, ay, Ra.x, Ra.y);
+            ea = qErr<kWin>(p, t, o, qx, ay, Ra.x, Ra.y);
             const int2 R = t.bR[br + dy][bx + dx];
-            const QCol ca = qCol<kIn>(qx, -R.x, p.w), cc = qCol<kIn>(qx, R.x, p.w);
-            const uint32_t fa = (uint32_t)(-R.y) & 31u, fc = (uint32_t)R.y & 31u, ga = 32u - fa, gc = 32u - fc;
-            const int ya = qy0 + ((-R.y) >> 5), yc = qy0 + (R.y >> 5);
-            if (kIn || __all_sync(0xffffffffu, min(ya, yc) >= 0 && max(ya, yc) + 8 < p.h)) {
-                uint32_t oa = 4u * (uint32_t)(ya * p.w + ca.x), oc = 4u * (uint32_t)(yc * p.w + cc.x);
-                uint32_t ta = __dp2a_lo(ldPair(p.pa, oa), ca.w, 0u), tc = __dp2a_lo(ldPair(p.pc, oc), cc.w, 0u);
+            if (kWin) {
+                const uint32_t wa = qWeights(-R.x), wc = qWeights(R.x);
+                const uint32_t fa = (uint32_t)(-R.y) & 31u, fc = (uint32_t)R.y & 31u, ga = 32u - fa, gc = 32u - fc;
+                const uint32_t* qa = t.win[0] + (qy0 + ((-R.y) >> 5) - o.ay) * kQfWX + qx + ((-R.x) >> 5) - o.ax;
+                const uint32_t* qc = t.win[1] + (qy0 + (R.y >> 5) - o.cy) * kQfWX + qx + (R.x >> 5) - o.cx;
+                uint32_t ta = __dp2a_lo(qa[0], wa, 0u), tc = __dp2a_lo(qc[0], wc, 0u);
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    oa += rowB;
-                    oc += rowB;
-                    const uint32_t ua = __dp2a_lo(ldPair(p.pa, oa), ca.w, 0u), uc = __dp2a_lo(ldPair(p.pc, oc), cc.w, 0u);
+                    const uint32_t ua = __dp2a_lo(qa[(j + 1) * kQfWX], wa, 0u), uc = __dp2a_lo(qc[(j + 1) * kQfWX], wc, 0u);
                     e[j] = __usad(ta * ga + ua * fa, tc * gc + uc * fc, 0u);
                     ta = ua;
                     tc = uc;
@@ -429,21 +446,21 @@ __device__ __forceinline__ void pixfieldQTile(const PixfieldParams& p, QfTile& t
             } else {
 #pragma unroll 1
                 for (int j = 0; j < 8; j++) {
-                    const uint32_t v = qErr<kIn>(p, qx, qy0 + j, R.x, R.y);
+                    const uint32_t v = qErr<kWin>(p, t, o, qx, qy0 + j, R.x, R.y);
 #pragma unroll
                     for (int i = 0; i < 8; i++) e[i] = i == j ? v : e[i];
                 }
             }
         } else {   // zero: the pixels themselves (weights 32 x 32)
             auto err0 = [&](int y) {
-                const uint32_t o = 4u * (uint32_t)((kIn ? y : clampi(y, 0, p.h - 1)) * p.w + qx);
-                return __usad(ldPair(p.pa, o) & 0xFFFFu, ldPair(p.pc, o) & 0xFFFFu, 0u) << 10;
+                const size_t i = (size_t)clampi(y, 0, p.h - 1) * p.w + qx;
+                return __usad(__ldg(p.pa + i) & 0xFFFFu, __ldg(p.pc + i) & 0xFFFFu, 0u) << 10;
             };
 #pragma unroll
             for (int j = 0; j < 8; j++) e[j] = err0(qy0 + j);
             ea = err0(ay);
         }
-        if (!kIn && rows < 8) {   // the frame's last row stands for the rows below it
+        if (rows < 8) {   // the frame's last row stands for the rows below it
 #pragma unroll
             for (int j = 1; j < 8; j++)
                 if (j >= rows) e[j] = e[j - 1];
@@ -497,7 +514,7 @@ __device__ __forceinline__ void pixfieldQTile(const PixfieldParams& p, QfTile& t
     const int lx = ex - kQfAp;
     if ((unsigned)lx >= (unsigned)kQfTW || X0 + lx >= p.w || Y0 + 8 * g >= p.h) return;
     const float2 lo = colField(br - 1), mid = colField(br), hi = colField(br + 1);
-    float2* o = p.pf + (size_t)qy0 * p.w + X0 + lx;
+    float2* dst = p.pf + (size_t)qy0 * p.w + X0 + lx;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
         if (j >= rows) break;
@@ -505,41 +522,198 @@ __device__ __forceinline__ void pixfieldQTile(const PixfieldParams& p, QfTile& t
         float2 v = make_float2(0.0f, 0.0f);
         if (k == 0) v = rowField(lo, mid, hi, j);
         else if (k < kQfNC - 1) v = t.bv[br + (k == 2 ? -1 : (k == 3 ? 1 : 0))][bx + (k == 4 ? -1 : (k == 5 ? 1 : 0))];
-        o[(size_t)j * p.w] = v;
+        dst[(size_t)j * p.w] = v;
     }
 }
-// CTA `cta` of an item: its tiles in raster order, then the CTAs that sum the leaves of the scene-cut mean, a warp each
-// (the sub-pixel launch before this one wrote the SADs)
+// interp.estimate :189-190, the mean of the sub-pixel pass' SADs in numpy's pairwise order, by the pixel-field launch's first
+// CTAs (beside its tiles; the synthesis is the first to need the decision). A warp sums a leaf of the tree: the leaf in
+// registers by 4 coalesced loads, handed round by shuffles in numpy's order. The CTA that completes the last leaf adds the
+// inner nodes, one height per step, from shared memory: a chain of dependent global loads per leaf and height took ~15 us
+// and was the tail of this launch (43 us at 4K, 17 us at 640x360).
+__device__ __forceinline__ float leafSum(const float* a, int n, int lane, unsigned int& s256) {
+    float v[4];
+    unsigned int s = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        v[k] = lane + 32 * k < n ? __ldcg(a + lane + 32 * k) : 0.0f;
+        s += (unsigned int)__float2int_rn(__fmul_rn(v[k], 256.0f));
+    }
+    s256 = __reduce_add_sync(0xffffffffu, s);
+    const int body = n >= 8 ? n - n % 8 : 0;   // below 8 elements they are added one by one from 0
+    float res = 0.0f;
+    if (body) {
+        float r = v[0];   // lanes 0..7: numpy's 8 accumulators
+#pragma unroll
+        for (int m = 1; m < 16; m++) {
+            const float x = __shfl_sync(0xffffffffu, v[m / 4], 8 * (m % 4) + (lane & 7));
+            if (8 * m < body) r = __fadd_rn(r, x);
+        }
+        const float p2 = __fadd_rn(r, __shfl_down_sync(0xffffffffu, r, 1));      // lane 2k: r[2k] + r[2k + 1]
+        const float p4 = __fadd_rn(p2, __shfl_down_sync(0xffffffffu, p2, 2));    // lane 4k: (r0 + r1) + (r2 + r3)
+        res = __fadd_rn(p4, __shfl_down_sync(0xffffffffu, p4, 4));
+    }
+    for (int i = body; i < n; i++) {
+        const float x = i < 32 ? v[0] : (i < 64 ? v[1] : (i < 96 ? v[2] : v[3]));
+        res = __fadd_rn(res, __shfl_sync(0xffffffffu, x, i & 31));
+    }
+    return res;   // lane 0
+}
+__device__ __forceinline__ void cutMeanQCta(const PixfieldParams& p, int cta, uint32_t* sm, size_t smBytes) {
+    const CutPlan& pl = p.plan;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, leaf = cta * 8 + warp;
+    __shared__ unsigned int last, tot;
+    if (leaf < pl.nLeaves) {
+        const int2 lf = pl.leaves[leaf];
+        unsigned int s256;
+        const float v = leafSum(p.sads + lf.x, lf.y, lane, s256);
+        if (lane == 0) {
+            pl.gvals[leaf] = v;
+            pl.leafS256[leaf] = s256;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        const unsigned int n = (unsigned int)min(8, pl.nLeaves - cta * 8);
+        last = atomicAdd(&p.st->subDone, n) + n == (unsigned int)pl.nLeaves;
+        tot = 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // node values and the inner nodes' operands in shared memory where they fit (else the values stay in gvals)
+    const bool fits = (size_t)pl.nLeaves * 16 <= smBytes;
+    float* vals = fits ? reinterpret_cast<float*>(sm) : pl.gvals;
+    int2* inner = reinterpret_cast<int2*>(sm + 2 * pl.nLeaves);
+    unsigned int s = 0;
+    for (int i = tid; i < pl.nLeaves; i += 256) {
+        s += __ldcg(pl.leafS256 + i);
+        if (fits) vals[i] = __ldcg(pl.gvals + i);
+        if (fits && i < pl.nInner) inner[i] = __ldg(pl.inner + i);
+    }
+    s = __reduce_add_sync(0xffffffffu, s);
+    if (lane == 0) atomicAdd(&tot, s);
+    __syncthreads();
+    for (int d = 0; d < pl.nSteps; d++) {
+        for (int j = pl.depthStart[d] + tid; j < pl.depthStart[d + 1]; j += 256) {
+            if (fits) {
+                const int2 c = inner[j];
+                vals[pl.nLeaves + j] = __fadd_rn(vals[c.x], vals[c.y]);
+            } else {
+                const int2 c = __ldg(pl.inner + j);
+                __stcg(pl.gvals + pl.nLeaves + j, __fadd_rn(__ldcg(pl.gvals + c.x), __ldcg(pl.gvals + c.y)));
+                __threadfence();
+            }
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        const float mean = __fdiv_rn(fits ? vals[pl.root] : __ldcg(pl.gvals + pl.root), (float)(p.bw * p.bh));
+        p.st->sadMean = mean;
+        p.st->cut = mean > p.cutSad ? 1u : 0u;
+        p.st->sadSum256 = tot;
+        p.st->subDone = 0;
+    }
+}
+
+// CTA `cta` of an item: the CTAs of the scene-cut mean, then the tiles in raster order
 __device__ __forceinline__ void pixfieldQCta(const PixfieldParams& p, int cta) {
     __shared__ QfTile t;
-    const int gx = (p.w + kQfTW - 1) / kQfTW, tiles = gx * ((p.h + kQfTH - 1) / kQfTH);
-    if (cta >= tiles) {
-        const int leaf = (cta - tiles) * 8 + (int)(threadIdx.x >> 5);
-        if (leaf < p.plan.nLeaves) cutMeanLeaf(p.plan, p.sads, p.bw * p.bh, p.cutSad, p.st, leaf, threadIdx.x & 31);
+    const int cutCtas = (p.plan.nLeaves + 7) / 8;
+    if (cta < cutCtas) {
+        cutMeanQCta(p, cta, &t.win[0][0], sizeof(t.win));
         return;
     }
+    cta -= cutCtas;
+    const int gx = (p.w + kQfTW - 1) / kQfTW;
     const int X0 = cta % gx * kQfTW, Y0 = cta / gx * kQfTH;
-    // the block-field region, clamped to the field (a replicated entry stands for every block outside); the tile is
-    // interior if no vector of the region (nor any blend of them) takes a tap of the tile's pixels outside the frame
+    // the block-field region, clamped to the field (a replicated entry stands for every block outside), and the range of
+    // its vectors (in 1/32 px): every candidate is one of them or a blend
     const int bx0 = (X0 >> 3) - 2, by0 = (Y0 >> 3) - 2;
-    bool out = false;
-    for (int i = threadIdx.x; i < kQfBX * kQfBY; i += 256) {
-        const float2 v = __ldg(p.v + clampi(by0 + i / kQfBX, 0, p.bh - 1) * p.bw + clampi(bx0 + i % kQfBX, 0, p.bw - 1));
-        t.bv[i / kQfBX][i % kQfBX] = v;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    static_assert(kQfBX * kQfBY == 96, "three warps hold the block-field region");
+    if (tid < 96) {
+        const float2 v = __ldg(p.v + clampi(by0 + tid / kQfBX, 0, p.bh - 1) * p.bw + clampi(bx0 + tid % kQfBX, 0, p.bw - 1));
+        t.bv[tid / kQfBX][tid % kQfBX] = v;
         const float2 r = rne32bits(v);
         const int2 R = make_int2(__float_as_int(r.x) - 0x4B400000, __float_as_int(r.y) - 0x4B400000);
-        t.bR[i / kQfBX][i % kQfBX] = R;
-        const int dx = (abs(R.x) >> 5) + 2, dy = (abs(R.y) >> 5) + 2;
-        out |= X0 - kQfAp - dx < 0 || X0 + kQfTW + kQfAp + dx > p.w || Y0 - kQfAp - dy < 0 || Y0 + kQfTH + kQfAp + dy > p.h;
+        t.bR[tid / kQfBX][tid % kQfBX] = R;
+        const int4 m = make_int4(__reduce_min_sync(0xffffffffu, R.x), __reduce_min_sync(0xffffffffu, R.y),
+                                 __reduce_max_sync(0xffffffffu, R.x), __reduce_max_sync(0xffffffffu, R.y));
+        if (lane == 0) t.range[warp] = m;
     }
-    if (__syncthreads_or(out)) pixfieldQTile<false>(p, t, X0, Y0);
-    else pixfieldQTile<true>(p, t, X0, Y0);
+    if (tid == 96) t.differ = 0;
+    __syncthreads();
+    // a neighbour candidate that names the own block's vector everywhere costs the same at every pixel and can never be
+    // the first minimum: it is left out (still scenes, wide uniform motion)
+    if (tid < 96) {
+        const int r = tid / kQfBX, c = tid % kQfBX;
+        const int2 R = t.bR[r][c], u = t.bR[max(r - 1, 0)][c], d = t.bR[min(r + 1, kQfBY - 1)][c];
+        const int2 l = t.bR[r][max(c - 1, 0)], e = t.bR[r][min(c + 1, kQfBX - 1)];
+        auto ne = [&](const int2& q) { return q.x != R.x || q.y != R.y; };
+        const uint32_t m = (ne(u) ? 4u : 0u) | (ne(d) ? 8u : 0u) | (ne(l) ? 16u : 0u) | (ne(e) ? 32u : 0u);
+        const uint32_t any = __reduce_or_sync(0xffffffffu, m);
+        if (lane == 0 && any) atomicOr(&t.differ, any);
+    }
+    const int4 r0 = t.range[0], r1 = t.range[1], r2 = t.range[2];
+    const int nx = min(r0.x, min(r1.x, r2.x)), ny = min(r0.y, min(r1.y, r2.y));
+    const int mx = max(r0.z, max(r1.z, r2.z)), my = max(r0.w, max(r1.w, r2.w));
+    QfWin o;
+    o.ax = X0 - kQfAp + ((-mx) >> 5);
+    o.ay = Y0 - kQfAp + ((-my) >> 5);
+    o.cx = X0 - kQfAp + (nx >> 5);
+    o.cy = Y0 - kQfAp + (ny >> 5);
+    // columns and rows (and the taps' lower row) from the origin to the other end of the range
+    const int ww = kQfE + max(((-nx) >> 5) - ((-mx) >> 5), (mx >> 5) - (nx >> 5));
+    const int wh = kQfTH + 2 * kQfAp + 1 + max(((-ny) >> 5) - ((-my) >> 5), (my >> 5) - (ny >> 5));
+    if (ww > kQfWX || wh > kQfWY) {
+        __syncthreads();
+        pixfieldQTile<false>(p, t, o, X0, Y0);
+        return;
+    }
+    if (min(o.ax, o.cx) >= 0 && min(o.ay, o.cy) >= 0 && max(o.ax, o.cx) + ww <= p.w && max(o.ay, o.cy) + wh <= p.h) {
+        const uint32_t* qa = p.pa + (size_t)(o.ay + warp) * p.w + o.ax + lane;
+        const uint32_t* qc = p.pc + (size_t)(o.cy + warp) * p.w + o.cx + lane;
+        uint32_t* wa = t.win[0] + warp * kQfWX + lane;
+        const bool more = lane + 64 < ww;
+        for (int r = warp; r < wh; r += 8) {   // (ww >= 64)
+            const uint32_t a0 = __ldg(qa), a1 = __ldg(qa + 32), c0 = __ldg(qc), c1 = __ldg(qc + 32);
+            const uint32_t a2 = more ? __ldg(qa + 64) : 0u, c2 = more ? __ldg(qc + 64) : 0u;
+            qa += 8 * p.w;
+            qc += 8 * p.w;
+            wa[0] = a0;
+            wa[32] = a1;
+            wa[kQfWY * kQfWX] = c0;
+            wa[kQfWY * kQfWX + 32] = c1;
+            if (more) {
+                wa[64] = a2;
+                wa[kQfWY * kQfWX + 64] = c2;
+            }
+            wa += 8 * kQfWX;
+        }
+    } else {
+        for (int r = warp; r < wh; r += 8)
+            for (int c = lane; c < ww; c += 32) {
+                t.win[0][r * kQfWX + c] = ldPairClamped(p.pa, p.w, p.h, o.ax + c, o.ay + r);
+                t.win[1][r * kQfWX + c] = ldPairClamped(p.pc, p.w, p.h, o.cx + c, o.cy + r);
+            }
+    }
+    __syncthreads();
+    pixfieldQTile<true>(p, t, o, X0, Y0);
 }
-__global__ void __launch_bounds__(256, 4) k_pixfield_q(const PixfieldParams p) {
+// 3 CTAs per SM: 4 (64 registers) spill in every candidate's loop (640x360's estimate 40 us against 48, 1080p 75 against
+// 83, 4K the same)
+__global__ void __launch_bounds__(256, 3) k_pixfield_q(const PixfieldParams p) {
     pdlEnter();
     pixfieldQCta(p, blockIdx.x);
 }
-__global__ void __launch_bounds__(256, 4) k_pixfield_q_m(const __grid_constant__ Merged<PixfieldParams> m) {
+// grids of at most 2 CTAs per SM: the registers of a third one (an estimate at 640x360 36 -> 34 us, 1080p 69 -> 66; 4K, 1120
+// CTAs, 143 -> 147)
+__global__ void __launch_bounds__(256, 2) k_pixfield_q_lat(const PixfieldParams p) {
+    pdlEnter();
+    pixfieldQCta(p, blockIdx.x);
+}
+__global__ void __launch_bounds__(256, 3) k_pixfield_q_m(const __grid_constant__ Merged<PixfieldParams> m) {
     pdlEnter();
     int bx, by;
     const int i = mergedItem(m, bx, by);
@@ -584,7 +758,8 @@ static int pixfieldQCtas(const PixfieldParams& p) {
     return (int)(divUp(p.w, kQfTW) * divUp(p.h, kQfTH) + divUp(p.plan.nLeaves, 8));
 }
 cudaError_t launchPixfieldQ(const PixfieldParams& p, cudaStream_t s) {
-    return launchPdl(k_pixfield_q, dim3(pixfieldQCtas(p)), dim3(256), 0, s, p);
+    const int ctas = pixfieldQCtas(p);
+    return launchPdl(ctas <= 2 * smCount() ? k_pixfield_q_lat : k_pixfield_q, dim3(ctas), dim3(256), 0, s, p);
 }
 cudaError_t launchPixfieldQMerged(Merged<PixfieldParams>& m, cudaStream_t s) {
     const int total = layoutMerged(m, [](const PixfieldParams& p, int& gx) { return gx = pixfieldQCtas(p); });

@@ -234,6 +234,40 @@ __device__ __forceinline__ int rneDiv(int num, int n) {
     return q;
 }
 
+// the cells of a tile off the vector path, as lumaCells of the 8-bit pass: 4 cells per thread, their loads in flight together
+template <int F, int FS>
+__device__ __forceinline__ void lumaFmtCells(const LumaPyrParams& p, float (*sl)[kTowerFloats], int tx0, int ty0) {
+    const int fw = p.lw[0], fh = p.lh[0];
+#pragma unroll (FS == 4 || F == kFmtF16 ? 1 : 4)
+    for (int q = 0; q < 4; q++) {
+        const int i = (int)threadIdx.x + 256 * q, x = tx0 + (i & 31), y = ty0 + (i >> 5);
+        float va = 0.0f, vc = 0.0f;
+        if (x < fw && y < fh) {
+            int sa = 0, sc = 0, n = 0;
+#pragma unroll
+            for (int j = 0; j < FS; j++)
+#pragma unroll
+                for (int k = 0; k < FS; k++) {
+                    const int xx = x * FS + k, yy = y * FS + j;
+                    const bool ok = xx < p.W && yy < p.H;
+                    const int cx = min(xx, p.W - 1), cy = min(yy, p.H - 1);
+                    const int qa = lumaQ<F>(p.f, p.a, p.pitch, cx, cy, p.pq), qc = lumaQ<F>(p.f, p.c, p.pitch, cx, cy, p.pq);
+                    sa += ok ? qa : 0;
+                    sc += ok ? qc : 0;
+                    n += ok;
+                }
+            va = __fmul_rn(i2f(rneDiv(4 * sa, n)), 1.0f / 16.0f);
+            vc = __fmul_rn(i2f(rneDiv(4 * sc, n)), 1.0f / 16.0f);
+            if (p.la[0]) {
+                p.la[0][(size_t)y * fw + x] = va;
+                p.lc[0][(size_t)y * fw + x] = vc;
+            }
+        }
+        sl[0][i] = va;
+        sl[1][i] = vc;
+    }
+}
+
 // interp.flow + pyramid for the other formats: one CTA = a 32x32 level-0 tile and its tower (as k_luma_pyr). Whole tiles of
 // aligned frames at flowScale 2 (p.vec16) take 4 frame pixels x 2 rows per thread and load (4K: Rgb10 49 -> 31 us, linear
 // RgbaF16 78 -> 66, Nv12 35 -> 20, P010 37 -> 21): bound by instruction issue, linear RgbaF16 by its table gathers.
@@ -272,32 +306,9 @@ __device__ __forceinline__ void lumaFmtCta(const LumaPyrParams& p, int bx, int b
         lumaTower<true>(p, sl, tx0, ty0);
         return;
     }
-    for (int i = threadIdx.x; i < 1024; i += 256) {
-        const int x = tx0 + (i & 31), y = ty0 + (i >> 5);
-        float va = 0.0f, vc = 0.0f;
-        if (x < fw && y < fh) {
-            int sa = 0, sc = 0, n = 0;
-            for (int j = 0; j < fs; j++) {
-                const int yy = y * fs + j;
-                if (yy >= p.H) break;
-                for (int k = 0; k < fs; k++) {
-                    const int xx = x * fs + k;
-                    if (xx >= p.W) break;
-                    sa += lumaQ<F>(p.f, p.a, p.pitch, xx, yy, p.pq);
-                    sc += lumaQ<F>(p.f, p.c, p.pitch, xx, yy, p.pq);
-                    n++;
-                }
-            }
-            va = __fmul_rn(i2f(rneDiv(4 * sa, n)), 1.0f / 16.0f);
-            vc = __fmul_rn(i2f(rneDiv(4 * sc, n)), 1.0f / 16.0f);
-            if (p.la[0]) {
-                p.la[0][(size_t)y * fw + x] = va;
-                p.lc[0][(size_t)y * fw + x] = vc;
-            }
-        }
-        sl[0][i] = va;
-        sl[1][i] = vc;
-    }
+    if (fs == 2) lumaFmtCells<F, 2>(p, sl, tx0, ty0);
+    else if (fs == 1) lumaFmtCells<F, 1>(p, sl, tx0, ty0);
+    else lumaFmtCells<F, 4>(p, sl, tx0, ty0);
     __syncthreads();
     storePairs(p, sl, tx0, ty0);
     lumaTower<true>(p, sl, tx0, ty0);

@@ -17,6 +17,51 @@
 namespace fgk {
 
 // ============================================================================================== luma + pyramid
+// the level-0 cells of a 32x32 tile at the frame's edge, or of a frame off the vector path: 4 cells per thread, every load of
+// a pair of cells in flight at once (pixels past the frame are read at the edge and not counted). With a loop per pixel
+// these tiles were the latency of the whole pass (1080p 14 us, now 6).
+template <int FS>
+__device__ __forceinline__ void lumaCells(const LumaPyrParams& p, float (*sl)[kTowerFloats], int tx0, int ty0) {
+    const int fw = p.lw[0], fh = p.lh[0];
+#pragma unroll (FS == 4 ? 1 : 4)
+    for (int q = 0; q < 4; q++) {
+        const int i = (int)threadIdx.x + 256 * q, x = tx0 + (i & 31), y = ty0 + (i >> 5);
+        float va = 0.0f, vc = 0.0f;
+        if (x < fw && y < fh) {
+            int sa = 0, sc = 0, n = 0;
+#pragma unroll
+            for (int j = 0; j < FS; j++)
+#pragma unroll
+                for (int k = 0; k < FS; k++) {
+                    const int xx = x * FS + k, yy = y * FS + j;
+                    const bool ok = xx < p.W && yy < p.H;
+                    const size_t o = (size_t)min(yy, p.H - 1) * p.pitch + (size_t)min(xx, p.W - 1) * 4;
+                    const int ga = gray8(__ldg(reinterpret_cast<const uint32_t*>(p.a + o)), p.ri, p.gi, p.bi);
+                    const int gc = gray8(__ldg(reinterpret_cast<const uint32_t*>(p.c + o)), p.ri, p.gi, p.bi);
+                    sa += ok ? ga : 0;
+                    sc += ok ? gc : 0;
+                    n += ok;
+                }
+            if (FS == 1) {
+                va = (float)sa;
+                vc = (float)sc;
+            } else if (n == FS * FS) {
+                va = __fmul_rn((float)sa, 1.0f / (float)(FS * FS));
+                vc = __fmul_rn((float)sc, 1.0f / (float)(FS * FS));
+            } else {
+                va = __fdiv_rn((float)sa, (float)n);
+                vc = __fdiv_rn((float)sc, (float)n);
+            }
+            if (p.la[0]) {
+                p.la[0][(size_t)y * fw + x] = va;
+                p.lc[0][(size_t)y * fw + x] = vc;
+            }
+        }
+        sl[0][i] = va;
+        sl[1][i] = vc;
+    }
+}
+
 // interp.flow :149-152 + interp.pyramid :73-77. One CTA = a 32x32 tile of level 0 (32 fs x 32 fs frame pixels) and
 // the aligned 16x16 .. 1x1 tiles of levels 1..5 above it: a level-(l+1) pixel only averages the 2x2 level-l pixels
 // below it, so the whole tower stays inside the tile. Mean of the valid pixels: sum * 1/n^2 when full, sum / count
@@ -60,45 +105,10 @@ __device__ __forceinline__ void lumaPyrCta(const LumaPyrParams& p, int bx, int b
         __syncthreads();
         lumaTower<false>(p, sl, tx0, ty0);
         return;
-    } else {
-        for (int i = threadIdx.x; i < 1024; i += 256) {
-            const int x = tx0 + (i & 31), y = ty0 + (i >> 5);
-            float va = 0.0f, vc = 0.0f;
-            if (x < fw && y < fh) {
-                int sa = 0, sc = 0, n = 0;
-                for (int j = 0; j < fs; j++) {
-                    const int yy = y * fs + j;
-                    if (yy >= p.H) break;
-                    const uint32_t* ra = reinterpret_cast<const uint32_t*>(p.a + (size_t)yy * p.pitch);
-                    const uint32_t* rc = reinterpret_cast<const uint32_t*>(p.c + (size_t)yy * p.pitch);
-                    for (int k = 0; k < fs; k++) {
-                        const int xx = x * fs + k;
-                        if (xx >= p.W) break;
-                        sa += gray8(__ldg(ra + xx), p.ri, p.gi, p.bi);
-                        sc += gray8(__ldg(rc + xx), p.ri, p.gi, p.bi);
-                        n++;
-                    }
-                }
-                if (fs == 1) {
-                    va = (float)sa;
-                    vc = (float)sc;
-                } else if (n == fs * fs) {
-                    const float inv = 1.0f / (float)(fs * fs);
-                    va = __fmul_rn((float)sa, inv);
-                    vc = __fmul_rn((float)sc, inv);
-                } else {
-                    va = __fdiv_rn((float)sa, (float)n);
-                    vc = __fdiv_rn((float)sc, (float)n);
-                }
-                if (p.la[0]) {
-                    p.la[0][(size_t)y * fw + x] = va;
-                    p.lc[0][(size_t)y * fw + x] = vc;
-                }
-            }
-            sl[0][i] = va;
-            sl[1][i] = vc;
-        }
     }
+    if (fs == 2) lumaCells<2>(p, sl, tx0, ty0);
+    else if (fs == 1) lumaCells<1>(p, sl, tx0, ty0);
+    else lumaCells<4>(p, sl, tx0, ty0);
     __syncthreads();
     if (p.pa) storePairs(p, sl, tx0, ty0);
     lumaTower<false>(p, sl, tx0, ty0);
@@ -576,6 +586,72 @@ __device__ __forceinline__ void medianFromHist(const Median3Params& p, const uns
     if (tid == 0) {
         p.medOut[0] = (float)(found[0] + found[1]);
         p.medOut[1] = (float)(found[2] + found[3]);
+    }
+}
+
+// interp.search at integer steps for the smallest levels (at most kSearchSplitBlocks blocks: the GPU is mostly idle, a
+// level costs its latency): a CTA of 4 warps per block, as k_search_r but with the window staged and the rows of all dy
+// (8 (2 R + 1) <= 104 lanes) scored by the whole CTA at once; every warp finds the seed for itself. (An estimate at 1280x720
+// 52 -> 50 us, 1080p 72 -> 69. The level's median3 pass in the CTA that finishes last saved its launch but ran longer there
+// than in its own kernel: 1 to 2 us slower from 720p on, not kept.)
+constexpr int kSearchSplitBlocks = 1024;
+template <int R>
+__global__ void __launch_bounds__(128) k_search_s(const SearchParams p) {
+    pdlEnter();
+    constexpr int T = 8 + 2 * R, D = 2 * R + 1, NI = 8 * D;
+    static_assert(NI <= 128, "one lane per row of every dy");
+    __shared__ float sA[T * T], sC[T * T], sad[D * D];
+    const int tid = threadIdx.x, lane = tid & 31, b = blockIdx.x;
+    const int bx = b % p.bw, by = b / p.bw, b0x = bx * kBlock, b0y = by * kBlock;
+    int sx, sy;
+    searchSeed<true>(p, bx, by, lane, sx, sy);
+    const int ax0 = b0x - sx - R, ay0 = b0y - sy - R, cx0 = b0x + sx - R, cy0 = b0y + sy - R;
+#pragma unroll
+    for (int j = 0; j < (T * T + 127) / 128; j++) {
+        const int i = tid + 128 * j;
+        if (i < T * T) {
+            const int x = i % T, y = i / T;
+            sA[i] = Lc(p.la, p.w, p.h, ax0 + x, ay0 + y);
+            sC[i] = Lc(p.lc, p.w, p.h, cx0 + x, cy0 + y);
+        }
+    }
+    __syncthreads();
+    if (tid < (NI + 31) / 32 * 32) {
+        const bool act = tid < NI;
+        const int dyi = act ? (tid >> 3) : 0, y = tid & 7, dy = dyi - R;
+        const float* ra = sA + (y - dy + R) * T;
+        const float* rc = sC + (y + dy + R) * T;
+        float a[T], c[T];
+#pragma unroll
+        for (int i = 0; i < T; i++) { a[i] = ra[i]; c[i] = rc[i]; }
+#pragma unroll
+        for (int dxi = 0; dxi < D; dxi++) {
+            const int dx = dxi - R;
+            float sum = 0.0f;
+#pragma unroll
+            for (int x = 0; x < 8; x++) sum += fabsf(a[x - dx + R] - c[x + dx + R]);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+            if (act && y == 0) sad[dyi * D + dxi] = sum;
+        }
+    }
+    __syncthreads();
+    if (tid < 32) {
+        unsigned int bc = 0xffffffffu;   // costs are not negative: their bits order as they do
+        int bci = 0x7fffffff;
+        float bsad = 0.0f;
+        for (int ci = lane; ci < D * D; ci += 32) {
+            const float sd = __fmul_rn(sad[ci], 1.0f / 64.0f);
+            const unsigned int c = __float_as_uint(__fadd_rn(sd, p.pen[abs(ci % D - R) + abs(ci / D - R)]));
+            if (c < bc) { bc = c; bci = ci; bsad = sd; }
+        }
+        const unsigned int least = __reduce_min_sync(0xffffffffu, bc);
+        const int ci = (int)__reduce_min_sync(0xffffffffu, bc == least ? (unsigned int)bci : 0x7fffffffu);
+        if (bci == ci && bc == least) {
+            p.out[b] = make_float2((float)(sx + ci % D - R), (float)(sy + ci / D - R));
+            if (p.sadOut) p.sadOut[b] = bsad;
+        }
     }
 }
 
@@ -1536,6 +1612,17 @@ static cudaError_t launchSearchR(const SearchParams& p, cudaStream_t s) {
 bool searchIsQ(const SearchParams& p) { return (p.pa || p.qscale > 0.0f) && p.R <= 2 && p.bw * p.bh > kSearchLatBlocks; }
 cudaError_t launchSearch(const SearchParams& p, cudaStream_t s) {
     if (searchIsQ(p)) return launchSearchQ(p, s);
+    if (p.R <= 6 && p.bw * p.bh <= kSearchSplitBlocks) {
+        const dim3 grid(p.bw * p.bh);
+        switch (p.R) {
+            case 1: return launchPdl(k_search_s<1>, grid, dim3(128), 0, s, p);
+            case 2: return launchPdl(k_search_s<2>, grid, dim3(128), 0, s, p);
+            case 3: return launchPdl(k_search_s<3>, grid, dim3(128), 0, s, p);
+            case 4: return launchPdl(k_search_s<4>, grid, dim3(128), 0, s, p);
+            case 5: return launchPdl(k_search_s<5>, grid, dim3(128), 0, s, p);
+            default: return launchPdl(k_search_s<6>, grid, dim3(128), 0, s, p);
+        }
+    }
     switch (p.R) {
         case 1: return launchSearchR<1>(p, s);
         case 2: return launchSearchR<2>(p, s);

@@ -116,6 +116,7 @@ struct SubpixParams {
     float cutSad;
     DevState* st;
     const uint32_t* pa; const uint32_t* pc;   // level 0's pair planes (LumaPyrParams), or null: the float kernel
+    float2* med;               // on pair planes: in is the search's field, its 3x3 medians are taken here and written to med
 };
 
 struct CutMeanParams {         // the same scene-cut reduction as a separate pass (sub-pixel refinement off)

@@ -691,6 +691,10 @@ struct Interpolator::Impl {
                 for (int k = 0; k < 3; k++) sp.pen[p][k] = (float)((double)lam * (double)steps[p] * (double)k);
             sp.plan = plan; sp.cutSad = set.sceneCutSad; sp.st = st;
             sp.pa = lp.pa; sp.pc = lp.pc;
+            if (pair) {
+                sp.in = field + l0.fS;
+                sp.med = field + l0.fM;
+            }
             vfin = field + L.sub1;
         } else {
             e.cut = fgk::CutMeanParams{sads, l0.bw * l0.bh, plan, set.sceneCutSad, st};
@@ -740,7 +744,9 @@ struct Interpolator::Impl {
                                       "level 6", "level 7"};
         for (int i = e.top; i >= 0; i--) {
             if (!check(fgk::launchSearch(e.search[i], s))) return false;
-            if (!check(fgk::launchMedian3(e.med[i], s))) return false;
+            // (level 0's medians: the sub-pixel pass takes them on pair planes)
+            const bool med = !(i == 0 && set.subpixel && e.sub.med);
+            if (med && !check(fgk::launchMedian3(e.med[i], s))) return false;
             stamp(s, names[std::min(i, 7)]);
         }
         if (!check(set.subpixel ? fgk::launchSubpix(e.sub, s) : fgk::launchCutMean(e.cut, s))) return false;
@@ -1588,6 +1594,7 @@ bool Batch::Impl::mergedEstimates(cudaStream_t s, const Frame* prev, const Frame
             if (l <= plans[j].top) {
                 se.push_back(plans[j].search[l]);
                 sk.push_back(fgk::searchVariant(se.back()));
+                if (l == 0 && slots[idx[j]]->m->set.subpixel && plans[j].sub.med) continue;   // the sub-pixel pass takes them
                 me.push_back(plans[j].med[l]);
                 mk.push_back(fgk::median3Variant(me.back()));
             }

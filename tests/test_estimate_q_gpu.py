@@ -67,3 +67,40 @@ def test_flow_scale_4():
 def test_formats_integer_levels(name):
     p, c, _ = workloads.flow_pair(515, 301, seed=77)
     check(name, p, c, [0.5], settings=oracle.Settings(flowScale=1))
+
+
+def test_vectors_wider_apart_than_the_window():
+    """halves of a frame moving 26 px apart from each other: tiles whose vectors differ by more than the staged window"""
+    W, H = 256, 176
+    a = workloads.value_noise(H, W + 64, np.random.Generator(np.random.PCG64(3)))
+    p = workloads._to_rgba(a[:, 32:32 + W])
+    c = np.concatenate([workloads._to_rgba(a[:, 32 + 26:32 + 26 + W // 2]), workloads._to_rgba(a[:, 32 + W // 2 - 26:32 + W - 26])], axis=1)
+    check_against_oracle(p, c, [0.5], oracle.Settings(flowScale=1, globalFallback=1.0, sceneCutSad=250.0))
+
+
+def test_still_and_uniform_motion():
+    """every neighbour's vector the own block's: candidates left out; and a still frame with one moving sprite"""
+    p, c, _ = workloads.flow_pair(300, 200, seed=2)
+    check_against_oracle(p, p, [0.5])
+    q = p.copy()
+    q[80:112, 100:140] = np.roll(p, 9, axis=1)[80:112, 100:140]
+    check_against_oracle(p, q, [0.25])
+
+
+@pytest.mark.parametrize("W,H,fs", [(16, 16, 4), (17, 16, 2), (64, 64, 1), (200, 120, 2), (1032, 1024, 1), (4096, 3744, 1)])
+def test_scene_cut_mean(W, H, fs):
+    """numpy's pairwise mean of the SADs: 1 block, a few, one leaf, several, many leaves, more than fit shared memory"""
+    import framegen as fg
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(W)
+    f = torch.randint(0, 256, (2, H, W, 4), generator=g, dtype=torch.uint8, device="cuda")
+    it = fg.Interpolator()
+    assert it.init(W, H, fg.VK_R8G8B8A8_UNORM, settings=fg.Settings(flowScale=fs)), it.init_error()
+    it.begin_frame()
+    assert it.record_estimate(f[0], f[1])
+    tr = fg.read_trace(it)
+    assert tr["sads"].size == -(-round(W / fs) // 8) * -(-round(H / fs) // 8)   # (sizes round half to even)
+    assert np.float32(tr["sad"]) == tr["sads"].mean(dtype=np.float32)
+    assert tr["sadSum256"] == int(np.rint(tr["sads"].ravel() * np.float32(256)).astype(np.int64).sum()) & 0xFFFFFFFF
+    it.close()

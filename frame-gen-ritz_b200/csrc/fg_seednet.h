@@ -40,10 +40,21 @@ struct SnBackArgs {
     float* dw;         // += dL/dW, float [cout][9][cin]
     float* db;         // += dL/db, float [cout]
     int B, H, W, Ho, Wo;
-    float* part;       // the weight gradient's per-CTA partial sums (kSnPartFloats per CTA, up to partCtas CTAs)
+    float* part;       // the weight gradient's per-CTA partial sums (snPartFloats(l) per CTA, up to partCtas CTAs)
     int partCtas;
 };
-constexpr int kSnPartFloats = (9 * 32 + 1) * 32;   // rows (tap, ci) + the bias row, times cout, of the widest layer
+constexpr int snPartFloats(int l) { return (9 * kSnCin[l] + 1) * kSnCout[l]; }   // rows (tap, ci) + the bias row, times cout
+
+// the partial sums of every layer's weight gradient and where their sums go
+struct SnSumLayer {
+    const float* part;
+    float* dw; float* db;
+    int ctas, cin, cout;
+};
+struct SnSumArgs {
+    SnSumLayer layer[kSnLayers];
+    int first[kSnLayers];   // the layer's first block (filled in by the launcher)
+};
 
 struct SnAdamArgs {
     float* p; float* m; float* v; float* grad;   // float32 master parameters, moments, gradients (zeroed here)
@@ -75,10 +86,11 @@ cudaError_t launchSnConv(int layer, const SnConvArgs& a, cudaStream_t s);
 // message
 bool seedNetForwardLuma(::fg_seednet* n, cudaStream_t s, const float* la, const float* lc, int h, int w, float* out,
                         unsigned int* err, const char** why);
-// one layer's weight / bias gradient (and its input gradient when needDx) on the tensor cores (fg_seednet_bwd.cu);
-// kErrSeedNet into *err if a tensor-core wait gave up
+// one layer's partial weight / bias gradients and (but for the first layer) its input gradient on the tensor cores
+// (fg_seednet_bwd.cu); ctas: the partial sums written; kErrSeedNet into *err if a tensor-core wait gave up. Then the sums.
 cudaError_t prepareSeedNetBackward();
-cudaError_t launchSnBackwardTc(int layer, const SnBackArgs& a, bool needDx, unsigned int* err, cudaStream_t s);
+cudaError_t launchSnBackwardTc(int layer, const SnBackArgs& a, int& ctas, unsigned int* err, cudaStream_t s);
+cudaError_t launchSnDwSum(SnSumArgs& a, cudaStream_t s);
 cudaError_t launchSnLoss(const float* out, const float* tgt, int n, float* dout, float* loss, float scale, cudaStream_t s);
 cudaError_t launchSnAdam(const SnAdamArgs& a, cudaStream_t s);
 

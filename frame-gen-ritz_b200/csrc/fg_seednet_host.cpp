@@ -61,8 +61,8 @@ struct fg_seednet {
     float* loss = nullptr;
     void* act[kSnLayers - 1] = {};   // bf16 outputs of layers 1..5
     unsigned int* errFlags = nullptr;   // the fused forward's sticky error bits (kErrSeedNet) when no other is given
-    float* part = nullptr;              // the weight gradient's per-CTA partial sums
-    int partCtas = 0;
+    float* part[kSnLayers] = {};        // the weight gradients' per-CTA partial sums, by layer
+    int partCtas[kSnLayers] = {};
     float* out = nullptr;            // last layer (float)
     float* dA = nullptr;             // gradient ping-pong buffers (float)
     float* dB = nullptr;
@@ -133,6 +133,7 @@ struct fg_seednet {
         const int nb = B * d.h[kSnLayers] * d.w[kSnLayers];
         if (!forwardFused(s, B, H, W, out, nullptr, nullptr, nullptr, x, true)) return false;   // keeps layers 1-5
         if (!ok(cudaMemsetAsync(loss, 0, sizeof(float), s))) return false;
+        SnSumArgs sum{};
         float* dy = dA;
         if (!ok(launchSnLoss(out, targets, nb, dy, loss, 1.0f / (float)nb, s), "loss")) return false;
         for (int l = kSnLayers - 1; l >= 0; l--) {
@@ -144,11 +145,13 @@ struct fg_seednet {
             a.dw = grad + snWeightOff(l);
             a.db = grad + snBiasOff(l);
             a.B = B; a.H = d.h[l]; a.W = d.w[l]; a.Ho = d.h[l + 1]; a.Wo = d.w[l + 1];
-            a.part = part; a.partCtas = partCtas;
-            if (!ok(launchSnBackwardTc(l, a, l > 0, errFlags, s), "backward", l)) return false;
+            a.part = part[l]; a.partCtas = partCtas[l];
+            int ctas = 0;
+            if (!ok(launchSnBackwardTc(l, a, ctas, errFlags, s), "backward", l)) return false;
+            sum.layer[l] = SnSumLayer{part[l], a.dw, a.db, ctas, kSnCin[l], kSnCout[l]};
             dy = a.dx;
         }
-        return true;
+        return ok(launchSnDwSum(sum, s), "gradient sums");
     }
 };
 
@@ -191,8 +194,12 @@ fg_seednet* fg_seednet_create(int device, int max_batch, int max_h, int max_w) {
     const size_t oErr = take(4);
     int sms = 148;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device) != cudaSuccess) { cudaGetLastError(); sms = 148; }
-    n->partCtas = 2 * sms;
-    const size_t oPart = take((size_t)n->partCtas * kSnPartFloats * 4);
+    // partial sums: half the SMs beside a layer's input gradient, all of them for the first layer, which has none
+    size_t oPart[kSnLayers];
+    for (int l = 0; l < kSnLayers; l++) {
+        n->partCtas[l] = l ? std::max(sms / 2, 1) : sms;
+        oPart[l] = take((size_t)n->partCtas[l] * snPartFloats(l) * 4);
+    }
     const size_t oDA = take(maxGrad * 4), oDB = take(maxGrad * 4);
     if (cudaMalloc(&n->mem, off) != cudaSuccess) {
         cudaGetLastError();
@@ -206,7 +213,7 @@ fg_seednet* fg_seednet_create(int device, int max_batch, int max_h, int max_w) {
     for (int l = 0; l < kSnLayers - 1; l++) n->act[l] = n->mem + oAct[l];
     n->out = (float*)(n->mem + oOut);
     n->errFlags = (unsigned int*)(n->mem + oErr);
-    n->part = (float*)(n->mem + oPart);
+    for (int l = 0; l < kSnLayers; l++) n->part[l] = (float*)(n->mem + oPart[l]);
     if (prepareSeedNetFused() != cudaSuccess || prepareSeedNetBackward() != cudaSuccess) {   // shared-memory limits
         cudaGetLastError();
         cudaFree(n->mem);

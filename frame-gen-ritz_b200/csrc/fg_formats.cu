@@ -596,7 +596,7 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
     if (tid == 0) cnt = nSlow = 0;
     uint8_t* e;
     unsigned short* hsum;
-    const SyField f = syFieldStage(p, X0, Y0, tid, ex, rowc, sm, e, hsum);
+    const SyField f = syFieldStage<kUi>(p, X0, Y0, tid, ex, rowc, sm, e, hsum);
     const SyCoef& cx = f.cx;
     const float kA = p.mid ? 1.0f : p.ka, kC = p.mid ? 1.0f : p.kc;
     constexpr bool kYuv = F == kFmtNv12 || F == kFmtP010;
@@ -626,7 +626,7 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
         const int Xc = __float_as_int(bc.x) - 0x4B400000, Yc = __float_as_int(bc.y) - 0x4B400000;
         warp<F, kIn>(p, p.a, p.ac, Xa, Ya, wa);
         warp<F, kIn>(p, p.c, p.cc, Xc, Yc, wc);
-        if (kUi) {
+        if (kUi && !kIn) {
             const bool ha = p.uiA && (kYuv ? uiHitMaskYuv(p.uiA, Xa, Ya) : uiHitMask(p.uiA, Xa, Ya));
             const bool hc = p.uiC && (kYuv ? uiHitMaskYuv(p.uiC, Xc, Yc) : uiHitMask(p.uiC, Xc, Yc));
             if (ha != hc) {
@@ -661,7 +661,7 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
                 const float qcx = __fadd_rn(bx, __fmul_rn(kC, h.x)), qcy = __fadd_rn(by, __fmul_rn(kC, h.y));
                 float2 ca = warpChroma<F, kIn>(p.ac, p.cpitch, p.W, p.H, rne32(qax), rne32(qay));
                 float2 cc = warpChroma<F, kIn>(p.cc, p.cpitch, p.W, p.H, rne32(qcx), rne32(qcy));
-                if (kUi) {   // uiRejectC: the block-centre taps, with their own footprints
+                if (kUi && !kIn) {   // uiRejectC: the block-centre taps, with their own footprints
                     const bool ha = p.uiA && uiHitMaskYuv(p.uiA, rne32(qax), rne32(qay));
                     const bool hc = p.uiC && uiHitMaskYuv(p.uiC, rne32(qcx), rne32(qcy));
                     if (ha != hc) {
@@ -676,7 +676,7 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
             for (int c = 0; c < 3; c++) mix[(c * kSyTH + ly) * kSyE + ex] = mixF(wa[c], wc[c], p);
         }
     };
-    if (!kUi && f.in) syWalk<true, kRows>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) { stage2(SyTrue(), ey, posy, h); });
+    if (f.in && !f.ui) syWalk<true, kRows>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) { stage2(SyTrue(), ey, posy, h); });
     else syWalk<false, kRows>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) { stage2(SyFalse(), ey, posy, h); });
     __syncthreads();
     if (pq) {   // the undecided pixels (about 1.6 % on natural content), dealt out over all threads: warped again, exact

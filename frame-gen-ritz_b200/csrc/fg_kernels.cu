@@ -1251,7 +1251,7 @@ __device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int 
     }
     uint8_t* e;
     unsigned short* hsum;
-    const SyField f = syFieldStage(p, X0, Y0, tid, ex, rowc, sm, e, hsum);
+    const SyField f = syFieldStage<kUi>(p, X0, Y0, tid, ex, rowc, sm, e, hsum);
     // 2. this thread's region column and kSyK rows: half-vector, both warps, mismatch. The warps wait in shared memory
     //    for the blend (in registers they would leave too few for the sample loads in flight).
     uint32_t* sWA = reinterpret_cast<uint32_t*>(hsum + kSyEH * kSyHS);   // the output rows: kSyTH x kSyE
@@ -1270,7 +1270,7 @@ __device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int 
         }
         e[ey * kSyES + ex] = (uint8_t)m;
     };
-    if (!kUi && f.in) {
+    if (f.in && !f.ui) {
         syWalk<true, kLat ? kSyK : 2>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) {
             float2 ba, bc;
             positions(posy, h, ba, bc);

@@ -70,15 +70,17 @@ __device__ __noinline__ float fmtPq255(float v, float kWhite) {
 
 // Linear RgbaF16's mismatch needs only the integer part of the largest channel difference of two fmtPq255 levels, so the
 // synthesis reads the levels off a piecewise linear table and evaluates fmtPq255 itself only where the table cannot
-// tell that integer. Segment i covers the floats y = clamp(v kWhite, 0, 1) whose bits >> kPqShift are kPqBase + i (64
+// tell that integer. Segment i covers the floats y = clamp(v kWhite, 0, 1) whose bits >> kPqShift are kPqBase + i (32
 // segments per octave, 2^-40 .. 1; all smaller y share segment 0), as (slope, intercept): level ~= y slope + intercept,
-// the chord moved half its sag up. Over every float y in [0, 1] the table is within 0.00383 of fmtPq255 (enumerated;
+// the chord moved half its sag up. Over every float y in [0, 1] the table is within 0.00501 of fmtPq255 (enumerated;
 // fmtPq255's own rounding noise is 0.0035 of that), so a difference of two levels is within kPqTol of the exact one.
 // The series costs ~140 instructions a level, six levels a pixel; a segment ~8. A 3840x2160 pair at t = 1/3, 2/3: 1175
-// us with the series for every pixel, 863 us so (1.6 % of the pixels undecided). 32 segments per octave would leave 2 %.
-constexpr int kPqShift = 17, kPqOctaves = 40, kPqSegs = (kPqOctaves << (23 - kPqShift)) + 1;
+// us with the series for every pixel, 863 us so at first (2 % of the pixels undecided; 64 segments per octave leave 1.6 % but take
+// the shared memory of a third CTA per SM).
+constexpr int kPqShift = 18, kPqOctaves = 40, kPqSegs = (kPqOctaves << (23 - kPqShift)) + 1;
 constexpr uint32_t kPqBase = (uint32_t)(127 - kPqOctaves) << (23 - kPqShift);
-constexpr float kPqTol = 0.008f;
+constexpr float kPqTol = 0.0102f;
+constexpr int kPqSlow = 1024;   // the queue of undecided pixels (a quarter of a region); past it they are evaluated in place
 constexpr size_t kPqSegBytes = (size_t)kPqSegs * 8;
 static_assert(kPqSegs <= fgk::kPqSegMax, "the host allocates kPqSegMax segments");
 
@@ -557,10 +559,10 @@ __device__ __forceinline__ void copyNear(const SynthParams& p, int x, int y) {
 
 // CTAs per SM a format's synthesis is compiled for, and region rows per loop round (syWalk), measured at 3840x2160, t = 1/2:
 // three CTAs (40 registers, rolled) are ahead of two (64 registers) where their shared memory fits and the taps are few
-// (Rgb10 129 against 143 us, P010 190 against 207); RgbaF16's table and blend planes leave room for two (211 -> 195),
-// and Nv12's 16 loads a pixel gain more from the registers (156 -> 152).
-__host__ __device__ constexpr int fmtCtas(int F) { return F == kFmtF16 || F == kFmtNv12 ? 2 : 3; }
-__host__ __device__ constexpr int fmtRows(int F) { return F == kFmtF16 ? 4 : (F == kFmtNv12 ? 8 : 2); }
+// (Rgb10 124 against 130 us in a graph, P010 178 against 196, linear RgbaF16 159 against 175); Nv12's 16 loads a pixel gain
+// more from the registers (156 -> 152).
+__host__ __device__ constexpr int fmtCtas(int F) { return F == kFmtNv12 ? 2 : 3; }
+__host__ __device__ constexpr int fmtRows(int F) { return F == kFmtNv12 ? 8 : (F == kFmtP010 ? 4 : 2); }
 
 // compile-time flags of the synthesis tile's lambdas: the tile is inside the frame (SyField::in), or not known to be
 struct SyTrue { static constexpr bool value = true; };
@@ -604,13 +606,14 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
     // the blend inputs m of the output pixels, kept from stage 2 for stage 4 (the warps are computed once): per channel
     // planes of kSyTH x kSyE floats (YUV: the luma plane, then the block-centre chroma (Cb, Cr) of the even-even
     // pixels, (kSyTH / 2) x (kSyE / 2))
-    float* mix = reinterpret_cast<float*>(hsum + kSyEH * kSyHS);
-    float2* mixc = reinterpret_cast<float2*>(mix + kSyTH * kSyE);
-    // linear RgbaF16: the PQ segment table, and the region pixels it cannot decide (a queue over hsum, written later)
+    // linear RgbaF16: the PQ segment table in the place of hsum, which is written when the table is done with, and after
+    // it the queue of the region pixels that the table cannot decide
     const bool pq = F == kFmtF16 && p.f.linear;
-    float2* seg = reinterpret_cast<float2*>(mix + 3 * kSyTH * kSyE);
-    unsigned short* slow = hsum;
-    static_assert(kSyE * kSyEH <= kSyEH * kSyHS && kSyE * kSyEH <= 65536, "every region pixel fits the queue");
+    float2* seg = reinterpret_cast<float2*>(hsum);
+    unsigned short* slow = reinterpret_cast<unsigned short*>(seg + kPqSegs);
+    static_assert(kPqSegBytes >= (size_t)kSyEH * kSyHS * 2 && kSyE * kSyEH <= 65536, "hsum fits under the table");
+    float* mix = F == kFmtF16 ? reinterpret_cast<float*>(slow + kPqSlow) : reinterpret_cast<float*>(hsum + kSyEH * kSyHS);
+    float2* mixc = reinterpret_cast<float2*>(mix + kSyTH * kSyE);
     if (pq) {
         for (int i = tid; i < kPqSegs; i += kSyThreads) seg[i] = __ldg(p.pqSeg + i);
         __syncthreads();
@@ -645,7 +648,11 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
         warps(in, cx.pos, posy, h, wa, wc);
         if (pq) {
             int m;
-            if (!mismatchPq(p.f, seg, wa, wc, m)) slow[atomicAdd(&nSlow, 1u)] = (unsigned short)(ey * kSyE + ex);
+            if (!mismatchPq(p.f, seg, wa, wc, m)) {
+                const unsigned int n = atomicAdd(&nSlow, 1u);
+                if (n < (unsigned)kPqSlow) slow[n] = (unsigned short)(ey * kSyE + ex);
+                else m = mismatch<F>(p.f, wa, wc);
+            }
             e[ey * kSyES + ex] = (uint8_t)m;
         } else {
             e[ey * kSyES + ex] = (uint8_t)mismatch<F>(p.f, wa, wc);
@@ -679,8 +686,8 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
     if (f.in && !f.ui) syWalk<true, kRows>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) { stage2(SyTrue(), ey, posy, h); });
     else syWalk<false, kRows>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) { stage2(SyFalse(), ey, posy, h); });
     __syncthreads();
-    if (pq) {   // the undecided pixels (about 1.6 % on natural content), dealt out over all threads: warped again, exact
-        const int n = (int)nSlow;
+    if (pq) {   // the undecided pixels (about 2 % on natural content), dealt out over all threads: warped again, exact
+        const int n = min((int)nSlow, kPqSlow);
         for (int i = tid; i < n; i += kSyThreads) {
             const int sx = slow[i] & (kSyE - 1), sy = slow[i] / kSyE;
             const float4 r = rowc[sy];
@@ -1027,10 +1034,18 @@ static size_t fmtSynthSmem(int format, int fs) {
     const size_t mix = format == kFmtNv12 || format == kFmtP010
                            ? (size_t)kSyTH * kSyE * 4 + (size_t)((kSyTH + 1) / 2) * (kSyE / 2) * 8
                            : (size_t)3 * kSyTH * kSyE * 4;
-    return synthSmemBytes(fs) + mix + (format == kFmtF16 ? kPqSegBytes : 0);   // linear RgbaF16: the PQ segments
+    if (format != kFmtF16) return synthSmemBytes(fs) + mix;
+    return synthSmemBytes(fs) - (size_t)kSyEH * kSyHS * 2 + kPqSegBytes + kPqSlow * 2 + mix;   // the PQ segments over hsum
 }
 
 cudaError_t prepareFormatKernels() {
+    // The linear RgbaF16 luma pass lives on its table's hits in L1 (3 gathers a pixel): it asks for the shared memory of its
+    // 8 CTAs and no more. Left to the driver it ran on in the synthesis' configuration, which three CTAs leave almost no
+    // L1, and a 3840x2160 pair at t = 1/3, 2/3 took 617 us in a row of pairs instead of 539.
+    for (const void* k : {(const void*)k_luma_fmt<kFmtF16>, (const void*)k_luma_fmt_m<kFmtF16>}) {
+        const cudaError_t c = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 40);
+        if (c != cudaSuccess) return c;
+    }
     const int smem = (int)fmtSynthSmem(kFmtF16, 1);   // the largest
     cudaError_t e = cudaFuncSetAttribute(k_synth_fmt<kFmtRgb10>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt<kFmtF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

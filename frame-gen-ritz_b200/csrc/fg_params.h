@@ -269,7 +269,7 @@ cudaError_t launchLumaFmt(const LumaPyrParams& p, cudaStream_t s);
 // the PQ level of every half value (65536 floats) for a linear RgbaF16 luma at this white level
 cudaError_t launchPqTable(float* tab, float kWhite, cudaStream_t s);
 // linear RgbaF16's synthesis: the PQ levels as a piecewise linear table (at most kPqSegMax segments, any white level)
-constexpr int kPqSegMax = 2562;
+constexpr int kPqSegMax = 1282;
 cudaError_t launchPqSegments(float2* seg, cudaStream_t s);
 cudaError_t launchSynthFmt(const SynthParams& p, cudaStream_t s);
 // many syntheses of one of the other formats in one persistent launch (as launchSynthBatch), and their fallbacks

@@ -750,8 +750,9 @@ def main():
                 assert I.record_synth(pool[k][0], pool[k][1], o, t, stream=stream)
         graphs.append(g)
     n_levels = I.trace_layout().nLevels
-    # luma (+ deeper downsamples), search + median3 per level, subpixel, pixel field, synth + fallback per t
-    launches_per_step = 1 + max(0, n_levels - 6) + 2 * n_levels + 2 + 2 * len(TS)
+    # luma (+ deeper downsamples), search per level, median3 per level but 0 (in the sub-pixel pass), subpixel,
+    # pixel field, synth + fallback per t
+    launches_per_step = 1 + max(0, n_levels - 6) + 2 * n_levels - 1 + 2 + 2 * len(TS)
 
     with torch.cuda.stream(stream):
         for i in range(max(a.warmup, 3)):

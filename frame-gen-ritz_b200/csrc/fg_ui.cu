@@ -9,7 +9,9 @@
 //                   mask / leave and re-entry counters). The local contrast, max channel |I - median7x7(I)|, is found
 //                   only where it can matter (out of the mask and still or matching its stored colour): per channel a
 //                   binary search on the value for the smallest m with at least 25 of the 49 levels <= m, the window's
-//                   49 pixels packed one word each in registers.
+//                   49 pixels packed one word each in registers, from the CTA's 22 x 14 pixels staged in shared memory
+//                   (each converted once; read from the frame by every thread, its 49 loads waited on one another
+//                   behind the format's branches: a 128 x 128 box 34 us, staged 11 us, ncu).
 //   k_ui_v2_mask    one thread per mask word (4 pixels): in the mask or within 1 px of it -> 255 if still in this pair,
 //                   else 64; writes the rectangle into the header.
 //   k_ui_patch      one thread per work-rectangle pixel: out = the real curr pixel (colour channels) where the byte is
@@ -26,6 +28,8 @@ namespace fgk {
 namespace {
 
 constexpr int kUiTX = 16, kUiTY = 8;   // threads per CTA of the update and patch passes
+// the update's staged pixels: the CTA's own and 3 around them. Row pitch 48: a warp's two rows of 16 lie 16 banks apart.
+constexpr int kUiSX = kUiTX + 6, kUiSY = kUiTY + 6, kUiSP = 48;
 
 // an RgbaF16 half's 8-bit-equivalent level
 __device__ __forceinline__ uint32_t uiLevelF16(const UiV2Params& p, uint32_t bits) {
@@ -72,13 +76,13 @@ __device__ __forceinline__ int maxAbsDiff(uint32_t a, uint32_t b) {
 }
 
 // max channel |v - median7x7| at (x, y); YUV: of the R'G'B' difference the (Y, Cb, Cr) difference stands for
-// (format.glsl fgYuvDiff, in the order of the synthesis' mismatch)
-__device__ float contrastAt(const UiV2Params& p, int x, int y, uint32_t v) {
+// (format.glsl fgYuvDiff, in the order of the synthesis' mismatch). px: the window's first staged pixel.
+__device__ float contrastAt(const UiV2Params& p, const uint32_t* px, uint32_t v) {
     uint32_t w[49];
 #pragma unroll
     for (int j = 0; j < 7; j++)
 #pragma unroll
-        for (int i = 0; i < 7; i++) w[j * 7 + i] = uiPixel(p, x + i - 3, y + j - 3);
+        for (int i = 0; i < 7; i++) w[j * 7 + i] = px[j * kUiSP + i];
     int d = 0, dc[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
@@ -107,9 +111,18 @@ __device__ float contrastAt(const UiV2Params& p, int x, int y, uint32_t v) {
 
 __global__ void __launch_bounds__(kUiTX * kUiTY) k_ui_v2_update(const UiV2Params p) {
     pdlEnter();
+    __shared__ uint32_t sPx[kUiSY * kUiSP];
     const int x = blockIdx.x * kUiTX + threadIdx.x, y = blockIdx.y * kUiTY + threadIdx.y;
-    if (x >= p.ww || y >= p.wh) return;
     const int sx = p.wx + x, sy = p.wy + y;
+    if (!p.reset && p.cthr > 0.0f) {
+#pragma unroll
+        for (int k = 0; k < (kUiSX * kUiSY + kUiTX * kUiTY - 1) / (kUiTX * kUiTY); k++) {
+            const int i = k * kUiTX * kUiTY + threadIdx.y * kUiTX + threadIdx.x, r = i / kUiSX, c = i - r * kUiSX;
+            if (r < kUiSY) sPx[r * kUiSP + c] = uiPixel(p, sx - (int)threadIdx.x - 3 + c, sy - (int)threadIdx.y - 3 + r);
+        }
+        __syncthreads();
+    }
+    if (x >= p.ww || y >= p.wh) return;
     const uint32_t now = uiPixel(p, sx, sy);
     uint32_t* s = p.st + ((size_t)y * p.ww + x) * 4;
     const int ix = sx - p.bx, iy = sy - p.by;
@@ -132,7 +145,7 @@ __global__ void __launch_bounds__(kUiTX * kUiTY) k_ui_v2_update(const UiV2Params
         bool inMask = (flags & 1u) != 0u, hasStored = (flags & 2u) != 0u;
         const bool matchS = !inMask && hasStored && p.reentry > 0 && (float)maxAbsDiff(now, stored) <= p.thr;
         bool contrasty = p.cthr <= 0.0f;
-        if (!inMask && !contrasty && (still || matchS)) contrasty = contrastAt(p, sx, sy, now) >= p.cthr;
+        if (!inMask && !contrasty && (still || matchS)) contrasty = contrastAt(p, sPx + threadIdx.y * kUiSP + threadIdx.x, now) >= p.cthr;
         if (inMask) {
             leave = still ? 0u : min(leave + 1u, 255u);
             if (still) stored = now;

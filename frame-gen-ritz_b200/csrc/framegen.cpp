@@ -225,7 +225,6 @@ struct Interpolator::Impl {
     float* luma = nullptr;
     float2* pqSeg = nullptr;  // linear RgbaF16: the PQ segment table of the synthesis
     float* pqTab = nullptr;   // linear RgbaF16: the PQ level of every half value (the luma pass looks them up)
-    bool lumaF0 = true;         // the latest estimate wrote level 0 as float too
     uint32_t* pair = nullptr;   // level 0's pair planes (prev, then curr; fg_params.h LumaPyrParams), or null
     float2* field = nullptr;
     float* sads = nullptr;
@@ -711,7 +710,6 @@ struct Interpolator::Impl {
         const bool fill = fillMask[0] && fillMask[1];
         EstPlan e;
         planEstimate(prev, curr, fill, e);
-        lumaF0 = e.luma.la[0] != nullptr;
         const fgk::LumaPyrParams& lp = e.luma;
         if (!check(fmt == Format::Rgba8 ? fgk::launchLumaPyr(lp, s) : fgk::launchLumaFmt(lp, s))) return false;
         stamp(s, "luma");
@@ -1380,8 +1378,9 @@ bool Interpolator::recordTrace(cudaStream_t stream, void* dst) {
     DeviceGuard g(m->device);
     char* d = (char*)dst;
     const auto D2D = cudaMemcpyDeviceToDevice;
-    // an estimate that kept level 0 as pair planes only left its float form to this call
-    if (!m->lumaF0 && fgk::launchUnpair(m->pair, m->luma + m->L.lv[0].lumaA, (size_t)2 * l.fw * l.fh, stream) != cudaSuccess) return false;
+    // level 0 from its pair planes where there are any: every estimate writes them, the float form only where a pass reads it,
+    // and which one ran last (a replayed graph, a batch) is not known here
+    if (m->pair && fgk::launchUnpair(m->pair, m->luma + m->L.lv[0].lumaA, (size_t)2 * l.fw * l.fh, stream) != cudaSuccess) return false;
     bool ok = cudaMemcpyAsync(d + l.lumaOff, m->luma, l.lumaBytes, D2D, stream) == cudaSuccess &&
               cudaMemcpyAsync(d + l.fieldOff, m->field, l.fieldBytes, D2D, stream) == cudaSuccess &&
               cudaMemcpyAsync(d + l.medOff, m->st->med, (size_t)l.nLevels * 8, D2D, stream) == cudaSuccess &&
@@ -1563,7 +1562,6 @@ bool Batch::Impl::mergedEstimates(cudaStream_t s, const Frame* prev, const Frame
         im.estSets++;
         im.haveEst = im.estUi = false;
         im.planEstimate(prev[i], curr[i], false, plans[j]);
-        im.lumaF0 = plans[j].luma.la[0] != nullptr;
         maxTop = std::max(maxTop, plans[j].top);
     }
     auto fail = [&](cudaError_t e) {

@@ -569,18 +569,21 @@ __device__ __forceinline__ void cutMeanQCta(const PixfieldParams& p, int cta, ui
         if (lane == 0) {
             pl.gvals[leaf] = v;
             pl.leafS256[leaf] = s256;
-            __threadfence();
         }
     }
+    // the ticket: the thread that takes it fences on both sides, between two barriers, so that it releases the leaves of all
+    // 8 warps (a fence by the warps that wrote them would not: release goes by the order within the ticket's thread) and
+    // acquires the other CTAs' for this one
     __syncthreads();
     if (tid == 0) {
         const unsigned int n = (unsigned int)min(8, pl.nLeaves - cta * 8);
+        __threadfence();
         last = atomicAdd(&p.st->subDone, n) + n == (unsigned int)pl.nLeaves;
+        __threadfence();
         tot = 0;
     }
     __syncthreads();
     if (!last) return;
-    __threadfence();
     // node values and the inner nodes' operands in shared memory where they fit (else the values stay in gvals)
     const bool fits = (size_t)pl.nLeaves * 16 <= smBytes;
     float* vals = fits ? reinterpret_cast<float*>(sm) : pl.gvals;

@@ -453,12 +453,14 @@ __device__ __forceinline__ void median3Cta(const Median3Params& p, int cta, int 
     __shared__ unsigned int ticket;
     __shared__ unsigned int part[256];
     __shared__ int found[4];
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) ticket = atomicAdd(p.done, 1u);
+    if (threadIdx.x == 0) {   // fenced on both sides: releases the whole CTA's adds, acquires the other CTAs'
+        __threadfence();
+        ticket = atomicAdd(p.done, 1u);
+        __threadfence();
+    }
     __syncthreads();
     if (ticket != (unsigned int)ctas - 1u) return;
-    __threadfence();
     if (threadIdx.x < 4) found[threadIdx.x] = 0;
     const int nb = 2 * p.B + 1;
     const unsigned int N = (unsigned int)(p.fbw * p.fbh), ks[2] = {(N - 1) / 2, N / 2};

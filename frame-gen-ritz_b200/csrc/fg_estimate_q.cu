@@ -733,7 +733,21 @@ __global__ void __launch_bounds__(256) k_unpair(const uint32_t* pair, float* out
 cudaError_t launchUnpair(const uint32_t* pair, float* out, size_t n, cudaStream_t s) {
     return launchPdl(k_unpair, dim3((unsigned int)((n + 255) / 256)), dim3(256), 0, s, pair, out, n);
 }
+// one item as a merged launch: its grid is one-dimensional. The per-pair launches have a block row per grid row, and a grid
+// ends at 65535 rows (a frame of 1048560 rows at flowScale 2; the passes before and after go to 3.6 M).
+constexpr int kGridRows = 65535;
+template <class P>
+static Merged<P> alone(const P& p) {
+    Merged<P> m{};
+    m.n = 1;
+    m.item[0] = p;
+    return m;
+}
 cudaError_t launchSearchQ(const SearchParams& p, cudaStream_t s) {
+    if (p.bh > kGridRows) {
+        Merged<SearchParams> m = alone(p);
+        return launchSearchQMerged(m, s);
+    }
     const dim3 grid(divUp(p.bw, 4), p.bh);
     if (p.R == 1) return launchPdl(p.pa ? k_search_q<1, true> : k_search_q<1, false>, grid, dim3(128), 0, s, p);
     return launchPdl(p.pa ? k_search_q<2, true> : k_search_q<2, false>, grid, dim3(128), 0, s, p);
@@ -748,6 +762,10 @@ cudaError_t launchSearchQMerged(Merged<SearchParams>& m, cudaStream_t s) {
     return launchPdl(pair ? k_search_q_m<2, true> : k_search_q_m<2, false>, dim3(total), dim3(128), 0, s, m);
 }
 cudaError_t launchSubpixQ(const SubpixParams& p, cudaStream_t s) {
+    if (p.bh > kGridRows) {
+        Merged<SubpixParams> m = alone(p);
+        return launchSubpixQMerged(m, s);
+    }
     return launchPdl(k_subpix_q, dim3(divUp(p.bw, 4), p.bh), dim3(128), 0, s, p);
 }
 cudaError_t launchSubpixQMerged(Merged<SubpixParams>& m, cudaStream_t s) {

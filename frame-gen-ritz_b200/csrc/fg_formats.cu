@@ -123,19 +123,11 @@ __device__ __forceinline__ uint32_t ldh(const uint8_t* base, size_t pitch, int x
     return __ldg(reinterpret_cast<const unsigned short*>(base + (size_t)y * pitch) + x);
 }
 
-// a raw channel of an Rgb10 word (k: 0 R, 1 G, 2 B)
-__device__ __forceinline__ int rgb10(const FmtConst& f, uint32_t w, int k) {
-    return (int)((w >> (f.rHigh ? 20 - 10 * k : 10 * k)) & 1023u);
-}
-
-// the three raw channels of texel (x, y): Rgb10 codes, F16 values; YUV: the Y level only (r[0])
+// texel (x, y): the three F16 values; YUV: the Y level only (r[0])
 template <int F>
-__device__ __forceinline__ void texel(const FmtConst& f, const uint8_t* base, size_t pitch, int x, int y, float r[3]) {
-    if (F == kFmtRgb10) {
-        const uint32_t w = ldw(base, pitch, x, y);
-#pragma unroll
-        for (int k = 0; k < 3; k++) r[k] = i2f(rgb10(f, w, k));
-    } else if (F == kFmtF16) {
+__device__ __forceinline__ void texel(const uint8_t* base, size_t pitch, int x, int y, float r[3]) {
+    static_assert(F != kFmtRgb10, "Rgb10 words are taken apart where they are read");
+    if (F == kFmtF16) {
         const uint2 q = __ldg(reinterpret_cast<const uint2*>(base + (size_t)y * pitch) + x);
         r[0] = h2f(q.x & 0xFFFFu);
         r[1] = h2f(q.x >> 16);
@@ -158,12 +150,9 @@ __device__ __forceinline__ float2 ctexel(const uint8_t* cbase, size_t cpitch, in
     return make_float2(__fmul_rn(i2f((int)(v & 0xFFFFu)), 0x1p-8f), __fmul_rn(i2f((int)(v >> 16)), 0x1p-8f));
 }
 
-// a raw channel -> its level (RGB formats)
-template <int F>
-__device__ __forceinline__ float levelOf(const FmtConst& f, float r) {
-    if (F == kFmtRgb10) return __fmul_rn(r, f.k10);
-    if (F == kFmtF16) return f.linear ? fmtPq255(r, f.kWhite) : __fmul_rn(r, 255.0f);
-    return r;
+// an F16 value -> its level
+__device__ __forceinline__ float levelF16(const FmtConst& f, float r) {
+    return f.linear ? fmtPq255(r, f.kWhite) : __fmul_rn(r, 255.0f);
 }
 
 // ============================================================================================== luma
@@ -188,21 +177,23 @@ __device__ __forceinline__ int quartersRgb10(const FmtConst& f, uint32_t w) {
 }
 __device__ __forceinline__ int quartersF16(const FmtConst& f, const float* pq, uint32_t rg, uint32_t b) {
     if (pq) return quartersRgb(__ldg(pq + (rg & 0xFFFFu)), __ldg(pq + (rg >> 16)), __ldg(pq + (b & 0xFFFFu)));
-    return quartersRgb(levelOf<kFmtF16>(f, h2f(rg & 0xFFFFu)), levelOf<kFmtF16>(f, h2f(rg >> 16)), levelOf<kFmtF16>(f, h2f(b & 0xFFFFu)));
+    return quartersRgb(levelF16(f, h2f(rg & 0xFFFFu)), levelF16(f, h2f(rg >> 16)), levelF16(f, h2f(b & 0xFFFFu)));
 }
 
 // the motion estimate's luma of pixel (x, y) in quarter levels
 template <int F>
 __device__ __forceinline__ int lumaQ(const FmtConst& f, const uint8_t* base, size_t pitch, int x, int y, const float* pq) {
     const uint8_t* row = base + (size_t)y * pitch;
-    if (F == kFmtRgb10) return quartersRgb10(f, __ldg(reinterpret_cast<const uint32_t*>(row) + x));
-    if (F == kFmtF16) {
+    if constexpr (F == kFmtRgb10) {
+        return quartersRgb10(f, __ldg(reinterpret_cast<const uint32_t*>(row) + x));
+    } else if constexpr (F == kFmtF16) {
         const uint2 q = __ldg(reinterpret_cast<const uint2*>(row) + x);
         return quartersF16(f, pq, q.x, q.y);
+    } else {
+        float r[3];
+        texel<F>(base, pitch, x, y, r);
+        return quartersY(f, r[0]);
     }
-    float r[3];
-    texel<F>(f, base, pitch, x, y, r);
-    return quartersY(f, r[0]);
 }
 
 // ... of the 4 pixels from x on of an aligned row, added up in pairs
@@ -387,23 +378,19 @@ __device__ __forceinline__ ITaps mkITaps(int X, int Y, int w, int h) {
     return t;
 }
 
-// the float taps of warpChroma (formats other than Nv12, and P010 samples off the 10-bit grid)
-template <int F>
-__device__ __forceinline__ float2 warpChromaF(const uint8_t* cbase, size_t cpitch, int W, int H, int X, int Y) {
-    const Taps t = mkTaps<6>(X - 16, Y - 16, (W + 1) >> 1, (H + 1) >> 1);
-    const float2 c00 = ctexel<F>(cbase, cpitch, t.x0, t.y0), c01 = ctexel<F>(cbase, cpitch, t.x1, t.y0);
-    const float2 c10 = ctexel<F>(cbase, cpitch, t.x0, t.y1), c11 = ctexel<F>(cbase, cpitch, t.x1, t.y1);
-    return make_float2(bil(t, c00.x, c01.x, c10.x, c11.x), bil(t, c00.y, c01.y, c10.y, c11.y));
-}
-// out of line: the rare off-grid P010 case keeps its registers out of the synthesis kernels' hot path
+// the float taps of P010 chroma samples off the 10-bit grid. Out of line: the rare case keeps its registers out of the
+// synthesis kernels' hot path.
 __device__ __noinline__ float2 warpChromaP010Off(const uint8_t* cbase, size_t cpitch, int W, int H, int X, int Y) {
-    return warpChromaF<kFmtP010>(cbase, cpitch, W, H, X, Y);
+    const Taps t = mkTaps<6>(X - 16, Y - 16, (W + 1) >> 1, (H + 1) >> 1);
+    const float2 c00 = ctexel<kFmtP010>(cbase, cpitch, t.x0, t.y0), c01 = ctexel<kFmtP010>(cbase, cpitch, t.x1, t.y0);
+    const float2 c10 = ctexel<kFmtP010>(cbase, cpitch, t.x0, t.y1), c11 = ctexel<kFmtP010>(cbase, cpitch, t.x1, t.y1);
+    return make_float2(bil(t, c00.x, c01.x, c10.x, c11.x), bil(t, c00.y, c01.y, c10.y, c11.y));
 }
 
 // the chroma (Cb, Cr) levels warped to the point whose 1/32-px coordinates are (X, Y)
 template <int F, bool kIn>
 __device__ __forceinline__ float2 warpChroma(const uint8_t* cbase, size_t cpitch, int W, int H, int X, int Y) {
-    if (F == kFmtNv12) {   // byte pairs (Cb, Cr): gathered as (Cb00, Cb01, Cr00, Cr01), two dp2a per channel, exact
+    if constexpr (F == kFmtNv12) {   // byte pairs (Cb, Cr): gathered as (Cb00, Cb01, Cr00, Cr01), two dp2a per channel, exact
         const ITaps t = mkITaps<6, kIn>(X - 16, Y - 16, (W + 1) >> 1, (H + 1) >> 1);
         const unsigned short* q0 = reinterpret_cast<const unsigned short*>(cbase + (size_t)t.y * cpitch) + t.x;
         const unsigned short* q1 = reinterpret_cast<const unsigned short*>(cbase + (size_t)(t.y + 1) * cpitch) + t.x;
@@ -411,8 +398,7 @@ __device__ __forceinline__ float2 warpChroma(const uint8_t* cbase, size_t cpitch
         const uint32_t c1 = __byte_perm((uint32_t)__ldg(q1), (uint32_t)__ldg(q1 + 1), 0x5140);
         const uint32_t cb = __dp2a_lo(t.w1, c1, __dp2a_lo(t.w0, c0, 0u)), cr = __dp2a_hi(t.w1, c1, __dp2a_hi(t.w0, c0, 0u));
         return make_float2(__fmul_rn((float)cb, 0x1p-12f), __fmul_rn((float)cr, 0x1p-12f));
-    }
-    if (F == kFmtP010) {   // 10-bit codes in the high bits of 16-bit samples: integer taps when the low 6 bits are zero
+    } else {   // P010: 10-bit codes in the high bits of 16-bit samples: integer taps when the low 6 bits are zero
         const ITaps t = mkITaps<6, kIn>(X - 16, Y - 16, (W + 1) >> 1, (H + 1) >> 1);
         const uint32_t* q0 = reinterpret_cast<const uint32_t*>(cbase + (size_t)t.y * cpitch) + t.x;
         const uint32_t* q1 = reinterpret_cast<const uint32_t*>(cbase + (size_t)(t.y + 1) * cpitch) + t.x;
@@ -425,7 +411,6 @@ __device__ __forceinline__ float2 warpChroma(const uint8_t* cbase, size_t cpitch
         }
         return warpChromaP010Off(cbase, cpitch, W, H, X, Y);
     }
-    return warpChromaF<F>(cbase, cpitch, W, H, X, Y);
 }
 
 // the float taps of a P010 luma sample off the 10-bit grid (out of line, as warpChromaP010Off)
@@ -439,7 +424,7 @@ __device__ __noinline__ float warpYP010Off(const uint8_t* base, size_t pitch, in
 // levels
 template <int F, bool kIn>
 __device__ __forceinline__ void warp(const SynthParams& p, const uint8_t* base, const uint8_t* cbase, int X, int Y, float out[3]) {
-    if (F == kFmtRgb10) {   // 10-bit codes: integer taps, exact (ITaps)
+    if constexpr (F == kFmtRgb10) {   // 10-bit codes: integer taps, exact (ITaps)
         const ITaps t = mkITaps<5, kIn>(X, Y, p.W, p.H);
         const uint32_t* q0 = reinterpret_cast<const uint32_t*>(base + (size_t)t.y * p.pitch) + t.x;
         const uint32_t* q1 = reinterpret_cast<const uint32_t*>(base + (size_t)(t.y + 1) * p.pitch) + t.x;
@@ -453,7 +438,7 @@ __device__ __forceinline__ void warp(const SynthParams& p, const uint8_t* base, 
         out[0] = __fmul_rn(__fmul_rn((float)s0, 0x1p-10f), p.f.k10);
         out[1] = __fmul_rn(__fmul_rn((float)s1, 0x1p-20f), p.f.k10);
         out[2] = __fmul_rn(__fmul_rn((float)s2, 0x1p-10f), p.f.k10);
-    } else if (F == kFmtNv12) {    // 8-bit luma: integer taps, two dp2a (as the 8-bit RGBA sampler), exact
+    } else if constexpr (F == kFmtNv12) {   // 8-bit luma: integer taps, two dp2a (as the 8-bit RGBA sampler), exact
         const ITaps t = mkITaps<5, kIn>(X, Y, p.W, p.H);
         const uint8_t* q0 = base + (size_t)t.y * p.pitch + t.x;
         const uint8_t* q1 = q0 + p.pitch;
@@ -463,7 +448,7 @@ __device__ __forceinline__ void warp(const SynthParams& p, const uint8_t* base, 
         const float2 c = warpChroma<F, kIn>(cbase, p.cpitch, p.W, p.H, X, Y);
         out[1] = c.x;
         out[2] = c.y;
-    } else if (F == kFmtP010) {    // integer taps when the four samples' low 6 bits are zero (then every float step is exact)
+    } else if constexpr (F == kFmtP010) {   // integer taps when the four samples' low 6 bits are zero (then every float step is exact)
         const ITaps t = mkITaps<5, kIn>(X, Y, p.W, p.H);
         const unsigned short* q0 = reinterpret_cast<const unsigned short*>(base + (size_t)t.y * p.pitch) + t.x;
         const unsigned short* q1 = reinterpret_cast<const unsigned short*>(base + (size_t)(t.y + 1) * p.pitch) + t.x;
@@ -480,10 +465,10 @@ __device__ __forceinline__ void warp(const SynthParams& p, const uint8_t* base, 
     } else {
         const Taps t = mkTaps<5, kIn>(X, Y, p.W, p.H);
         float r00[3], r01[3], r10[3], r11[3];
-        texel<F>(p.f, base, p.pitch, t.x0, t.y0, r00);
-        texel<F>(p.f, base, p.pitch, t.x1, t.y0, r01);
-        texel<F>(p.f, base, p.pitch, t.x0, t.y1, r10);
-        texel<F>(p.f, base, p.pitch, t.x1, t.y1, r11);
+        texel<F>(base, p.pitch, t.x0, t.y0, r00);
+        texel<F>(base, p.pitch, t.x1, t.y0, r01);
+        texel<F>(base, p.pitch, t.x0, t.y1, r10);
+        texel<F>(base, p.pitch, t.x1, t.y1, r11);
 #pragma unroll
         for (int k = 0; k < 3; k++) out[k] = bil(t, r00[k], r01[k], r10[k], r11[k]);
     }
@@ -727,7 +712,7 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
                 iu = __fsub_rn(1.0f, u);
             }
             myCnt += u > 0.5f;
-            if (F == kFmtRgb10) {
+            if constexpr (F == kFmtRgb10) {
                 const uint32_t nw = ldw(nearF, p.pitch, x, y);
                 uint32_t ow = nw & 0xC0000000u;
 #pragma unroll
@@ -738,7 +723,7 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
                     ow |= (uint32_t)code << (10 * c);
                 }
                 sink.word(k, x, y, ow);
-            } else if (F == kFmtF16) {
+            } else if constexpr (F == kFmtF16) {
                 const uint2 nq = __ldg(reinterpret_cast<const uint2*>(nearF + (size_t)y * p.pitch) + x);
                 const float n0 = h2f(nq.x & 0xFFFFu), n1 = h2f(nq.x >> 16), n2 = h2f(nq.y & 0xFFFFu);
                 const uint32_t o0 = __half_as_ushort(__float2half_rn(blendM(mix[(0 * kSyTH + ly) * kSyE + ex], n0, u, iu)));
@@ -749,7 +734,7 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
                 constexpr float ql = F == kFmtP010 ? 4.0f : 1.0f;   // 1 / YU_QL
                 constexpr int codes = F == kFmtP010 ? 1023 : 255;
                 float ny[3];
-                texel<F>(p.f, nearF, p.pitch, x, y, ny);
+                texel<F>(nearF, p.pitch, x, y, ny);
                 const float v = blendM(mix[ly * kSyE + ex], ny[0], u, iu);
                 sink.luma(k, x, y, clampi((int)floorf(__fadd_rn(__fmul_rn(v, ql), 0.5f)), 0, codes));
                 if (((x | y) & 1) == 0) {   // the chroma of this 2x2 block (warped in stage 2)

@@ -90,23 +90,35 @@ __device__ __forceinline__ int gray8dp(uint32_t px, uint32_t wlo, uint32_t whi) 
 __device__ __forceinline__ float2 pmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 
-// round-half-even(x * 32) for |x * 32| < 2^22 (cv2's saturate_cast<int>(x * INTER_TAB_SIZE)), as the float's bits
-// CrosshairV2's warp-tap rejection (gpu/shaders/ui_reject.glsl): does the bilinear tap whose position rounded to
-// 1/32 px is (X, Y) (in 1/32 px) read, with a non-zero weight, a pixel that the UI mask m (header + bytes, fg_params.h
-// UiV2Params) marks? The tap reads lo = (X >> 5, Y >> 5) .. lo + (the fraction is not 0) per axis.
+// CrosshairV2's warp-tap rejection: does the UI mask m (header + bytes, fg_params.h UiV2Params) mark a pixel of the
+// rectangle (ax0, ay0) .. (ax1, ay1) of at most kN x kN frame pixels? At most 4 pixels lie in two words of a row, and all rows'
+// words are loaded before any is looked at: a thread's rows are neighbours, and with a byte at a time, each behind the
+// one before, a tile on the overlay waited for up to 8 x 16 loads in a row (a protected synthesis with its fallback
+// check and paste: P010 1366x768 69 -> 48 us, 8-bit RGBA 1280x720 28.9 -> 23.1, with one vote for three below).
+template <int kN>
+__device__ __forceinline__ bool uiHitSpan(const uint32_t* __restrict__ m, int ax0, int ay0, int ax1, int ay1) {
+    static_assert(kN <= 4, "two words a row");
+    const uint4 hd = __ldg(reinterpret_cast<const uint4*>(m));   // kUiMaskHeader words: -, origin, size, row stride
+    const int ox = (int)(hd.y & 0xFFFFu), oy = (int)(hd.y >> 16), w = (int)(hd.z & 0xFFFFu), h = (int)(hd.z >> 16);
+    const int x0 = max(ax0 - ox, 0), y0 = max(ay0 - oy, 0), x1 = min(ax1 - ox, w - 1), y1 = min(ay1 - oy, h - 1);
+    if (x0 > x1 || y0 > y1) return false;
+    const uint32_t* q = m + kUiMaskHeader + y0 * (int)hd.w + (x0 >> 2);
+    const bool two = (x1 >> 2) != (x0 >> 2);
+    const uint32_t lo = 0xFFFFFFFFu << (8 * (x0 & 3)), hi = 0xFFFFFFFFu >> (24 - 8 * (x1 & 3));
+    uint32_t v0 = 0u, v1 = 0u;
+#pragma unroll
+    for (int j = 0; j < kN; j++) {
+        const bool ok = y0 + j <= y1;
+        v0 |= ok ? __ldg(q + j * (int)hd.w) : 0u;
+        v1 |= ok && two ? __ldg(q + j * (int)hd.w + 1) : 0u;
+    }
+    return ((v0 & (two ? lo : lo & hi)) | (v1 & hi)) != 0u;
+}
+// the pixels that the bilinear tap whose position rounded to 1/32 px is (X, Y) (in 1/32 px) reads with a non-zero weight
+// (gpu/shaders/ui_reject.glsl): lo = (X >> 5, Y >> 5) .. lo + (the fraction is not 0) per axis
 __device__ __forceinline__ bool uiHitMask(const uint32_t* __restrict__ m, int X, int Y) {
-    const uint32_t wh = __ldg(m + 2);
-    if (wh == 0u) return false;
-    const uint32_t o = __ldg(m + 1);
-    const int ox = (int)(o & 0xFFFFu), oy = (int)(o >> 16), w = (int)(wh & 0xFFFFu), h = (int)(wh >> 16);
-    const int stride = (int)__ldg(m + 3);
     const int lx = X >> 5, ly = Y >> 5;
-    const int x0 = max(lx - ox, 0), y0 = max(ly - oy, 0);
-    const int x1 = min(lx + ((X & 31) != 0) - ox, w - 1), y1 = min(ly + ((Y & 31) != 0) - oy, h - 1);
-    for (int y = y0; y <= y1; y++)
-        for (int x = x0; x <= x1; x++)
-            if ((__ldg(m + 4 + y * stride + (x >> 2)) >> (8 * (x & 3))) & 255u) return true;
-    return false;
+    return uiHitSpan<2>(m, lx, ly, lx + ((X & 31) != 0), ly + ((Y & 31) != 0));
 }
 
 // CrosshairV2's estimate fill of one level-0 cell by a warp (gpu/shaders/ui_v2_lumafill.comp): if the fs x fs pixels from
@@ -148,20 +160,11 @@ __device__ __forceinline__ bool uiFillWindow(const uint32_t* __restrict__ m, int
 // chroma plane around it, c = X - 16 in 1/64 chroma texels, i = c >> 6, the second texel only if the fraction is not
 // 0: the pixels 2 i .. 2 (i + n) + 1 per axis, which contain the luma taps too
 __device__ __forceinline__ bool uiHitMaskYuv(const uint32_t* __restrict__ m, int X, int Y) {
-    const uint32_t wh = __ldg(m + 2);
-    if (wh == 0u) return false;
-    const uint32_t o = __ldg(m + 1);
-    const int ox = (int)(o & 0xFFFFu), oy = (int)(o >> 16), w = (int)(wh & 0xFFFFu), h = (int)(wh >> 16);
-    const int stride = (int)__ldg(m + 3);
     const int cx = X - 16, cy = Y - 16, ix = cx >> 6, iy = cy >> 6;
-    const int x0 = max(2 * ix - ox, 0), y0 = max(2 * iy - oy, 0);
-    const int x1 = min(2 * (ix + ((cx & 63) != 0)) + 1 - ox, w - 1), y1 = min(2 * (iy + ((cy & 63) != 0)) + 1 - oy, h - 1);
-    for (int y = y0; y <= y1; y++)
-        for (int x = x0; x <= x1; x++)
-            if ((__ldg(m + 4 + y * stride + (x >> 2)) >> (8 * (x & 3))) & 255u) return true;
-    return false;
+    return uiHitSpan<4>(m, 2 * ix, 2 * iy, 2 * (ix + ((cx & 63) != 0)) + 1, 2 * (iy + ((cy & 63) != 0)) + 1);
 }
 
+// round-half-even(x * 32) for |x * 32| < 2^22 (cv2's saturate_cast<int>(x * INTER_TAB_SIZE)), as the float's bits
 __device__ __forceinline__ float2 rne32bits(float2 v) {
     return __ffma2_rn(v, make_float2(32.0f, 32.0f), make_float2(12582912.0f, 12582912.0f));
 }
@@ -307,7 +310,9 @@ constexpr int kSyES = kSyE + 4, kSyHS = kSyE + 2;
 
 // cv2.remap INTER_LINEAR / BORDER_REPLICATE of the 2-channel float field at (x, y): quantisation and weights paired
 // (exact), the taps' weighted sum as cv2 rounds it, ((p00 w00 + p01 w01) + p10 w10) + p11 w11 per channel (paired
-// products, scalar sums: never fused). One address where the four taps lie inside the field.
+// products, scalar sums: never fused). One address where the four taps lie inside the field; kLat: clamped, without the
+// branch (a latency form has the instructions to spare).
+template <bool kLat>
 __device__ __forceinline__ float2 remapF2m(const float2* __restrict__ F, int w, int h, float x, float y) {
     const float2 bits = rne32bits(make_float2(x, y));
     const int X = __float_as_int(bits.x) - 0x4B400000, Y = __float_as_int(bits.y) - 0x4B400000;
@@ -317,7 +322,7 @@ __device__ __forceinline__ float2 remapF2m(const float2* __restrict__ F, int w, 
     const float2 wA = pmul(make_float2(g.y, g.y), make_float2(g.x, f.x));   // (w00, w01)
     const float2 wB = pmul(make_float2(f.y, f.y), make_float2(g.x, f.x));   // (w10, w11)
     float2 p00, p01, p10, p11;
-    if ((unsigned)ix < (unsigned)(w - 1) && (unsigned)iy < (unsigned)(h - 1)) {
+    if (!kLat && (unsigned)ix < (unsigned)(w - 1) && (unsigned)iy < (unsigned)(h - 1)) {
         const float2* q = F + (iy * w + ix);
         p00 = __ldg(q);
         p01 = __ldg(q + 1);
@@ -391,7 +396,10 @@ struct SyField {
 __device__ __forceinline__ int uiGap(int o, int side, int lo, int n) {
     return max(o - kSyAp - 4 - (lo + n - 1), lo - 4 - (o - kSyAp + side - 1));
 }
-template <bool kUi>
+// kSplit: a loop for the lookup at t and one for the plain field, the vectors' largest parts voted on after it. The 8-bit
+// kernels, the latency forms and the protected ones gain by it (3840x2160: 81 -> 80 us, 1280x720 17.9 -> 16.9); the formats'
+// 40-register kernels lose 1 to 2 % at 3840x2160 and keep one loop.
+template <bool kUi, bool kLat, bool kSplit>
 __device__ __forceinline__ SyField syFieldStage(const SynthParams& p, int X0, int Y0, int tid, int ex, float4* rowc,
                                                 unsigned char* sm, uint8_t*& e, unsigned short*& hsum) {
     const int fs = p.fs, uw = p.fw * fs, uh = p.fh * fs, sh = fs == 1 ? 1 : (fs == 2 ? 2 : 3);
@@ -417,7 +425,6 @@ __device__ __forceinline__ SyField syFieldStage(const SynthParams& p, int X0, in
     const bool wide = fs != 2 || (uint64_t)p.H * (p.pitch >> 2) >= 0xF0000000u;
     const float mx = wide ? -1.0f : (float)(min(X0 - kSyAp, Wt - (X0 - kSyAp + kSyE)) - 3);
     const float my = wide ? -1.0f : (float)(min(Y0 - kSyAp, Ht - (Y0 - kSyAp + kSyEH)) - 3);
-    bool out = false, nearX = false, nearY = false;
     float gapX = FLT_MAX, gapY = FLT_MAX;   // the moves along each axis below which no tap touches a mask's rectangle
     if (kUi) {
 #pragma unroll
@@ -432,28 +439,52 @@ __device__ __forceinline__ SyField syFieldStage(const SynthParams& p, int X0, in
     // the region's GW x GH samples spread over all threads (GW is about half the CTA's width at flowScale 2): row
     // r = floor((i + 0.5) / GW), exact in float for these sizes (the quotient stays >= 0.5 / GW from an integer)
     const float invGW = 1.0f / (float)GW;
-    for (int i = tid; i < GW * GH; i += kSyThreads) {
+    auto sample = [&](int i, bool lookup) {
         const int r = (int)__fmul_rz(__int2float_rn(i) + 0.5f, invGW), c = i - r * GW;
         const int qx = gx0 + c, qy = gy0 + r;
         float2 v = __ldg(p.pf + (size_t)qy * p.fw + qx);
-        if (p.lookup) {
+        if (lookup) {
             const float fx = (float)qx, fy = (float)qy;
 #pragma unroll
             for (int it = 0; it < 2; it++)
-                v = remapF2m(p.pf, p.fw, p.fh, __fsub_rn(fx, __fmul_rn(p.s, v.x)), __fsub_rn(fy, __fmul_rn(p.s, v.y)));
+                v = remapF2m<kLat>(p.pf, p.fw, p.fh, __fsub_rn(fx, __fmul_rn(p.s, v.x)), __fsub_rn(fy, __fmul_rn(p.s, v.y)));
         }
         g[i] = v;
-        out |= !(fabsf(v.x) * kf <= mx) || !(fabsf(v.y) * kf <= my);   // (a NaN is out too)
-        if (kUi) {
-            nearX |= !(fabsf(v.x) * kf < gapX);
-            nearY |= !(fabsf(v.y) * kf < gapY);
+        return v;
+    };
+    bool out = false, nearX = false, nearY = false;
+    if (kSplit) {
+        uint32_t ax = 0, ay = 0;   // the largest |v.x|, |v.y| as bits (a NaN is above every number)
+        auto largest = [&](float2 v) {
+            ax = max(ax, __float_as_uint(fabsf(v.x)));
+            ay = max(ay, __float_as_uint(fabsf(v.y)));
+        };
+        if (p.lookup)
+            for (int i = tid; i < GW * GH; i += kSyThreads) largest(sample(i, true));
+        else
+            for (int i = tid; i < GW * GH; i += kSyThreads) largest(sample(i, false));
+        const float vx = __uint_as_float(ax) * kf, vy = __uint_as_float(ay) * kf;
+        out = !(vx <= mx) || !(vy <= my);   // (a NaN is out too)
+        nearX = !(vx < gapX);
+        nearY = !(vy < gapY);
+    } else {
+        static_assert(kSplit || !kUi, "the protected kernels vote after the loop");
+        for (int i = tid; i < GW * GH; i += kSyThreads) {
+            const float2 v = sample(i, p.lookup);
+            out |= !(fabsf(v.x) * kf <= mx) || !(fabsf(v.y) * kf <= my);
         }
     }
-    f.in = !__syncthreads_or(out);
     f.ui = false;
-    if (kUi) {
-        const int nx = __syncthreads_or(nearX), ny = __syncthreads_or(nearY);
-        f.ui = nx && ny;
+    if (kUi) {   // three votes, one barrier
+        __shared__ uint32_t vote[kSyThreads / 32];
+        const uint32_t mine = __reduce_or_sync(0xffffffffu, (out ? 1u : 0u) | (nearX ? 2u : 0u) | (nearY ? 4u : 0u));
+        if ((tid & 31) == 0) vote[tid >> 5] = mine;
+        __syncthreads();
+        const uint32_t all = __reduce_or_sync(0xffffffffu, vote[tid & (kSyThreads / 32 - 1)]);
+        f.in = !(all & 1u);
+        f.ui = (all & 6u) == 6u;
+    } else {
+        f.in = !__syncthreads_or(out);
     }
     return f;
 }
@@ -473,8 +504,10 @@ __device__ __forceinline__ float2 syLerp(float2 h0, float2 h1, float a0, float a
 // ::in): rows follow flowScale 2's pattern, the tile's first row odd: two rows share their pair of field rows, weights
 // (3/4, 1/4) and (1/4, 3/4) x 2. Else from the row coefficients, a field row loaded when the pair moves on. kRows rows
 // per loop round: the 8-bit kernels stay rolled (2) where many CTAs share an SM (a 4K synthesis at t = 1/2: 78 us rolled,
-// 83 us unrolled) and unroll (8) for grids of about one CTA per SM.
-template <bool kIn, int kRows, class F>
+// 83 us unrolled) and unroll (8) for grids of about one CTA per SM. kFlat: both field rows read for every row, no branch between
+// the samples of neighbouring rows: for the latency forms, and for the border tiles of the 8-bit kernels, which
+// end a small grid (1280x720: 17.4 -> 16.9 us, 1920x1080 at flowScale 4 26.1 -> 24.7).
+template <bool kIn, int kRows, bool kFlat = false, class F>
 __device__ __forceinline__ void syWalk(const SyField& f, const float4* rowc, int ey0, F&& fn) {
     if (kIn) {
         const float y0 = rowc[ey0 * kSyK].w;
@@ -493,6 +526,10 @@ __device__ __forceinline__ void syWalk(const SyField& f, const float4* rowc, int
         for (int k = 0; k < kSyK; k++) {
             const float4 r = rowc[ey0 * kSyK + k];
             const int i0 = __float_as_int(r.x) & 0xFFFF, i1 = __float_as_int(r.x) >> 16;
+            if (kFlat) {   // no branch between the rows' samples
+                fn(k, ey0 * kSyK + k, r.w, syLerp(syColField(f, i0), syColField(f, i1), r.y, r.z));
+                continue;
+            }
             if (i0 != c0) {   // uniform over the warp
                 h0 = i0 == c1 ? h1 : syColField(f, i0);
                 c0 = i0;

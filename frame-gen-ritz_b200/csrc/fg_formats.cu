@@ -566,7 +566,7 @@ struct SyFalse { static constexpr bool value = false; };
 // kUi: CrosshairV2's warp-tap rejection (gpu/shaders/ui_reject.glsl): a tap whose footprint (YUV: the 2x2 chroma
 // texels around it) touches its own frame's UI mask (p.uiA / p.uiC) takes the other frame's tap (both or neither:
 // kept); the block-centre chroma of the even-even pixels is rejected on its own positions (uiRejectC)
-template <int F, bool kCut, bool kUi = false, class Sink>
+template <int F, bool kCut, bool kUi = false, bool kLat = false, class Sink>
 __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int by, Sink& sink) {
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ float4 rowc[kSyEH];
@@ -583,11 +583,11 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
     if (tid == 0) cnt = nSlow = 0;
     uint8_t* e;
     unsigned short* hsum;
-    const SyField f = syFieldStage<kUi>(p, X0, Y0, tid, ex, rowc, sm, e, hsum);
+    const SyField f = syFieldStage<kUi, kLat, kLat || kUi>(p, X0, Y0, tid, ex, rowc, sm, e, hsum);
     const SyCoef& cx = f.cx;
     const float kA = p.mid ? 1.0f : p.ka, kC = p.mid ? 1.0f : p.kc;
     constexpr bool kYuv = F == kFmtNv12 || F == kFmtP010;
-    constexpr int kRows = fmtRows(F);
+    constexpr int kRows = kLat ? kSyK : fmtRows(F);
     // the blend inputs m of the output pixels, kept from stage 2 for stage 4 (the warps are computed once): per channel
     // planes of kSyTH x kSyE floats (YUV: the luma plane, then the block-centre chroma (Cb, Cr) of the even-even
     // pixels, (kSyTH / 2) x (kSyE / 2))
@@ -669,7 +669,7 @@ __device__ __forceinline__ void synthFmtTile(const SynthParams& p, int bx, int b
         }
     };
     if (f.in && !f.ui) syWalk<true, kRows>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) { stage2(SyTrue(), ey, posy, h); });
-    else syWalk<false, kRows>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) { stage2(SyFalse(), ey, posy, h); });
+    else syWalk<false, kUi && kRows < 4 ? 4 : kRows, kLat || kUi>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) { stage2(SyFalse(), ey, posy, h); });
     __syncthreads();
     if (pq) {   // the undecided pixels (about 2 % on natural content), dealt out over all threads: warped again, exact
         const int n = min((int)nSlow, kPqSlow);
@@ -787,6 +787,15 @@ __global__ void __launch_bounds__(kSyThreads, fmtCtas(F)) k_synth_fmt_ui(const S
     pdlEnter();
     FmtStore<F> store{p};
     synthFmtTile<F, true, true>(p, blockIdx.x, blockIdx.y, store);
+}
+// grids of at most 2 CTAs per SM, as k_synth_lat: all rows' samples in flight together. A frame here is one tile's latency:
+// with its fallback check, Rgb10 640x360 25.5 -> 16.6 us, 1024x576 22.5 -> 18.2, encoded RgbaF16 24.1 -> 16.9 and 21.1 -> 17.8.
+// One more wave costs more than it gives: from 297 tiles on the three CTAs per SM of k_synth_fmt.
+template <int F, bool kUi>
+__global__ void __launch_bounds__(kSyThreads, 2) k_synth_fmt_lat(const SynthParams p) {
+    pdlEnter();
+    FmtStore<F> store{p};
+    synthFmtTile<F, true, kUi, true>(p, blockIdx.x, blockIdx.y, store);
 }
 
 // Many syntheses of one format in one persistent launch (as k_synth_batch for 8-bit RGBA): every CTA takes the next
@@ -1023,6 +1032,17 @@ static size_t fmtSynthSmem(int format, int fs) {
     return synthSmemBytes(fs) - (size_t)kSyEH * kSyHS * 2 + kPqSegBytes + kPqSlow * 2 + mix;   // the PQ segments over hsum
 }
 
+template <int F>
+static cudaError_t prepareSynthF(int smem) {
+    for (const void* k : {(const void*)k_synth_fmt<F>, (const void*)k_synth_fmt_ui<F>, (const void*)k_synth_fmt_lat<F, false>,
+                          (const void*)k_synth_fmt_lat<F, true>, (const void*)k_synth_fmt_batch<F>, (const void*)k_synth_blur_fmt<F, false>,
+                          (const void*)k_synth_blur_fmt<F, true>}) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 cudaError_t prepareFormatKernels() {
     // The linear RgbaF16 luma pass lives on its table's hits in L1 (3 gathers a pixel): it asks for the shared memory of its
     // 8 CTAs and no more. Left to the driver it ran on in the synthesis' configuration, which three CTAs leave almost no
@@ -1032,30 +1052,10 @@ cudaError_t prepareFormatKernels() {
         if (c != cudaSuccess) return c;
     }
     const int smem = (int)fmtSynthSmem(kFmtF16, 1);   // the largest
-    cudaError_t e = cudaFuncSetAttribute(k_synth_fmt<kFmtRgb10>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt<kFmtF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt<kFmtNv12>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt<kFmtP010>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt_batch<kFmtRgb10>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt_batch<kFmtF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt_batch<kFmtNv12>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt_batch<kFmtP010>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt_ui<kFmtRgb10>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt_ui<kFmtF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt_ui<kFmtNv12>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_fmt_ui<kFmtP010>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_synth_blur_fmt<kFmtNv12, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_synth_blur_fmt<kFmtP010, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_synth_blur_fmt<kFmtRgb10, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_synth_blur_fmt<kFmtF16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_blur_fmt<kFmtRgb10>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_blur_fmt<kFmtF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_blur_fmt<kFmtNv12>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_blur_fmt<kFmtP010>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = prepareSynthF<kFmtRgb10>(smem);
+    if (e == cudaSuccess) e = prepareSynthF<kFmtF16>(smem);
+    if (e == cudaSuccess) e = prepareSynthF<kFmtNv12>(smem);
+    if (e == cudaSuccess) e = prepareSynthF<kFmtP010>(smem);
     return e;
 }
 
@@ -1132,23 +1132,20 @@ cudaError_t launchPqSegments(float2* seg, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launchSynthFmt(const SynthParams& p, cudaStream_t s) {
+template <int F>
+static cudaError_t launchSynthF(const SynthParams& p, cudaStream_t s) {
     const dim3 grid(divUp(p.W, kSyT), divUp(p.H, kSyTH));
-    const size_t smem = fmtSynthSmem(p.f.format, p.fs);
-    if (p.uiA || p.uiC) {   // CrosshairV2: the tap rejection compiled in
-        switch (p.f.format) {
-            case kFmtRgb10: return launchPdl(k_synth_fmt_ui<kFmtRgb10>, grid, dim3(kSyThreads), smem, s, p);
-            case kFmtF16: return launchPdl(k_synth_fmt_ui<kFmtF16>, grid, dim3(kSyThreads), smem, s, p);
-            case kFmtNv12: return launchPdl(k_synth_fmt_ui<kFmtNv12>, grid, dim3(kSyThreads), smem, s, p);
-            case kFmtP010: return launchPdl(k_synth_fmt_ui<kFmtP010>, grid, dim3(kSyThreads), smem, s, p);
-            default: return cudaErrorInvalidValue;
-        }
-    }
+    const bool ui = p.uiA || p.uiC;   // CrosshairV2: the tap rejection compiled in
+    auto k = (int)(grid.x * grid.y) <= 2 * smCount() ? (ui ? k_synth_fmt_lat<F, true> : k_synth_fmt_lat<F, false>)
+                                                     : (ui ? k_synth_fmt_ui<F> : k_synth_fmt<F>);
+    return launchPdl(k, grid, dim3(kSyThreads), fmtSynthSmem(F, p.fs), s, p);
+}
+cudaError_t launchSynthFmt(const SynthParams& p, cudaStream_t s) {
     switch (p.f.format) {
-        case kFmtRgb10: return launchPdl(k_synth_fmt<kFmtRgb10>, grid, dim3(kSyThreads), smem, s, p);
-        case kFmtF16: return launchPdl(k_synth_fmt<kFmtF16>, grid, dim3(kSyThreads), smem, s, p);
-        case kFmtNv12: return launchPdl(k_synth_fmt<kFmtNv12>, grid, dim3(kSyThreads), smem, s, p);
-        case kFmtP010: return launchPdl(k_synth_fmt<kFmtP010>, grid, dim3(kSyThreads), smem, s, p);
+        case kFmtRgb10: return launchSynthF<kFmtRgb10>(p, s);
+        case kFmtF16: return launchSynthF<kFmtF16>(p, s);
+        case kFmtNv12: return launchSynthF<kFmtNv12>(p, s);
+        case kFmtP010: return launchSynthF<kFmtP010>(p, s);
         default: return cudaErrorInvalidValue;
     }
 }

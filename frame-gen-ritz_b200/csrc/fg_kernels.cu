@@ -1253,7 +1253,7 @@ __device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int 
     }
     uint8_t* e;
     unsigned short* hsum;
-    const SyField f = syFieldStage<kUi>(p, X0, Y0, tid, ex, rowc, sm, e, hsum);
+    const SyField f = syFieldStage<kUi, kLat, true>(p, X0, Y0, tid, ex, rowc, sm, e, hsum);
     // 2. this thread's region column and kSyK rows: half-vector, both warps, mismatch. The warps wait in shared memory
     //    for the blend (in registers they would leave too few for the sample loads in flight).
     uint32_t* sWA = reinterpret_cast<uint32_t*>(hsum + kSyEH * kSyHS);   // the output rows: kSyTH x kSyE
@@ -1280,7 +1280,7 @@ __device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int 
             keep(ey, A, C, maxDiffU8(A, C));
         });
     } else {
-        syWalk<false, 2>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) {
+        syWalk<false, kLat ? kSyK : 4, true>(f, rowc, ey0, [&](int, int ey, float posy, float2 h) {
             float2 ba, bc;
             positions(posy, h, ba, bc);
             uint32_t A = sampleU8(fa32, pw, p.W, p.H, ba.x, ba.y), C = sampleU8(fc32, pw, p.W, p.H, bc.x, bc.y);
@@ -1386,14 +1386,10 @@ __device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int 
             }
             sink.put(k, __byte_perm(o, nq, 0x7210));
         };
-        if constexpr (Sink::kIndexed) {   // unrolled: k indexes the sink's registers (a pragma with Sink's number does nothing)
-#pragma unroll
-            for (int k = 0; k < kSyK; k++) {
-                if (k >= rows) break;
-                pixel(k);
-            }
-        } else {
-            for (int k = 0; k < rows; k++) pixel(k);
+#pragma unroll   // the sink's registers need every k known; rolled, unrelated frames took 1920x1080 27.7 us instead of 26.0
+        for (int k = 0; k < kSyK; k++) {
+            if (k >= rows) break;
+            pixel(k);
         }
     }
     if (p.emap)
@@ -1406,7 +1402,6 @@ __device__ __forceinline__ void synthTileCore(const SynthParams& p, int bx, int 
 
 // the store of a synthesis: rows of p.out from (x, y0) down
 struct SynthStore {
-    static constexpr bool kIndexed = false;
     const SynthParams& p;
     uint8_t* o;
     __device__ __forceinline__ void begin(int x, int y0) { o = p.out + (size_t)y0 * p.outPitch + (size_t)x * 4; }
@@ -1419,8 +1414,7 @@ struct SynthStore {
 // a blur's sample: acc += q x the pixel
 struct BlurAdd {
     // acc in registers needs every put's k known. With the mixed-trust rows rolled it was a 96-byte stack frame: 7680x4320
-    // with 16 samples 6.78 ms a frame and its estimate, now 6.47 (unrelated frames 7.20 -> 6.79).
-    static constexpr bool kIndexed = true;
+    // with 16 samples 6.78 ms a frame and its estimate, unrolled 6.47 (unrelated frames 7.20 -> 6.79).
     uint32_t (&acc)[kSyK][3];
     uint32_t q;
     __device__ __forceinline__ void begin(int, int) {}
@@ -1452,6 +1446,11 @@ __global__ void __launch_bounds__(kSyThreads, 2) k_synth_lat(const SynthParams p
 __global__ void __launch_bounds__(kSyThreads, 3) k_synth_ui(const SynthParams p) {
     pdlEnter();
     synthTile<true>(p, blockIdx.x, blockIdx.y);
+}
+// (640x360 with the fallback check and the paste 24.8 -> 16.5 us, 1024x576 25.8 -> 18.4)
+__global__ void __launch_bounds__(kSyThreads, 2) k_synth_ui_lat(const SynthParams p) {
+    pdlEnter();
+    synthTile<true, true>(p, blockIdx.x, blockIdx.y);
 }
 
 // Motion blur (gpu/framegen.h:553-573, gpu/shaders/blur_resolve.comp): out = round(sum_k w_k frame_k), frame_k the
@@ -1776,6 +1775,8 @@ cudaError_t prepareKernels() {
                                  (int)(synthSmemBytes(1) + kSyWarpBytes));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_synth_ui, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(synthSmemBytes(1) + kSyWarpBytes));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_synth_ui_lat, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(synthSmemBytes(1) + kSyWarpBytes));
     return e;
 }
 cudaError_t launchSubpix(const SubpixParams& p, cudaStream_t s) {
@@ -1801,10 +1802,10 @@ int synthTilesY(int H) { return (int)divUp(H, kSyTH); }
 cudaError_t launchSynth(const SynthParams& p, cudaStream_t s) {
     const size_t smem = synthSmemBytes(p.fs) + kSyWarpBytes;
     const dim3 grid(divUp(p.W, kSyT), divUp(p.H, kSyTH));
-    if (p.uiA || p.uiC) return launchPdl(k_synth_ui, grid, dim3(kSyThreads), smem, s, p);
+    const bool lat = (int)(grid.x * grid.y) <= 2 * smCount();
+    if (p.uiA || p.uiC) return launchPdl(lat ? k_synth_ui_lat : k_synth_ui, grid, dim3(kSyThreads), smem, s, p);
     // one wave of 2 CTAs per SM (a 640x360 frame: 14.6 -> 11 us, 1280x720 and up about even): the latency form
-    if ((int)(grid.x * grid.y) <= 2 * smCount()) return launchPdl(k_synth_lat, grid, dim3(kSyThreads), smem, s, p);
-    return launchPdl(k_synth, grid, dim3(kSyThreads), smem, s, p);
+    return launchPdl(lat ? k_synth_lat : k_synth, grid, dim3(kSyThreads), smem, s, p);
 }
 cudaError_t launchSynthBlur(const BlurParams& bp, int fix, cudaStream_t s) {
     const size_t smem = synthSmemBytes(bp.base.fs) + kSyWarpBytes;

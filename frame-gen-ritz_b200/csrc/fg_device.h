@@ -293,10 +293,12 @@ __device__ __forceinline__ void storePairPx(uint32_t* plane, int fw, int x, int 
 // output pixel, against 1.29 for 128 x 32) within the shared memory of 3 CTAs per SM.
 //
 // The synthesis kernels are bound by instruction issue and by the latency of the sample loads (8-bit RGBA at 3840x2160,
-// t = 1/2: 74 % issue, 62 M warp instructions, 78 us in a graph; 91 us before the rows of a thread became consecutive with
-// the upsampled field in registers, interior tiles went without clamps, the row sums became byte dot products and fully
-// trusted warps only blend; t = 1/4 105 -> 88 us). Other shapes measured within 3 % of it (64 x 60 with 4 x 384 threads,
-// 64 x 72) or slower (64 x 40, 64 x 48).
+// t = 1/2: 74 % issue, 62.6 M warp instructions, 82.9 us under ncu; back to back with the fallback check 79.5 us, 92.3 before
+// the rows of a thread became consecutive with the upsampled field in registers, interior tiles went without clamps, the
+// row sums became byte dot products and fully trusted warps only blend; t = 1/3 110 -> 94 us). Other shapes measured within
+// 3 % of it (64 x 60 with 4 x 384 threads, 64 x 72) or slower (64 x 40, 64 x 48). The forms of three CTAs per SM spill up
+// to 48 bytes a thread at their 40 registers (-Xptxas -v); two CTAs per SM spill nothing and are slower on large grids but
+// for Nv12 (fmtCtas).
 constexpr int kSyE = 64, kSyEH = 64, kSyAp = 3;
 constexpr int kSyT = kSyE - 2 * kSyAp, kSyTH = kSyEH - 2 * kSyAp;
 constexpr int kSyThreads = 512, kSyK = kSyEH / (kSyThreads / kSyE);   // region rows per thread (512 = 64 columns x 8)
@@ -397,8 +399,8 @@ __device__ __forceinline__ int uiGap(int o, int side, int lo, int n) {
     return max(o - kSyAp - 4 - (lo + n - 1), lo - 4 - (o - kSyAp + side - 1));
 }
 // kSplit: a loop for the lookup at t and one for the plain field, the vectors' largest parts voted on after it. The 8-bit
-// kernels, the latency forms and the protected ones gain by it (3840x2160: 81 -> 80 us, 1280x720 17.9 -> 16.9); the formats'
-// 40-register kernels lose 1 to 2 % at 3840x2160 and keep one loop.
+// kernels, the latency forms and the protected ones gain by it (8-bit 1280x720 17.9 -> 17.4 us, unrelated frames of 1920x1080
+// 27.0 -> 26.6); the formats' 40-register kernels lose 1 % at 3840x2160 and keep one loop.
 template <bool kUi, bool kLat, bool kSplit>
 __device__ __forceinline__ SyField syFieldStage(const SynthParams& p, int X0, int Y0, int tid, int ex, float4* rowc,
                                                 unsigned char* sm, uint8_t*& e, unsigned short*& hsum) {
@@ -506,7 +508,7 @@ __device__ __forceinline__ float2 syLerp(float2 h0, float2 h1, float a0, float a
 // per loop round: the 8-bit kernels stay rolled (2) where many CTAs share an SM (a 4K synthesis at t = 1/2: 78 us rolled,
 // 83 us unrolled) and unroll (8) for grids of about one CTA per SM. kFlat: both field rows read for every row, no branch between
 // the samples of neighbouring rows: for the latency forms, and for the border tiles of the 8-bit kernels, which
-// end a small grid (1280x720: 17.4 -> 16.9 us, 1920x1080 at flowScale 4 26.1 -> 24.7).
+// end a small grid (with the mixed-trust rows unrolled: 1280x720 17.9 -> 16.9 us, 1920x1080 at flowScale 4 26.1 -> 24.7).
 template <bool kIn, int kRows, bool kFlat = false, class F>
 __device__ __forceinline__ void syWalk(const SyField& f, const float4* rowc, int ey0, F&& fn) {
     if (kIn) {

@@ -3,10 +3,11 @@
 // weights, absolute differences one instruction (sad), all sums exact in 32 bits: the same values as the float kernels
 // of fg_kernels.cu, which run where level 0 is not a multiple of 1/16 (flowScale 4 with 3-pixel cells).
 //
-// All three passes are bound by instruction issue (66-77 % issue, ALU and FMA-heavy pipes 40-60 %). Measured (ncu,
-// 3840x2160 at flowScale 2, float kernel -> this one; warp instructions): level-0 search 41.4 -> 28.6 us (30.1 -> 20.1
-// M), sub-pixel 65.9 -> 24 us (38.6 -> 17 M, the scene-cut sum moved to the pixel-field launch), pixel field 80.4 ->
-// 43 us (52.8 -> 26.2 M). The pair planes cost the luma pass nothing: float level 0 is written only where a pass reads it.
+// The searches and the sub-pixel pass are bound by instruction issue (76 and 83 % of the issue slots), the pixel field by
+// issue and its barriers (66 %, 24 warps per SM). Measured (ncu, 3840x2160 at flowScale 2, float kernel -> this one; warp
+// instructions): level-0 search 41.4 -> 29.7 us (30.1 -> 20.1 M), sub-pixel 65.9 -> 26.9 us (38.6 -> 20.1 M; it took the
+// scene-cut sum then and takes level 0's median3 now), pixel field 80.4 -> 42.4 us (52.8 -> 25.4 M, the scene-cut sum with
+// it). The pair planes cost the luma pass nothing: float level 0 is written only where a pass reads it.
 #include "fg_device.h"
 
 namespace fgk {

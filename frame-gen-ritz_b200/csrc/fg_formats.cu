@@ -262,8 +262,8 @@ __device__ __forceinline__ void lumaFmtCells(const LumaPyrParams& p, float (*sl)
 }
 
 // interp.flow + pyramid for the other formats: one CTA = a 32x32 level-0 tile and its tower (as k_luma_pyr). Whole tiles of
-// aligned frames at flowScale 2 (p.vec16) take 4 frame pixels x 2 rows per thread and load (4K: Rgb10 49 -> 31 us, linear
-// RgbaF16 78 -> 66, Nv12 35 -> 20, P010 37 -> 21): bound by instruction issue, linear RgbaF16 by its table gathers.
+// aligned frames at flowScale 2 (p.vec16) take 4 frame pixels x 2 rows per thread and load (ncu, 4K: Rgb10 41 -> 38 us, linear
+// RgbaF16 59 -> 58, Nv12 30 -> 18, P010 30 -> 19): bound by instruction issue, linear RgbaF16 by its table gathers.
 template <int F>
 __device__ __forceinline__ void lumaFmtCta(const LumaPyrParams& p, int bx, int by) {
     __shared__ __align__(8) float sl[2][kTowerFloats];

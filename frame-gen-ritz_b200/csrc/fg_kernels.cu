@@ -19,7 +19,7 @@ namespace fgk {
 // ============================================================================================== luma + pyramid
 // the level-0 cells of a 32x32 tile at the frame's edge, or of a frame off the vector path: 4 cells per thread, every load of
 // a pair of cells in flight at once (pixels past the frame are read at the edge and not counted). With a loop per pixel
-// these tiles were the latency of the whole pass (1080p 14 us, now 6).
+// these tiles were the latency of the whole pass (1080p 13.3 us, now 10.4, ncu).
 template <int FS>
 __device__ __forceinline__ void lumaCells(const LumaPyrParams& p, float (*sl)[kTowerFloats], int tx0, int ty0) {
     const int fw = p.lw[0], fh = p.lh[0];
@@ -1414,7 +1414,7 @@ struct SynthStore {
 // a blur's sample: acc += q x the pixel
 struct BlurAdd {
     // acc in registers needs every put's k known. With the mixed-trust rows rolled it was a 96-byte stack frame: 7680x4320
-    // with 16 samples 6.78 ms a frame and its estimate, unrolled 6.47 (unrelated frames 7.20 -> 6.79).
+    // with 16 samples 6.77 ms a frame and its estimate, now 6.33 (unrelated frames 7.22 -> 6.67).
     uint32_t (&acc)[kSyK][3];
     uint32_t q;
     __device__ __forceinline__ void begin(int, int) {}

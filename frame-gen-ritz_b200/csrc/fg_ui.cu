@@ -11,7 +11,7 @@
 //                   binary search on the value for the smallest m with at least 25 of the 49 levels <= m, the window's
 //                   49 pixels packed one word each in registers, from the CTA's 22 x 14 pixels staged in shared memory
 //                   (each converted once; read from the frame by every thread, its 49 loads waited on one another
-//                   behind the format's branches: a 128 x 128 box 34 us, staged 11 us, ncu).
+//                   behind the format's branches: a 128 x 128 box 34 us, staged 13 us, ncu).
 //   k_ui_v2_mask    one thread per mask word (4 pixels): in the mask or within 1 px of it -> 255 if still in this pair,
 //                   else 64; writes the rectangle into the header.
 //   k_ui_patch      one thread per work-rectangle pixel: out = the real curr pixel (colour channels) where the byte is
@@ -253,11 +253,11 @@ __global__ void __launch_bounds__(kUiTX * kUiTY) k_ui_patch_chroma(const UiPatch
             __ldg(reinterpret_cast<const uint32_t*>(p.currC + (size_t)ty * p.cpitch) + tx);
 }
 
-// The estimate fill (gpu/shaders/ui_v2_lumafill.comp), one thread per level-0 cell of the mask rectangle, z = 0 prev,
+// The estimate fill (gpu/shaders/ui_v2_lumafill.comp), one warp per level-0 cell of the mask rectangle, y = 0 prev,
 // 1 curr: a cell holding a UI pixel takes the mean gray level (cv2's weights, the library's level-0 source) of its
 // not-UI pixels, the window widened by fs px per side per step up to 8 px while there are none, rounded half up to the
 // level-0 grid (multiples of 1 / fs^2) so the estimate's sums stay exact.
-__global__ void __launch_bounds__(128) k_ui_v2_fill(const UiFillParams p) {   // a warp per cell
+__global__ void __launch_bounds__(128) k_ui_v2_fill(const UiFillParams p) {
     pdlEnter();
     const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int cx = p.cx0 + i % p.ncx, cy = p.cy0 + i / p.ncx;

@@ -671,19 +671,27 @@ static int layoutMerged(Merged<P>& m, F ctasOf) {   // ctasOf(item, gx&) -> the 
     return total;
 }
 
+// carveout: the launch's preferred share of shared memory in the SM's L1, in percent (0: no more than a CTA needs)
 template <typename... KArgs, typename... Args>
-cudaError_t launchPdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+cudaError_t launchPdlCarveout(int carveout, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = (unsigned int)carveout;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = carveout < 0 ? 1 : 2;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+// ... left to the driver
+template <typename... KArgs, typename... Args>
+cudaError_t launchPdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+    return launchPdlCarveout(-1, kernel, grid, block, smem, s, args...);
 }
 
 }  // namespace fgk

@@ -1640,9 +1640,16 @@ cudaError_t launchSearch(const SearchParams& p, cudaStream_t s) {
         case 4: return launchSearchR<4>(p, s);
         case 5: return launchSearchR<5>(p, s);
         case 6: return launchSearchR<6>(p, s);
-        default: {   // radii 7..12 (settings beyond the defaults): the runtime-radius kernel
+        default: {
+            // radii 7..12 (settings beyond the defaults): the runtime-radius kernel, 16 to 32 KB of windows per CTA. On its own
+            // the driver splits the SM's L1 for as many of these CTAs as fit, and the level waits until every SM is idle to
+            // change the split and the next pass to change it back; a small level has a CTA or two per SM and asks for no
+            // more (searchRadiusTop 12, an estimate: 640x360 84 -> 46 us, 1280x720 106 -> 60, 1920x1080 91 -> 80; with radius 9
+            // everywhere 640x360 87 -> 63). Large levels need the occupancy: 3840x2160 with radius 9 654 us, 928 at no more
+            // than a CTA's need.
             const int T = 8 + 2 * p.R;
-            return launchPdl(k_search, dim3(divUp(p.bw * p.bh, 4)), dim3(128), (size_t)4 * 2 * T * T * sizeof(float), s, p);
+            return launchPdlCarveout(p.bw * p.bh <= kSearchLatBlocks ? 0 : -1, k_search, dim3(divUp(p.bw * p.bh, 4)), dim3(128),
+                                     (size_t)4 * 2 * T * T * sizeof(float), s, p);
         }
     }
 }

@@ -693,5 +693,12 @@ template <typename... KArgs, typename... Args>
 cudaError_t launchPdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
     return launchPdlCarveout(-1, kernel, grid, block, smem, s, args...);
 }
+// The carveout of a synthesis. A tile of flowScale 1 takes 75 to 105 KB (the whole field region); on a grid of at most one
+// CTA per SM the driver splits the L1 for two or three of them, and each change of the split waits for an idle SM: such
+// grids ask for one CTA's need (back to back with the fallback check, 640x360 at t = 1/3: 8-bit 17.7 -> 14.1 us, Rgb10 22.8
+// -> 14.8, P010 28.4 -> 21.0; a pair doubled 63 -> 61, 69 -> 63, 77 -> 69). With more CTAs a second one per SM pays
+// (1024x576, 180 tiles: 20.8 us, 23.4 so), and at flowScale 4 the estimate changes the split back (a Rgb10 pair at 640x360
+// 48 -> 55).
+inline int synthCarveout(const SynthParams& p, dim3 grid) { return p.fs == 1 && (int)(grid.x * grid.y) <= smCount() ? 0 : -1; }
 
 }  // namespace fgk

@@ -1138,7 +1138,7 @@ static cudaError_t launchSynthF(const SynthParams& p, cudaStream_t s) {
     const bool ui = p.uiA || p.uiC;   // CrosshairV2: the tap rejection compiled in
     auto k = (int)(grid.x * grid.y) <= 2 * smCount() ? (ui ? k_synth_fmt_lat<F, true> : k_synth_fmt_lat<F, false>)
                                                      : (ui ? k_synth_fmt_ui<F> : k_synth_fmt<F>);
-    return launchPdl(k, grid, dim3(kSyThreads), fmtSynthSmem(F, p.fs), s, p);
+    return launchPdlCarveout(synthCarveout(p, grid), k, grid, dim3(kSyThreads), fmtSynthSmem(F, p.fs), s, p);
 }
 cudaError_t launchSynthFmt(const SynthParams& p, cudaStream_t s) {
     switch (p.f.format) {

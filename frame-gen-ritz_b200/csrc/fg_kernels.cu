@@ -1810,9 +1810,9 @@ cudaError_t launchSynth(const SynthParams& p, cudaStream_t s) {
     const size_t smem = synthSmemBytes(p.fs) + kSyWarpBytes;
     const dim3 grid(divUp(p.W, kSyT), divUp(p.H, kSyTH));
     const bool lat = (int)(grid.x * grid.y) <= 2 * smCount();
-    if (p.uiA || p.uiC) return launchPdl(lat ? k_synth_ui_lat : k_synth_ui, grid, dim3(kSyThreads), smem, s, p);
+    if (p.uiA || p.uiC) return launchPdlCarveout(synthCarveout(p, grid), lat ? k_synth_ui_lat : k_synth_ui, grid, dim3(kSyThreads), smem, s, p);
     // one wave of 2 CTAs per SM (a 640x360 frame: 14.6 -> 11 us, 1280x720 and up about even): the latency form
-    return launchPdl(lat ? k_synth_lat : k_synth, grid, dim3(kSyThreads), smem, s, p);
+    return launchPdlCarveout(synthCarveout(p, grid), lat ? k_synth_lat : k_synth, grid, dim3(kSyThreads), smem, s, p);
 }
 cudaError_t launchSynthBlur(const BlurParams& bp, int fix, cudaStream_t s) {
     const size_t smem = synthSmemBytes(bp.base.fs) + kSyWarpBytes;

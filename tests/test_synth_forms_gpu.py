@@ -1,5 +1,5 @@
 """The synthesis' forms by grid: at most 2 CTAs per SM (the latency form) and more, at 289 and 306 tiles of 58 x 58 (B200 has
-148 SMs), in every format and flow scale, plain and with the overlay protection, against the oracle; and the mask test of
+148 SMs; up to 148 tiles ask for another split of the L1 at flowScale 1), in every format and flow scale, plain and with the overlay protection, against the oracle; and the mask test of
 a tap's pixels, which reads whole words, with masks whose rows end at every place of a word."""
 import numpy as np
 import pytest
@@ -14,7 +14,7 @@ from test_ui_v2_fmt_gpu import SPECS, dev, empty_like, host, same
 from test_ui_v2_gpu import grain_scene, oracle_settings, v2_settings
 
 pytestmark = pytest.mark.gpu
-SIZES = [(986, 986), (1044, 986)]
+SIZES = [(986, 986), (1044, 986), (696, 696), (232, 2146)]   # 289, 306, 144 and 148 tiles
 
 
 @pytest.fixture(scope="module", autouse=True)

@@ -1,6 +1,7 @@
 """The synthesis' forms by grid: at most 2 CTAs per SM (the latency form) and more, at 289 and 306 tiles of 58 x 58 (B200 has
-148 SMs; up to 148 tiles ask for another split of the L1 at flowScale 1), in every format and flow scale, plain and with the overlay protection, against the oracle; and the mask test of
-a tap's pixels, which reads whole words, with masks whose rows end at every place of a word."""
+148 SMs; up to 148 tiles ask for another split of the L1 at flowScale 1), in every format and flow scale, plain and with
+the overlay protection, against the oracle; and the mask test of a tap's pixels, which reads whole words, with masks
+whose rows end at every place of a word."""
 import numpy as np
 import pytest
 import torch
@@ -75,8 +76,8 @@ def protected(name, W, H, box, offset, ts, **kw):
 
 
 @pytest.mark.parametrize("name", ["rgba8", "rgb10", "f16_linear", "f16_encoded", "nv12", "p010"])
-@pytest.mark.parametrize("fs", [1, 2, 4])
-@pytest.mark.parametrize("W,H", SIZES)
+@pytest.mark.parametrize("fs", [1, 2])
+@pytest.mark.parametrize("W,H", [SIZES[1], SIZES[2]])
 def test_protected_one_wave_and_more(W, H, fs, name):
     protected(name, W, H, (90, 70), (20, -14), [0.5, T13], flowScale=fs)
 
